@@ -367,6 +367,43 @@ def test_delta_decode_int8_matches_oracle(cuda, ops, batch, v_heads):
         assert np.array_equal(scales[slot], case["scales"][slot])
 
 
+@pytest.mark.parametrize("batch,v_heads", [(18, 32), (19, 32), (12, 48), (13, 48), (2, 32), (3, 48)],
+                         ids=["last_four_lanes", "first_eight_lanes", "last_four_lanes_h48", "first_eight_lanes_h48",
+                              "row_split_8", "row_split_4"])
+@pytest.mark.parametrize("exponent", [0, -100], ids=["fixed_point", "fp32_sums"])
+def test_delta_decode_both_forms(cuda, ops, batch, v_heads, exponent):
+    """On either side of the line between four and eight lanes per row, with row splits, and with a k that
+    the fixed-point sums do not take.  Bounds: out within 1e-5 of its largest value (128 fp32 roundings
+    of 6e-8 in the oracle's sums, one here), codes within one step, where u moves by a unit in the last place."""
+    case = synth.delta_case(11, batch, v_heads)
+    k = case["k"].copy()
+    k[0] = 0.0
+    k[1] = np.ldexp(k[1], exponent)
+    case = dict(case, k=k, kq=np.einsum("bhd,bhd->bh", case["q"], k).astype(np.float32))
+    want_state, want_scales = case["state"].copy(), case["scales"].copy()
+    want_out = oracle.delta_decode_int8(want_state, want_scales, case["slots"], case["q"], case["k"], case["v"],
+                                        case["alpha"], case["beta"], case["kq"], batch, v_heads)
+    state, scales, out = run_delta(cuda, ops, case, batch, v_heads)
+    assert np.max(np.abs(out - want_out)) <= 1e-5 * np.max(np.abs(want_out))
+    diff = np.abs(state.astype(np.int32) - want_state.astype(np.int32))
+    assert diff.max() <= 1 and np.mean(diff > 0) < 1e-4
+    assert np.allclose(scales, want_scales, rtol=1e-5, atol=0)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_delta_non_finite_key_stays_in_its_head(cuda, ops, value):
+    batch, v_heads = 3, 32
+    case = synth.delta_case(12, batch, v_heads)
+    k = case["k"].copy()
+    k[1, 4, 17] = value
+    _, _, clean = run_delta(cuda, ops, case, batch, v_heads)
+    _, _, out = run_delta(cuda, ops, dict(case, k=k), batch, v_heads)
+    hit = np.zeros((batch, v_heads), dtype=bool)
+    hit[1, 8:10] = True  # two value heads per key head
+    assert not np.isfinite(out[hit]).any()
+    assert np.array_equal(out[~hit], clean[~hit])
+
+
 def test_delta_requantiser_is_bit_exact(cuda, ops):
     """beta = 0 makes every fp32 row value alpha * s exactly (tests/delta_net.rs:138-182), so the
     int8 codes and scales must equal the oracle's bit for bit."""
