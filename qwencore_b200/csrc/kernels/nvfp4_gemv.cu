@@ -42,6 +42,9 @@ namespace cg = cooperative_groups;
 namespace qwc {
 
 // tcgen05 paths (nvfp4_umma.cu): NVFP4 projections, and the e4m3 vocabulary head.
+cudaError_t launch_nvfp4_native(const void* packed0, const void* scales0, const void* packed1, const void* scales1,
+                                const __nv_bfloat16* x, __nv_bfloat16* y, int out_features, int in_features, int batch,
+                                float inverse_scale0, float inverse_scale1, bool swiglu, cudaStream_t stream);
 cudaError_t launch_nvfp4_umma(const void* packed0, const void* scales0, const void* packed1, const void* scales1,
                               const void* x, void* y, int out_features, int in_features, int batch, float inverse0,
                               float inverse1, bool swiglu, cudaStream_t stream);
@@ -657,7 +660,7 @@ cudaError_t dispatch(const GemvParams& p, cudaStream_t stream) {
     const bool wide = MODE == kNvfp4 && wide_tiles >= 2 * sm_count();
     // The tcgen05 kernel streams weights faster than the mma.sync one at every batch size but has a
     // longer start-up (TMEM allocation, first TMA round trip, cluster reduction): it takes over
-    // above eight rows, and below that for matrices of 30 MB and more.
+    // above eight rows, and below that for vocabulary heads of 60 MB and more.
     const bool large = static_cast<long long>(p.out_features) * p.in_features >= 60ll * 1000 * 1000;
     // its stores are 16 bytes wide and its activation fetch is a tiled TMA copy
     const bool aligned = p.out_features % 8 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0 &&
@@ -666,6 +669,16 @@ cudaError_t dispatch(const GemvParams& p, cudaStream_t stream) {
                            reinterpret_cast<uintptr_t>(p.scales[0]) | reinterpret_cast<uintptr_t>(p.scales[1])) & 15) == 0 &&
                          (MODE != kFp8Rows || ((reinterpret_cast<uintptr_t>(p.y_f32) & 15) == 0 &&
                                                (reinterpret_cast<uintptr_t>(p.row_scales) & 15) == 0));
+    // Up to eight rows both operands enter the tensor cores in four bits (nvfp4_native.cuh), unless the
+    // matrix is so small that its start-up shows.  Measured (us, mma.sync or f16 tcgen05 / four bits):
+    // 1040 x 512 at 1 and 8 rows 3.1, 3.8 / 3.8, 4.7; 5120 x 4096 8.1, 8.2 / 6.1, 7.4; 34816 x 5120 25.7,
+    // 24.5 / 20.7, 21.6; above eight rows the digits take longer than the weights (16: 24.6 / 30.3).
+    if (MODE != kFp8Rows && aligned && p.batch <= 8 &&
+        static_cast<long long>(p.out_features) * p.in_features >= 16ll * 1000 * 1000) {
+        return launch_nvfp4_native(p.packed[0], p.scales[0], p.packed[1], p.scales[1], p.x, p.y, p.out_features,
+                                   p.in_features, p.batch, p.inverse_scale[0], p.inverse_scale[1],
+                                   MODE == kNvfp4Swiglu, stream);
+    }
     if (p.batch <= 8 && !(large && aligned)) {
         (void)take_next_projection();  // only the tcgen05 kernel acts on the hint; it is good for one launch
         return launch<1, 1, MODE>(p, stream);

@@ -100,6 +100,7 @@ constexpr size_t kWorkspaceBytes = kPartialBytes + kTicketBytes + kCandidateByte
 struct StreamKParams {
     const uint8_t* scales[2];
     const __half* x;          // staged activations: [K / 8][n_pad][8] f16
+    const __nv_bfloat16* x_rows;  // or bf16 rows [batch][K] (nvfp4_native.cuh only)
     __nv_bfloat16* y;         // bf16 rows [batch][N], or null
     __half* y_staged;         // the same values staged for the next projection: [N / 8][n_pad][8] f16, or null
     float* y_f32;             // vocabulary head: fp32 logits [batch][N], or null
@@ -267,6 +268,45 @@ __device__ __forceinline__ const float* piece_of(const float* partials, int unit
     return partials + (static_cast<size_t>(owner * 2 + slot) * kEpilogueWarps + e) * kPartialWarpFloats;
 }
 
+// Asks L2 for the first stages of the shares of the launch that follows, dealt over this launch's CTAs
+// (one thread).
+__device__ __forceinline__ void prefetch_next_launch(const StreamKParams::Next& next, const CUtensorMap& map0,
+                                                     const CUtensorMap& map1, int cta, int ctas) {
+    for (int other = cta; other < next.ctas; other += ctas) {
+        int first, end;
+        if (next.splits > 0) {
+            const int its_pair = other / next.splits;
+            const int its_slice = other - its_pair * next.splits;
+            first = its_pair * next.stages_in_k + next.stages_in_k * its_slice / next.splits;
+            end = its_pair * next.stages_in_k + next.stages_in_k * (its_slice + 1) / next.splits;
+        } else {
+            first = share_begin(next.units, other, next.ctas);
+            end = share_begin(next.units, other + 1, next.ctas);
+        }
+        const int count = min(kWeightStages, end - first);
+        int next_pair = first / next.stages_in_k;
+        int next_stage = first - next_pair * next.stages_in_k;
+        for (int i = 0; i < count; ++i) {
+#pragma unroll
+            for (int t = 0; t < kTiles; ++t) {
+                const int row0 = next.swiglu ? next_pair * kTileRows : (next_pair * kTiles + t) * kTileRows;
+                if (row0 < next.out_features) {
+                    tma_box_prefetch_l2(t == 1 ? &map1 : &map0, next_stage * kBoxRowBytes, row0);
+                    if (next.nvfp4) {
+                        bulk_prefetch_l2(next.scales[t] + (static_cast<size_t>(row0 >> 7) * next.group_blocks +
+                                                             4 * next_stage) * 512,
+                                         kScaleStageBytes);
+                    }
+                }
+            }
+            if (++next_stage == next.stages_in_k) {
+                next_stage = 0;
+                ++next_pair;
+            }
+        }
+    }
+}
+
 // Sums `count` pieces of a tile pair into this warp's stash (shared memory), in the fixed order
 // first + 1, first + 2, .., last, first (the first piece comes last because its owner is the one who
 // usually finishes the sum, with that piece still on chip).  The piece of CTA `own` (-1: none) is
@@ -315,6 +355,14 @@ __device__ __forceinline__ void sum_pieces_to_stash(const float* partials, int u
         }
     }
 }
+
+}  // namespace
+}  // namespace qwc
+
+#include "nvfp4_native.cuh"
+
+namespace qwc {
+namespace {
 
 template <bool kFp8, bool kSwiglu, int kPad, bool kSplitOut>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -581,40 +629,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         QWC_TRACE_LANE0(7);  // last stage requested
         if (ok && p.next.valid && elect_one()) {
-            // the first stages of the shares of the launch that follows, dealt over this launch's CTAs
-            for (int other = cta; other < p.next.ctas; other += ctas) {
-                int first, end;
-                if (p.next.splits > 0) {
-                    const int its_pair = other / p.next.splits;
-                    const int its_slice = other - its_pair * p.next.splits;
-                    first = its_pair * p.next.stages_in_k + p.next.stages_in_k * its_slice / p.next.splits;
-                    end = its_pair * p.next.stages_in_k + p.next.stages_in_k * (its_slice + 1) / p.next.splits;
-                } else {
-                    first = share_begin(p.next.units, other, p.next.ctas);
-                    end = share_begin(p.next.units, other + 1, p.next.ctas);
-                }
-                const int count = min(kWeightStages, end - first);
-                int next_pair = first / p.next.stages_in_k;
-                int next_stage = first - next_pair * p.next.stages_in_k;
-                for (int i = 0; i < count; ++i) {
-#pragma unroll
-                    for (int t = 0; t < kTiles; ++t) {
-                        const int row0 = p.next.swiglu ? next_pair * kTileRows : (next_pair * kTiles + t) * kTileRows;
-                        if (row0 < p.next.out_features) {
-                            tma_box_prefetch_l2(t == 1 ? &next_map1 : &next_map0, next_stage * kBoxRowBytes, row0);
-                            if (p.next.nvfp4) {
-                                bulk_prefetch_l2(p.next.scales[t] + (static_cast<size_t>(row0 >> 7) * p.next.group_blocks +
-                                                                     4 * next_stage) * 512,
-                                                 kScaleStageBytes);
-                            }
-                        }
-                    }
-                    if (++next_stage == p.next.stages_in_k) {
-                        next_stage = 0;
-                        ++next_pair;
-                    }
-                }
-            }
+            prefetch_next_launch(p.next, next_map0, next_map1, cta, ctas);
         }
     } else if (warp < kXWarp) {
         // ---------------- tensor-core issue ----------------
@@ -1304,6 +1319,37 @@ LaunchShape shape_of(int out_features, int in_features, bool swiglu, bool fp8, b
     return shape;
 }
 
+// The caller's hint about the projection that follows (one use).
+void take_hint(StreamKParams& p, CUtensorMap& next_map0, CUtensorMap& next_map1) {
+    p.next.valid = 0;
+    const NextProjection hint = take_next_projection();
+    if (hint.packed[0] != nullptr && hint.out_features > 0 && hint.in_features > 0) {
+        const bool next_fp8 = hint.kind == 2;
+        const bool next_swiglu = hint.kind == 1 || hint.kind == 4;
+        const int next_row_bytes = next_fp8 ? hint.in_features : hint.in_features / 2;
+        // kinds 3 and 4: a matrix / a SwiGLU pair that will run as a regular K split (qwc_nvfp4_w4a16_split,
+        // the latency-mode projections)
+        const LaunchShape next =
+            shape_of(hint.out_features, hint.in_features, next_swiglu, next_fp8, hint.kind == 3 || hint.kind == 4);
+        if (next.units > 0 &&
+            encode_weight_map(&next_map0, hint.packed[0], hint.out_features, next_row_bytes) == cudaSuccess &&
+            encode_weight_map(&next_map1, hint.packed[next_swiglu ? 1 : 0], hint.out_features, next_row_bytes) ==
+                cudaSuccess) {
+            p.next.valid = 1;
+            p.next.swiglu = next_swiglu ? 1 : 0;
+            p.next.nvfp4 = next_fp8 ? 0 : 1;
+            p.next.out_features = hint.out_features;
+            p.next.ctas = next.ctas;
+            p.next.units = next.units;
+            p.next.splits = next.splits;
+            p.next.stages_in_k = next.stages_in_k;
+            p.next.group_blocks = hint.in_features / 64;
+            p.next.scales[0] = static_cast<const uint8_t*>(hint.scales[0]);
+            p.next.scales[1] = static_cast<const uint8_t*>(hint.scales[next_swiglu ? 1 : 0]);
+        }
+    }
+}
+
 cudaError_t launch_streamk(StreamKParams p, const void* packed0, const void* packed1, bool swiglu, bool fp8,
                            void* workspace, cudaStream_t stream) {
     const bool split_out = p.split_out != nullptr || (p.exchange.ranks > 0 && !fp8);
@@ -1352,35 +1398,8 @@ cudaError_t launch_streamk(StreamKParams p, const void* packed0, const void* pac
         (void)take_next_projection();
         return opted == nullptr ? cudaErrorInvalidDevice : *opted;
     }
-    // The caller's hint about the projection that follows (one use).
     CUtensorMap next_map0 = map0, next_map1 = map1;
-    p.next.valid = 0;
-    const NextProjection hint = take_next_projection();
-    if (hint.packed[0] != nullptr && hint.out_features > 0 && hint.in_features > 0) {
-        const bool next_fp8 = hint.kind == 2;
-        const bool next_swiglu = hint.kind == 1 || hint.kind == 4;
-        const int next_row_bytes = next_fp8 ? hint.in_features : hint.in_features / 2;
-        // kinds 3 and 4: a matrix / a SwiGLU pair that will run as a regular K split (qwc_nvfp4_w4a16_split,
-        // the latency-mode projections)
-        const LaunchShape next =
-            shape_of(hint.out_features, hint.in_features, next_swiglu, next_fp8, hint.kind == 3 || hint.kind == 4);
-        if (next.units > 0 &&
-            encode_weight_map(&next_map0, hint.packed[0], hint.out_features, next_row_bytes) == cudaSuccess &&
-            encode_weight_map(&next_map1, hint.packed[next_swiglu ? 1 : 0], hint.out_features, next_row_bytes) ==
-                cudaSuccess) {
-            p.next.valid = 1;
-            p.next.swiglu = next_swiglu ? 1 : 0;
-            p.next.nvfp4 = next_fp8 ? 0 : 1;
-            p.next.out_features = hint.out_features;
-            p.next.ctas = next.ctas;
-            p.next.units = next.units;
-            p.next.splits = next.splits;
-            p.next.stages_in_k = next.stages_in_k;
-            p.next.group_blocks = hint.in_features / 64;
-            p.next.scales[0] = static_cast<const uint8_t*>(hint.scales[0]);
-            p.next.scales[1] = static_cast<const uint8_t*>(hint.scales[next_swiglu ? 1 : 0]);
-        }
-    }
+    take_hint(p, next_map0, next_map1);
     p.status = status_ptr();
     if (p.status == nullptr) {
         return cudaErrorInvalidValue;
@@ -1401,6 +1420,115 @@ cudaError_t launch_streamk(StreamKParams p, const void* packed0, const void* pac
     config.numAttrs = 1;
     return cudaLaunchKernelEx(&config, kernel, map0, map1, next_map0, next_map1, p);
 }
+
+}  // namespace
+
+// bf16 rows in, bf16 rows out, at most kNativeRows of them (the reference's signature; see nvfp4_gemv.cu).
+cudaError_t launch_nvfp4_native(const void* packed0, const void* scales0, const void* packed1, const void* scales1,
+                                const __nv_bfloat16* x, __nv_bfloat16* y, int out_features, int in_features, int batch,
+                                float inverse_scale0, float inverse_scale1, bool swiglu, cudaStream_t stream) {
+    StreamKParams p = {};
+    p.scales[0] = static_cast<const uint8_t*>(scales0);
+    p.scales[1] = static_cast<const uint8_t*>(swiglu ? scales1 : scales0);
+    p.x_rows = x;
+    p.y = y;
+    p.inverse_scale[0] = inverse_scale0;
+    p.inverse_scale[1] = inverse_scale1;
+    p.out_features = out_features;
+    p.in_features = in_features;
+    p.batch = batch;
+    using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
+                            const StreamKParams);
+    static const Kernel kernels[2] = {nvfp4_native_kernel<false>, nvfp4_native_kernel<true>};
+    struct Setup {
+        cudaError_t opted;
+        int clusters[9];  // of each size, resident at once (a cluster must sit inside one GPC)
+    };
+    static PerDevice<Setup> setup_per_device;
+    const Setup* setup = setup_per_device.get([]() {
+        Setup s = {};
+        for (const Kernel kernel : kernels) {
+            s.opted = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNativeSmemBytes);
+            if (s.opted != cudaSuccess) {
+                return s;
+            }
+        }
+        s.clusters[1] = sm_count_streamk();
+        for (int size = 2; size <= 8; ++size) {
+            cudaLaunchConfig_t probe = {};
+            probe.gridDim = dim3(size * 64);
+            probe.blockDim = dim3(kNativeThreads);
+            probe.dynamicSmemBytes = kNativeSmemBytes;
+            cudaLaunchAttribute attribute[1];
+            attribute[0].id = cudaLaunchAttributeClusterDimension;
+            attribute[0].val.clusterDim.x = size;
+            attribute[0].val.clusterDim.y = 1;
+            attribute[0].val.clusterDim.z = 1;
+            probe.attrs = attribute;
+            probe.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&s.clusters[size], kernels[0], &probe) != cudaSuccess) {
+                s.clusters[size] = 0;
+                (void)cudaGetLastError();
+            }
+        }
+        return s;
+    });
+    if (setup == nullptr || setup->opted != cudaSuccess) {
+        (void)take_next_projection();
+        return setup == nullptr ? cudaErrorInvalidDevice : setup->opted;
+    }
+    const int rows_per_pair = swiglu ? kTileRows : kTiles * kTileRows;
+    p.pair_tiles = (out_features + rows_per_pair - 1) / rows_per_pair;
+    p.stages_in_k = in_features / (kChunkK * kStageChunks);
+    p.units = p.pair_tiles * p.stages_in_k;
+    // Stages one after the other on the busiest SM, plus what a wave costs beside its stages and a
+    // cluster beside its slices (in stages).
+    p.splits = 1;
+    double best = 1e30;
+    for (int size = 1; size <= 8 && size <= p.stages_in_k; ++size) {
+        if (setup->clusters[size] <= 0) {
+            continue;
+        }
+        const int waves = (p.pair_tiles + setup->clusters[size] - 1) / setup->clusters[size];
+        const double cost = waves * ((p.stages_in_k + size - 1) / size + 3.0) + (size > 1 ? 1.0 : 0.0) + 0.2 * size;
+        if (cost < best) {
+            best = cost;
+            p.splits = size;
+        }
+    }
+    CUtensorMap map0, map1;
+    cudaError_t encoded = encode_weight_map(&map0, packed0, out_features, in_features / 2);
+    if (encoded == cudaSuccess) {
+        encoded = encode_weight_map(&map1, swiglu ? packed1 : packed0, out_features, in_features / 2);
+    }
+    if (encoded != cudaSuccess) {
+        (void)take_next_projection();
+        return encoded;
+    }
+    CUtensorMap next_map0 = map0, next_map1 = map1;
+    take_hint(p, next_map0, next_map1);
+    p.status = status_ptr();
+    if (p.status == nullptr) {
+        return cudaErrorInvalidValue;
+    }
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(p.pair_tiles * p.splits);
+    config.blockDim = dim3(kNativeThreads);
+    config.dynamicSmemBytes = kNativeSmemBytes;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[0].val.programmaticStreamSerializationAllowed = 1;
+    attributes[1].id = cudaLaunchAttributeClusterDimension;
+    attributes[1].val.clusterDim.x = p.splits;
+    attributes[1].val.clusterDim.y = 1;
+    attributes[1].val.clusterDim.z = 1;
+    config.attrs = attributes;
+    config.numAttrs = p.splits > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&config, kernels[swiglu ? 1 : 0], map0, map1, next_map0, next_map1, p);
+}
+
+namespace {
 
 bool aligned16(const void* pointer) { return (reinterpret_cast<uintptr_t>(pointer) & 15) == 0; }
 

@@ -767,3 +767,54 @@ def test_page_table_apply_edits(cuda, ops):
     assert host(seq_tokens).tolist() == [0, 0, 17, 6, 0]
     assert host(seq_blocks)[2].tolist() == [9, 4, 0, 0]
     assert abi.lib.qwc_page_table_apply(0, 0, 0, 1, capacity, max_blocks, 0) == abi.CUDA_ERROR_INVALID_VALUE
+
+
+# ---------------------------------------------------------------------------------------
+# NVFP4 projections with both operands in four bits (at most eight rows, large matrices)
+# ---------------------------------------------------------------------------------------
+
+@pytest.mark.parametrize("out_features,in_features,batch", [(5128, 4096, 1), (5120, 4096, 2), (5120, 4096, 3),
+                                                            (1040, 17408, 5), (5120, 4096, 8), (34816, 512, 7)])
+@pytest.mark.parametrize("std", [1.0, 3000.0, 1e-3], ids=["unit", "large", "small"])
+def test_four_bit_projection_matches_oracle(cuda, ops, out_features, in_features, batch, std):
+    """Every padding of the activation rows, ragged last tiles, one and several K slices, block scales of
+    either sign, blocks whose activations differ by nine orders of magnitude, and saturation at 65504."""
+    torch = cuda
+    packed, scales, _ = synth.nvfp4_matrix(41, "four_bit", out_features, in_features)
+    flip = synth.generator(41, "signs").random(scales.shape) < 0.02
+    scales = np.where(flip, scales | 0x80, scales).astype(np.uint8)
+    swizzled = synth.swizzle_block_scales(scales, out_features, in_features)
+    values = synth.bf16_value(synth.normal_bf16(41, "four_bit.x", (batch, in_features), std=std)).copy()
+    values[:, 5::64] *= 30.0
+    values[:, 7::64] *= 1e-6
+    values[:, 256:512] = 0.0
+    x = synth.bf16_bits(np.clip(values, -65280.0, 65280.0))
+    want = oracle.gemv_w4a16(packed, scales, 2.0, x, out_features, in_features, batch)
+    linear = ops.Linear(dev(torch, packed), dev(torch, swizzled), 2.0, out_features, in_features)
+    out = bf16_out(torch, batch, out_features)
+    linear.forward_w4a16(dev(torch, x), out, batch)
+    torch.cuda.synchronize()
+    clean = host(out).copy()
+    assert_rms_close(synth.bf16_value(clean), want, "four-bit projection")
+    poisoned = x.copy()
+    poisoned[batch - 1, 17] = 0x7FC0  # a NaN stays in its row
+    linear.forward_w4a16(dev(torch, poisoned), out, batch)
+    torch.cuda.synchronize()
+    assert np.isnan(synth.bf16_value(host(out))[batch - 1]).all()
+    assert np.array_equal(host(out)[: batch - 1], clean[: batch - 1])
+
+
+def test_four_bit_swiglu_matches_oracle(cuda, ops):
+    torch = cuda
+    out_features, in_features, batch = 3336, 5120, 6
+    gate, gate_scales, gate_swizzled = synth.nvfp4_matrix(42, "gate", out_features, in_features)
+    up, up_scales, up_swizzled = synth.nvfp4_matrix(42, "up", out_features, in_features)
+    x = synth.normal_bf16(42, "swiglu.x", (batch, in_features))
+    want = oracle.swiglu_combine(oracle.gemv_w4a16(gate, gate_scales, 10.0, x, out_features, in_features, batch),
+                                 oracle.gemv_w4a16(up, up_scales, 12.0, x, out_features, in_features, batch))
+    out = bf16_out(torch, batch, out_features)
+    ops.swiglu_w4a16(ops.Linear(dev(torch, gate), dev(torch, gate_swizzled), 10.0, out_features, in_features),
+                     ops.Linear(dev(torch, up), dev(torch, up_swizzled), 12.0, out_features, in_features),
+                     dev(torch, x), out, batch)
+    torch.cuda.synchronize()
+    assert_rms_close(synth.bf16_value(host(out)), want, "four-bit SwiGLU")
