@@ -12,15 +12,12 @@
 //     memory by bulk-async copies (TMA 1-D) in 4 KiB quarters, each signalling its own
 //     mbarrier, so the first rows are processed while the rest are in flight, and the
 //     requantised tile leaves by one bulk store;
-//   * the two dot products of a row run on the integer tensor cores: the codes are s8 already, and k
-//     and q enter as four s8 digits each of a 31-bit fixed-point number (one binary exponent per
-//     vector), so that one m16n8k32 instruction multiplies 16 rows by all eight digit columns.  The
-//     sums are exact in s32 and are rounded once, when the digits are put together: closer to the
-//     real product than the fp32 chain that rounds each of its 128 steps;
-//   * the update: eight lanes share a row (16 codes each) when the grid is deep enough to keep seven CTAs
-//     per SM resident - their warps hide the dependent-instruction latency that bounds the kernel
-//     beside its issue slots - and four lanes (32 codes each) when all CTAs fit the SMs at four each
-//     (kernel_for);
+//   * a lane owns one or two groups of 16 codes of a row (one 16-byte shared-memory access each) and keeps
+//     its elements of k and q in registers for all rows of the tile.  Eight lanes share a row when the grid
+//     is deep enough to keep seven CTAs per SM resident (112 KiB of state in flight per SM): the kernel is
+//     bound by dependent-instruction latency, and the warps of more resident CTAs are what hides it.  Four
+//     lanes share one when every CTA is resident at once anyway: half as many dependent steps per warp
+//     (kernel_for).  Both forms take every sum in the same order, so their results are the same bits;
 //   * the elementwise fp32 work uses the packed f32x2 pipe, and both int8 <-> fp32
 //     conversions are bit tricks on the 2^23 binade (exact, round-to-nearest-even),
 //     which keeps the instruction count under what the memory stream allows.
@@ -39,55 +36,6 @@ constexpr int kPartRows = 32;        // rows per bulk copy / per CTA iteration
 constexpr int kMaxParts = kDim / kPartRows;
 
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
-
-// D[16 rows][8] += A[16][32] (s8, row major) x B[32][8] (s8, column major), exact in s32.
-__device__ __forceinline__ void mma_s8_16832(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// Fixed point is for vectors whose largest magnitude lies in [2^-90, 2^91) (or that are all zero);
-// anything else - infinities and NaN among it - takes the fp32 sums of dots_fp32.
-constexpr uint32_t kFixedLowest = 37u << 23;
-constexpr uint32_t kFixedBeyond = 218u << 23;
-
-__device__ __forceinline__ bool fixed_point_fits(uint32_t peak_bits) {
-    return peak_bits == 0u || (peak_bits >= kFixedLowest && peak_bits < kFixedBeyond);
-}
-
-// x as a multiple of 2^(E - 30), E the exponent with peak < 2^E, in four balanced s8 digits (byte j
-// counts 256^j).
-__device__ __forceinline__ uint32_t fixed_digits(float x, uint32_t peak_bits) {
-    const float up = peak_bits == 0u ? 0.0f : __uint_as_float((283u - (peak_bits >> 23)) << 23);
-    return (static_cast<uint32_t>(__float2int_rn(x * up)) + 0x00808080u) ^ 0x00808080u;
-}
-
-__device__ __forceinline__ float fixed_unit(uint32_t peak_bits) {
-    return peak_bits == 0u ? 0.0f : __uint_as_float(((peak_bits >> 23) - 29u) << 23);
-}
-
-// Row . k and row . q in fp32 for vectors outside the fixed-point range: four lanes per row.
-__device__ __noinline__ float2 dots_fp32(const uint8_t* row, float scale, const float* k, const float* q, int t) {
-    float u = 0.0f, w = 0.0f;
-#pragma unroll 1
-    for (int i = t; i < kDim; i += 4) {
-        const float s = static_cast<float>(static_cast<int8_t>(row[i])) * scale;
-        u = fmaf(s, k[i], u);
-        w = fmaf(s, q[i], w);
-    }
-#pragma unroll
-    for (int offset = 1; offset < 4; offset <<= 1) {
-        u += __shfl_xor_sync(0xffffffffu, u, offset);
-        w += __shfl_xor_sync(0xffffffffu, w, offset);
-    }
-    return make_float2(u, w);
-}
-
-__device__ __forceinline__ float max3_magnitude(float2 s, float peak) {
-    return fmaxf(fmaxf(fabsf(s.x), fabsf(s.y)), peak);
-}
 
 // What the fused output stage needs (the gated RMSNorm of cuda/delta_output.cu:20-64 on this CTA's head,
 // staged for the output projection); `staged == nullptr`: no fusion, `out` is written instead.
@@ -110,9 +58,7 @@ struct GatedNorm {
 // wait for the preceding kernel (which produces q, k, v and the gates).  Callers outside a step, who
 // may have written slots or state just before on the same stream, get the conservative order.
 //
-// `kLanes`: lanes that share a row in the update.  Eight: 16 elements each, 66 registers, seven CTAs per
-// SM.  Four: 32 elements each, 105 registers, four CTAs per SM, but a third fewer instructions and half
-// as many dependent steps per warp (see kernel_for).
+// `kLanes`: lanes that share a row, eight (16 elements of it each) or four (32 each); see kernel_for.
 template <bool kEarly, int kLanes>
 __global__ void __launch_bounds__(kThreads, kLanes == 8 ? 7 : 4) delta_decode_int8_kernel(
     int8_t* __restrict__ state, float* __restrict__ state_scales, const uint32_t* __restrict__ state_slots,
@@ -120,37 +66,24 @@ __global__ void __launch_bounds__(kThreads, kLanes == 8 ? 7 : 4) delta_decode_in
     const float* __restrict__ alpha, const float* __restrict__ beta, const float* __restrict__ kq,
     float* __restrict__ out, int v_heads, int state_capacity, int* status, const GatedNorm norm) {
     pdl_launch_dependents();
-    __shared__ __align__(128) uint8_t tile[kDim * kDim];
-    __shared__ __align__(16) float row_scale[kDim];
-    __shared__ float out_rows[kDim];
-    __shared__ float change_rows[kDim];  // eight lanes: c of every row
-    __shared__ __align__(16) float v_rows[kDim];
-    __shared__ __align__(16) uint32_t digits[2][kDim];  // k and q in fixed point
-    __shared__ uint32_t peaks[2][kThreads / 32];
-    __shared__ uint32_t b_words[kLanes == 8 ? 1 : 8][32];  // B fragments: [word of the lane's codes][lane]
-    __shared__ uint64_t bars[kMaxParts];
-    __shared__ int failed;
-
-    const int rows_here = kDim / gridDim.z;
-    const int parts = (rows_here + kPartRows - 1) / kPartRows;
-    const int part_rows = rows_here < kPartRows ? rows_here : kPartRows;
-    if (threadIdx.x == 0) {
-        failed = 0;
-        for (int part = 0; part < parts; ++part) {
-            mbar_init(&bars[part], 1);
-        }
-        mbar_fence_init();
-    }
     if (!kEarly) {
         pdl_wait();
     }
-    const int h = blockIdx.x;
-    const int b = blockIdx.y;
-    const int row_begin = blockIdx.z * rows_here;
-    const int slot = state_slots == nullptr ? b : static_cast<int>(state_slots[b]);
-    if (status_is_set(status)) {  // (after the slot was asked for: one round trip for both)
+    __shared__ __align__(128) uint8_t tile[kDim * kDim];
+    __shared__ __align__(16) float row_scale[kDim];
+    __shared__ float out_rows[kDim];
+    __shared__ __align__(16) float v_rows[kDim];
+    __shared__ uint64_t bars[kMaxParts];
+    __shared__ int failed;
+
+    if (status_is_set(status)) {
         return;
     }
+    const int h = blockIdx.x;
+    const int b = blockIdx.y;
+    const int rows_here = kDim / gridDim.z;
+    const int row_begin = blockIdx.z * rows_here;
+    const int slot = state_slots == nullptr ? b : static_cast<int>(state_slots[b]);
     if (static_cast<uint32_t>(slot) >= static_cast<uint32_t>(state_capacity)) {
         // a slot beyond the pool: nothing of this row is read or written, the host learns of it
         // through the status word (the whole CTA takes this branch: the slot is per row)
@@ -160,11 +93,20 @@ __global__ void __launch_bounds__(kThreads, kLanes == 8 ? 7 : 4) delta_decode_in
         return;
     }
     const int hk = h / (v_heads / kDeltaKeyHeads);
+    const int parts = (rows_here + kPartRows - 1) / kPartRows;
+    const int part_rows = rows_here < kPartRows ? rows_here : kPartRows;
 
     int8_t* S = state + (static_cast<size_t>(slot) * v_heads + h) * (kDim * kDim) + row_begin * kDim;
     float* scales = state_scales + (static_cast<size_t>(slot) * v_heads + h) * kDim + row_begin;
 
-    // the thread that set the barriers up is the one that uses them here
+    if (threadIdx.x == 0) {
+        failed = 0;
+        for (int part = 0; part < parts; ++part) {
+            mbar_init(&bars[part], 1);
+        }
+        mbar_fence_init();
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
         for (int part = 0; part < parts; ++part) {
             const uint32_t bytes = part_rows * kDim;
@@ -178,156 +120,66 @@ __global__ void __launch_bounds__(kThreads, kLanes == 8 ? 7 : 4) delta_decode_in
     if (kEarly) {
         pdl_wait();  // q, k, v and the gates come from the preceding kernel
     }
+    for (int i = threadIdx.x; i < rows_here; i += kThreads) {
+        v_rows[i] = v[(static_cast<size_t>(b) * v_heads + h) * kDim + row_begin + i];
+    }
+    __syncthreads();
+
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const float* k_head = k + (static_cast<size_t>(b) * kDeltaKeyHeads + hk) * kDim;
-    const float* q_head = q + (static_cast<size_t>(b) * kDeltaKeyHeads + hk) * kDim;
-    const float my_k = k_head[threadIdx.x];  // a thread per element of the key head
-    const float my_q = q_head[threadIdx.x];
-    const int g = lane >> 2;  // row of an eight
-    const int t = lane & 3;   // the lane's columns of the row: 16 t .. + 15 and 64 + 16 t .. + 15
-    // eight lanes: the lane's columns in the update are 16 sub .. + 15
-    const int sub = lane & 7;
-    const int row_in_warp = lane >> 3;
-    float2 kk[64 / kLanes];
+    constexpr int kGroups = 8 / kLanes;       // groups of 16 columns per lane: 16 (sub + kLanes g) .. + 15
+    constexpr int kRowsPerWarp = 32 / kLanes;  // rows a warp works on at once
+    const int sub = lane & (kLanes - 1);
+    const int row_in_warp = lane / kLanes;
+
+    float2 kk[8 * kGroups], qq[8 * kGroups];
 #pragma unroll
-    for (int i = 0; i < 32 / kLanes; ++i) {
-        const int column = kLanes == 8 ? 16 * sub + 4 * i : 64 * (i >> 2) + 16 * t + 4 * (i & 3);
-        const float4 kv = *reinterpret_cast<const float4*>(k_head + column);
-        kk[2 * i] = f2(kv.x, kv.y);
-        kk[2 * i + 1] = f2(kv.z, kv.w);
-    }
-    if (threadIdx.x < rows_here) {
-        v_rows[threadIdx.x] = v[(static_cast<size_t>(b) * v_heads + h) * kDim + row_begin + threadIdx.x];
+    for (int g = 0; g < kGroups; ++g) {
+        const size_t first = (static_cast<size_t>(b) * kDeltaKeyHeads + hk) * kDim + 16 * (sub + kLanes * g);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 kv = *reinterpret_cast<const float4*>(k + first + 4 * i);
+            const float4 qv = *reinterpret_cast<const float4*>(q + first + 4 * i);
+            kk[8 * g + 2 * i] = f2(kv.x, kv.y);
+            kk[8 * g + 2 * i + 1] = f2(kv.z, kv.w);
+            qq[8 * g + 2 * i] = f2(qv.x, qv.y);
+            qq[8 * g + 2 * i + 1] = f2(qv.z, qv.w);
+        }
     }
     const float a = alpha[static_cast<size_t>(b) * v_heads + h];
     const float bt = beta[static_cast<size_t>(b) * v_heads + h];
     const float kq_token = kq[static_cast<size_t>(b) * kDeltaKeyHeads + hk];
 
-    const uint32_t k_peak_warp = __reduce_max_sync(0xffffffffu, __float_as_uint(my_k) & 0x7fffffffu);
-    const uint32_t q_peak_warp = __reduce_max_sync(0xffffffffu, __float_as_uint(my_q) & 0x7fffffffu);
-    if (lane == 0) {
-        peaks[0][warp] = k_peak_warp;
-        peaks[1][warp] = q_peak_warp;
-    }
-    __syncthreads();
-    uint32_t k_peak = 0, q_peak = 0;  // the largest magnitudes as bits: ordered like the magnitudes, NaN above all
-#pragma unroll
-    for (int i = 0; i < kThreads / 32; ++i) {
-        k_peak = max(k_peak, peaks[0][i]);
-        q_peak = max(q_peak, peaks[1][i]);
-    }
-    const bool fixed = fixed_point_fits(k_peak) && fixed_point_fits(q_peak);
-    if (fixed) {
-        digits[0][threadIdx.x] = fixed_digits(my_k, k_peak);
-        digits[1][threadIdx.x] = fixed_digits(my_q, q_peak);
-    }
-    __syncthreads();
-
-    // B fragments: column g is digit g & 3 of k (g < 4) or q.  The contraction is over columns in the
-    // order in which a lane holds its codes: chunk c of lane t is columns 16 (4 c + t) .. + 15.
-    // Eight lanes: every warp gathers all of them for itself.  Four lanes have no registers to keep them
-    // in: a warp gathers a quarter of them for all.
-    uint32_t b_own[8];
-    {
-        const uint32_t pick = (g & 3) | ((4 + (g & 3)) << 4);
-        const auto gather = [&](int word) {
-            const uint4 four =
-                *reinterpret_cast<const uint4*>(digits[g >> 2] + 16 * (4 * (word >> 2) + t) + 4 * (word & 3));
-            return __byte_perm(__byte_perm(four.x, four.y, pick), __byte_perm(four.z, four.w, pick), 0x5410);
-        };
-        if constexpr (kLanes == 8) {
-#pragma unroll
-            for (int word = 0; word < 8; ++word) {
-                b_own[word] = gather(word);
-            }
-        } else {
-            b_words[2 * warp][lane] = gather(2 * warp);
-            b_words[2 * warp + 1][lane] = gather(2 * warp + 1);
-            __syncthreads();
-        }
-    }
-    const auto b_word = [&](int word) { return kLanes == 8 ? b_own[word] : b_words[word][lane]; };
-    const float unit = fixed_unit(t < 2 ? k_peak : q_peak) * ((t & 1) ? 65536.0f : 1.0f);
-
     constexpr float kMagic = 12582912.0f;        // 1.5 * 2^23
     constexpr float kMagicBiased = 12583040.0f;  // kMagic + 128
 
-    // A warp takes 16 rows at a time: rows 16 warp .. of the first 64, then of the last 64.
-    for (int first = 16 * warp; first < rows_here; first += 16 * (kThreads / 32)) {
+    for (int part = 0; part < parts; ++part) {
         // a warp leaves as a whole: the row reductions below are full-warp shuffles
-        const bool arrived = __all_sync(
-            0xffffffffu, mbar_wait_bounded(&bars[first / kPartRows], 0, kStatusDeltaTileWait, status) &&
-                             (first < kPartRows || mbar_wait_bounded(&bars[0], 0, kStatusDeltaTileWait, status)));
+        const bool arrived =
+            __all_sync(0xffffffffu, mbar_wait_bounded(&bars[part], 0, kStatusDeltaTileWait, status));
         if (!arrived) {
             failed = 1;
             break;
         }
-        // rows g and g + 8 of the sixteen; the second eight are absent when the split leaves eight rows
-        const int row_lo = first + g;
-        const int row_hi = min(first + g + 8, rows_here - 1);
-        float u[2], w[2];
-        if (fixed) {
-            int sums[4] = {0, 0, 0, 0};
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const uint4 lo = *reinterpret_cast<const uint4*>(tile + row_lo * kDim + 16 * (4 * c + t));
-                const uint4 hi = *reinterpret_cast<const uint4*>(tile + row_hi * kDim + 16 * (4 * c + t));
-                const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y};
-                const uint32_t a1[4] = {lo.z, hi.z, lo.w, hi.w};
-                mma_s8_16832(sums, a0, b_word(4 * c), b_word(4 * c + 1));
-                mma_s8_16832(sums, a1, b_word(4 * c + 2), b_word(4 * c + 3));
-            }
-            // this lane: two digits of k (t < 2) or q, the low two (t even) or the high two
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const float part =
-                    fmaf(static_cast<float>(sums[2 * r + 1]), 256.0f, static_cast<float>(sums[2 * r])) * unit;
-                const float whole = part + __shfl_xor_sync(0xffffffffu, part, 1);
-                const float other = __shfl_xor_sync(0xffffffffu, whole, 2);
-                u[r] = t < 2 ? whole : other;
-                w[r] = t < 2 ? other : whole;
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const int row = r == 0 ? row_lo : row_hi;
-                const float2 both = dots_fp32(tile + row * kDim, row_scale[row], k_head, q_head, t);
-                u[r] = both.x;
-                w[r] = both.y;
-            }
+        if (warp * 8 >= part_rows) {
+            continue;  // whole warp beyond the split's rows
         }
-        if constexpr (kLanes == 8) {
-            if (t < 2) {  // lane t finishes row g (t = 0) or g + 8
-                const int row = t == 0 ? row_lo : row_hi;
-                const float scale = row_scale[row];
-                // (an infinite scale marks a row that has overflowed: its dots are NaN, as 0 * inf is)
-                const float dot_k = fmaf(t == 0 ? u[0] : u[1], fixed ? scale : 1.0f, scale - scale);
-                const float dot_q = fmaf(t == 0 ? w[0] : w[1], fixed ? scale : 1.0f, scale - scale);
-                const float c = bt * (v_rows[row] - a * dot_k);
-                change_rows[row] = c;
-                out_rows[row] = a * dot_q + c * kq_token;
-            }
-            __syncwarp();
+#pragma unroll
+        for (int pass = 0; pass < 8 / kRowsPerWarp; ++pass) {
+            const int local = part * kPartRows + warp * 8 + pass * kRowsPerWarp + row_in_warp;
+            uint8_t* row_ptr = tile + local * kDim + 16 * sub;
+            const float scale = row_scale[local];
+            const float v_row = v_rows[local];
 
-#pragma unroll 1
-            for (int pass = 0; pass < 4; ++pass) {
-                if (first + pass * 4 >= rows_here) {
-                    break;
-                }
-                const int local = first + pass * 4 + row_in_warp;
-                uint8_t* row_ptr = tile + local * kDim + 16 * sub;
-                const uint4 codes = *reinterpret_cast<const uint4*>(row_ptr);
-                const float scale = row_scale[local];
-                const float c = change_rows[local];
-
+            float2 s[8 * kGroups];
+            const float2 bias = f2(-kMagicBiased, -kMagicBiased);
+            const float2 scale2 = f2(scale, scale);
+            float u[kGroups], w[kGroups];
+#pragma unroll
+            for (int g = 0; g < kGroups; ++g) {
+                const uint4 codes = *reinterpret_cast<const uint4*>(row_ptr + 16 * kLanes * g);
                 const uint32_t words[4] = {codes.x, codes.y, codes.z, codes.w};
-                float2 s[8];
-                const float2 bias = f2(-kMagicBiased, -kMagicBiased);
-                const float2 scale2 = f2(scale, scale);
-                const float2 a2 = f2(a, a);
-                const float2 cc = f2(c, c);
-                float peak = 0.0f;
+                float2 u2 = f2(0.0f, 0.0f), w2 = f2(0.0f, 0.0f);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const uint32_t x = words[i] ^ 0x80808080u;
@@ -335,92 +187,65 @@ __global__ void __launch_bounds__(kThreads, kLanes == 8 ? 7 : 4) delta_decode_in
                                          __uint_as_float(__byte_perm(x, 0x4B400000u, 0x7651)));
                     const float2 hi = f2(__uint_as_float(__byte_perm(x, 0x4B400000u, 0x7652)),
                                          __uint_as_float(__byte_perm(x, 0x4B400000u, 0x7653)));
-                    s[2 * i] = __ffma2_rn(cc, kk[2 * i], __fmul2_rn(a2, __fmul2_rn(__fadd2_rn(lo, bias), scale2)));
-                    s[2 * i + 1] = __ffma2_rn(cc, kk[2 * i + 1], __fmul2_rn(a2, __fmul2_rn(__fadd2_rn(hi, bias), scale2)));
-                    peak = max3_magnitude(s[2 * i], peak);
-                    peak = max3_magnitude(s[2 * i + 1], peak);
+                    const int e = 8 * g + 2 * i;
+                    s[e] = __fmul2_rn(__fadd2_rn(lo, bias), scale2);
+                    s[e + 1] = __fmul2_rn(__fadd2_rn(hi, bias), scale2);
+                    u2 = __ffma2_rn(s[e], kk[e], u2);
+                    w2 = __ffma2_rn(s[e], qq[e], w2);
+                    u2 = __ffma2_rn(s[e + 1], kk[e + 1], u2);
+                    w2 = __ffma2_rn(s[e + 1], qq[e + 1], w2);
                 }
+                u[g] = u2.x + u2.y;
+                w[g] = w2.x + w2.y;
+            }
+            // over the four lanes that hold a half of the row, then the two halves
 #pragma unroll
-                for (int offset = 1; offset < 8; offset <<= 1) {
-                    peak = fmaxf(peak, __shfl_xor_sync(0xffffffffu, peak, offset));
+            for (int offset = 1; offset < 4; offset <<= 1) {
+#pragma unroll
+                for (int g = 0; g < kGroups; ++g) {
+                    u[g] += __shfl_xor_sync(0xffffffffu, u[g], offset);
+                    w[g] += __shfl_xor_sync(0xffffffffu, w[g], offset);
                 }
+            }
+            const float dot_k = u[0] + (kLanes == 8 ? __shfl_xor_sync(0xffffffffu, u[0], 4) : u[kGroups - 1]);
+            const float dot_q = w[0] + (kLanes == 8 ? __shfl_xor_sync(0xffffffffu, w[0], 4) : w[kGroups - 1]);
 
-                const float inverse = peak == 0.0f ? 0.0f : __fdiv_rn(127.0f, peak);
-                const float2 inverse2 = f2(inverse, inverse);
-                const float2 magic2 = f2(kMagic, kMagic);
+            const float c = bt * (v_row - a * dot_k);
+            const float contribution = a * dot_q + c * kq_token;
+
+            const float2 a2 = f2(a, a);
+            const float2 cc = f2(c, c);
+            float peak = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8 * kGroups; ++i) {
+                s[i] = __ffma2_rn(cc, kk[i], __fmul2_rn(a2, s[i]));
+                peak = fmaxf(peak, fmaxf(fabsf(s[i].x), fabsf(s[i].y)));
+            }
+#pragma unroll
+            for (int offset = 1; offset < kLanes; offset <<= 1) {
+                peak = fmaxf(peak, __shfl_xor_sync(0xffffffffu, peak, offset));
+            }
+
+            const float inverse = peak == 0.0f ? 0.0f : __fdiv_rn(127.0f, peak);
+            const float2 inverse2 = f2(inverse, inverse);
+            const float2 magic2 = f2(kMagic, kMagic);
+#pragma unroll
+            for (int g = 0; g < kGroups; ++g) {
                 uint32_t packed[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const float2 y0 = __fadd2_rn(__fmul2_rn(s[2 * i], inverse2), magic2);
-                    const float2 y1 = __fadd2_rn(__fmul2_rn(s[2 * i + 1], inverse2), magic2);
+                    const float2 y0 = __fadd2_rn(__fmul2_rn(s[8 * g + 2 * i], inverse2), magic2);
+                    const float2 y1 = __fadd2_rn(__fmul2_rn(s[8 * g + 2 * i + 1], inverse2), magic2);
                     const uint32_t lo = __byte_perm(__float_as_uint(y0.x), __float_as_uint(y0.y), 0x0040);
                     const uint32_t hi = __byte_perm(__float_as_uint(y1.x), __float_as_uint(y1.y), 0x0040);
                     packed[i] = __byte_perm(lo, hi, 0x5410);
                 }
-                *reinterpret_cast<uint4*>(row_ptr) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                if (sub == 0) {
-                    row_scale[local] = __fmul_rn(peak, 1.0f / 127.0f);
-                }
+                *reinterpret_cast<uint4*>(row_ptr + 16 * kLanes * g) =
+                    make_uint4(packed[0], packed[1], packed[2], packed[3]);
             }
-        } else {
-#pragma unroll 1
-            for (int r = 0; r < 2; ++r) {
-                const int local = r == 0 ? row_lo : row_hi;
-                const float scale = row_scale[local];
-                // (an infinite scale marks a row that has overflowed: its dots are NaN, as 0 * inf is)
-                const float dot_k = fmaf(r == 0 ? u[0] : u[1], fixed ? scale : 1.0f, scale - scale);
-                const float dot_q = fmaf(r == 0 ? w[0] : w[1], fixed ? scale : 1.0f, scale - scale);
-                const float c = bt * (v_rows[local] - a * dot_k);
-                const float contribution = a * dot_q + c * kq_token;
-                uint8_t* const at = tile + local * kDim + 16 * t;
-                const uint4 first_codes = *reinterpret_cast<const uint4*>(at);
-                const uint4 second_codes = *reinterpret_cast<const uint4*>(at + 64);
-                const uint32_t words[8] = {first_codes.x,  first_codes.y,  first_codes.z,  first_codes.w,
-                                           second_codes.x, second_codes.y, second_codes.z, second_codes.w};
-                float2 s[16];
-                const float2 bias = f2(-kMagicBiased, -kMagicBiased);
-                const float2 scale2 = f2(scale, scale);
-                const float2 a2 = f2(a, a);
-                const float2 cc = f2(c, c);
-                float peak_a = 0.0f, peak_b = 0.0f;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const uint32_t x = words[i] ^ 0x80808080u;
-                    const float2 lo = f2(__uint_as_float(__byte_perm(x, 0x4B400000u, 0x7650)),
-                                         __uint_as_float(__byte_perm(x, 0x4B400000u, 0x7651)));
-                    const float2 hi = f2(__uint_as_float(__byte_perm(x, 0x4B400000u, 0x7652)),
-                                         __uint_as_float(__byte_perm(x, 0x4B400000u, 0x7653)));
-                    s[2 * i] = __ffma2_rn(cc, kk[2 * i], __fmul2_rn(a2, __fmul2_rn(__fadd2_rn(lo, bias), scale2)));
-                    s[2 * i + 1] = __ffma2_rn(cc, kk[2 * i + 1], __fmul2_rn(a2, __fmul2_rn(__fadd2_rn(hi, bias), scale2)));
-                    peak_a = max3_magnitude(s[2 * i], peak_a);
-                    peak_b = max3_magnitude(s[2 * i + 1], peak_b);
-                }
-                float peak = fmaxf(peak_a, peak_b);
-#pragma unroll
-                for (int offset = 1; offset < 4; offset <<= 1) {
-                    peak = fmaxf(peak, __shfl_xor_sync(0xffffffffu, peak, offset));
-                }
-
-                const float inverse = peak == 0.0f ? 0.0f : __fdiv_rn(127.0f, peak);
-                const float2 inverse2 = f2(inverse, inverse);
-                const float2 magic2 = f2(kMagic, kMagic);
-                uint32_t packed[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float2 y0 = __fadd2_rn(__fmul2_rn(s[2 * i], inverse2), magic2);
-                    const float2 y1 = __fadd2_rn(__fmul2_rn(s[2 * i + 1], inverse2), magic2);
-                    const uint32_t lo = __byte_perm(__float_as_uint(y0.x), __float_as_uint(y0.y), 0x0040);
-                    const uint32_t hi = __byte_perm(__float_as_uint(y1.x), __float_as_uint(y1.y), 0x0040);
-                    packed[i] = __byte_perm(lo, hi, 0x5410);
-                }
-                if (first + g + 8 * r < rows_here) {
-                    *reinterpret_cast<uint4*>(at) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                    *reinterpret_cast<uint4*>(at + 64) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                    if (t == 0) {
-                        row_scale[local] = __fmul_rn(peak, 1.0f / 127.0f);
-                        out_rows[local] = contribution;
-                    }
-                }
+            if (sub == 0) {
+                row_scale[local] = __fmul_rn(peak, 1.0f / 127.0f);
+                out_rows[local] = contribution;
             }
         }
     }
@@ -513,7 +338,7 @@ int splits_for(int batch, int v_heads) {
     const int sms = sm_count_delta();
     const int base = v_heads * batch;
     int split = 1;
-    while (split < 8 && base * split < 2 * sms) {
+    while (split < 16 && base * split < 2 * sms) {
         split *= 2;
     }
     return split;
@@ -522,10 +347,10 @@ int splits_for(int batch, int v_heads) {
 using DeltaKernel = void (*)(int8_t*, float*, const uint32_t*, const float*, const float*, const float*, const float*,
                              const float*, const float*, float*, int, int, int*, const GatedNorm);
 
-// Four lanes per row while every CTA is resident at once with them (four per SM), eight beyond.
-// Measured (us, layers that L2 does not hold, four / eight lanes): 48 heads at 1 row 3.54 / 4.62, at 9
-// rows (432 CTAs) 7.7 / 11.1; 32 heads at 32 rows (1024 CTAs, two waves of the first) 13.6 / 12.5.
-// (The fp32 dot products that the integer tensor cores replaced: 4.94, 12.06 and 14.0.)
+// Four lanes per row (123 registers) while every CTA is resident at once with them, four per SM; eight (71
+// registers, seven CTAs per SM) beyond.  Measured (us, layers that L2 does not hold, four / eight lanes): 48
+// heads at 1 row 3.62 / 4.90, at 9 rows (432 CTAs) 8.28 / 12.00, at 12 rows (576) 8.70 / 12.54; 32 heads at 32
+// rows (1024 CTAs, two waves of the first) 14.55 / 13.97.
 template <bool kEarly>
 DeltaKernel kernel_for(int ctas) {
     return ctas <= 4 * sm_count_delta() ? delta_decode_int8_kernel<kEarly, 4> : delta_decode_int8_kernel<kEarly, 8>;

@@ -367,32 +367,64 @@ def test_delta_decode_int8_matches_oracle(cuda, ops, batch, v_heads):
         assert np.array_equal(scales[slot], case["scales"][slot])
 
 
-@pytest.mark.parametrize("batch,v_heads", [(18, 32), (19, 32), (12, 48), (13, 48), (2, 32), (3, 48)],
+@pytest.mark.parametrize("batch,v_heads", [(18, 32), (19, 32), (12, 48), (13, 48), (1, 32), (2, 32), (3, 48)],
                          ids=["last_four_lanes", "first_eight_lanes", "last_four_lanes_h48", "first_eight_lanes_h48",
-                              "row_split_8", "row_split_4"])
-@pytest.mark.parametrize("exponent", [0, -100], ids=["fixed_point", "fp32_sums"])
+                              "row_split_16", "row_split_8", "row_split_4"])
+@pytest.mark.parametrize("exponent", [0, -100, 92], ids=["unit_q", "tiny_q", "huge_q"])
 def test_delta_decode_both_forms(cuda, ops, batch, v_heads, exponent):
-    """On either side of the line between four and eight lanes per row, with row splits, and with a k that
-    the fixed-point sums do not take.  Bounds: out within 1e-5 of its largest value (128 fp32 roundings
-    of 6e-8 in the oracle's sums, one here), codes within one step, where u moves by a unit in the last place."""
+    """On either side of the line between four and eight lanes per row, with row splits, with a key of zeros
+    and with a query at the ends of the fp32 range (a power of two: only `out` scales with it, the update
+    does not see q).  Bounds: out within 1e-5 of its row's largest value (128 fp32 roundings of 6e-8 on either
+    side, in different orders), codes within one step, where row . k moves by a unit in the last place."""
     case = synth.delta_case(11, batch, v_heads)
-    k = case["k"].copy()
+    k, q = case["k"].copy(), case["q"].copy()
     k[0] = 0.0
-    k[1] = np.ldexp(k[1], exponent)
-    case = dict(case, k=k, kq=np.einsum("bhd,bhd->bh", case["q"], k).astype(np.float32))
+    q[batch - 1] = np.ldexp(q[batch - 1], exponent)
+    case = dict(case, k=k, q=q, kq=np.einsum("bhd,bhd->bh", q, k).astype(np.float32))
     want_state, want_scales = case["state"].copy(), case["scales"].copy()
     want_out = oracle.delta_decode_int8(want_state, want_scales, case["slots"], case["q"], case["k"], case["v"],
                                         case["alpha"], case["beta"], case["kq"], batch, v_heads)
     state, scales, out = run_delta(cuda, ops, case, batch, v_heads)
-    assert np.max(np.abs(out - want_out)) <= 1e-5 * np.max(np.abs(want_out))
+    row_peak = np.max(np.abs(want_out), axis=(1, 2), keepdims=True)
+    assert np.all(np.abs(out - want_out) <= 1e-5 * row_peak)
     diff = np.abs(state.astype(np.int32) - want_state.astype(np.int32))
     assert diff.max() <= 1 and np.mean(diff > 0) < 1e-4
     assert np.allclose(scales, want_scales, rtol=1e-5, atol=0)
 
 
+@pytest.mark.parametrize("batch,v_heads", [(3, 32), (19, 32)], ids=["four_lanes", "eight_lanes"])
+@pytest.mark.parametrize("vector", ["k", "q"])
+def test_delta_dot_products_keep_small_elements_beside_an_outlier(cuda, ops, batch, v_heads, vector):
+    """k (then q) holds a 1 where every state row's code is 0, and elements of 1e-5 to 1e-8 elsewhere: the dot
+    product is the sum of the small ones alone.  The other inputs are chosen so that `out` is that dot product
+    times a gate: v = 0 and q the unit vector of the outlier's column (out = -alpha beta row . k), or k = 0
+    (out = alpha row . q).  Bound against float64: one rounding of each state element and at most 24 of the
+    sum (16 in a lane, its two halves, three exchanges, the gates), 2^-24 of the sum of magnitudes each."""
+    case = synth.delta_case(13, batch, v_heads)
+    rng = synth.generator(13, "outlier")
+    column = 77
+    state = case["state"].copy()
+    state[..., column] = 0
+    x = (rng.choice([-1.0, 1.0], (batch, 16, 128)) * 10.0 ** rng.uniform(-8, -5, (batch, 16, 128))).astype(np.float32)
+    x[..., column] = 1.0
+    unit, zero = np.zeros_like(x), np.zeros_like(x)
+    unit[..., column] = 1.0
+    k, q = (x, unit) if vector == "k" else (zero, x)
+    kq = np.full((batch, 16), 1.0 if vector == "k" else 0.0, dtype=np.float32)
+    case = dict(case, state=state, k=k, q=q, kq=kq, v=np.zeros_like(case["v"]))
+    _, _, out = run_delta(cuda, ops, case, batch, v_heads)
+    rows = state[case["slots"]].astype(np.float64) * case["scales"][case["slots"]].astype(np.float64)[..., None]
+    terms = rows * np.repeat(x.astype(np.float64), v_heads // 16, axis=1)[:, :, None, :]
+    gate = case["alpha"].astype(np.float64) * (-case["beta"].astype(np.float64) if vector == "k" else 1.0)
+    want = gate[..., None] * terms.sum(-1)
+    bound = 25 * 2.0 ** -24 * np.abs(gate)[..., None] * np.abs(terms).sum(-1)
+    assert np.all(np.abs(out - want) <= bound)
+
+
+@pytest.mark.parametrize("batch", [3, 19], ids=["four_lanes", "eight_lanes"])
 @pytest.mark.parametrize("value", [np.nan, np.inf])
-def test_delta_non_finite_key_stays_in_its_head(cuda, ops, value):
-    batch, v_heads = 3, 32
+def test_delta_non_finite_key_stays_in_its_head(cuda, ops, value, batch):
+    v_heads = 32
     case = synth.delta_case(12, batch, v_heads)
     k = case["k"].copy()
     k[1, 4, 17] = value
