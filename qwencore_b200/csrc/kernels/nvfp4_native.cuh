@@ -5,10 +5,10 @@
 // What the f16 kernels (nvfp4_umma.cu, nvfp4_streamk.cu) spend their time on at these batches is widening
 // weights: one conversion per two weights keeps the conversion unit 70 % busy, a stage takes as long as
 // its bytes need from HBM, and the stages in the ring are still to be widened when the last byte has
-// landed.  Here nobody touches a weight: a stage is consumed in 0.2 us, the end of the launch follows the
-// last byte, and what bounds the kernel is the weight stream.  Measured (us, bf16 rows in, layers that L2
-// does not hold, before -> now): 34816 x 5120 at one row 24.1 -> 18.4 (5.45 TB/s), 5120 x 17408 16.4 ->
-// 12.8 at one row and 17.1 -> 14.2 at eight, 12352 x 5120 13.3 -> 10.3 and 13.5 -> 11.7.
+// landed.  Here nobody touches a weight: the end of the launch follows the last byte, and what bounds the
+// kernel is the weight stream, between a start and a tail of about 3 us.  Measured (us, bf16 rows in, layers
+// that L2 does not hold, f16 / four bits at one and at eight rows): 34816 x 5120 26.3 / 20.7 (4.9 TB/s) and
+// 24.0 / 22.6, 5120 x 17408 16.5 / 12.9 and 17.0 / 15.1, 12352 x 5120 13.2 / 10.6 and 13.5 / 12.4.
 //
 // Not above eight rows, and not for staged activations inside a decode step: making digits costs about 25
 // instructions per activation in every CTA, after the activations have arrived.  At sixteen rows that
@@ -17,14 +17,18 @@
 // alone went from 3.09 to 2.99 ms).
 //
 // Digits.  The sixteen activations of a block (16 features of one row) share a power of two; each is
-// rounded to 23 bits of fixed point below it, written in balanced base 8 (digits -4 .. 3, which are e2m1
-// values), and digit j of row r becomes column j R + r of the B operand (R: rows padded to a power of
-// two).  The sum over K of every column is an fp32 accumulator of its own, and the epilogue adds the
-// eight with their weights 8^(j - 7).  An activation arrives as f16, eleven significant bits: it is
-// represented exactly unless it is 2^-11 times smaller than the largest of its block, and then within
-// 2^-22 of that largest - the size of one rounding of the fp32 accumulation it goes into.  Measured against
-// float64 (5120 x 4096, N(0, 1)): 2.9e-8 of the result; the f16 kernel, whose weights and activations are
-// exact, 1.4e-7.
+// written as 23 bits of fixed point below it, in balanced base 8 (digits -4 .. 4, which are e2m1 values),
+// and digit j of row r becomes column j R + r of the B operand (R: rows padded to a power of two).  The sum
+// over K of every column is an fp32 accumulator of its own, and the epilogue adds the eight with their
+// weights 8^(j - 7).  An activation arrives as the f16 that the other kernels multiply with, here with the
+// eight significant bits of a bf16: the 23 bits hold it exactly unless it is 2^-14 times smaller than its
+// block's power of two.  A warp that meets such a one (N(0, 1) activations: one warp and stage in thirty)
+// writes what is left of its activations as eight digits more, 2^-23 times smaller, and they are multiplied
+// into accumulators of their own; a launch with such a warp somewhere takes 0.1 to 0.9 us longer, and nobody
+// else pays.  Together they reach from f16's largest to its smallest bit: both operands
+// are exact, as they are in the f16 kernels, and only the sums are rounded.  That can be seen where the exact
+// result is 0 (every block of features twice, with opposite weights, shuffled over K = 4096): outputs of
+// 3.4e-8 of the uncancelled sums, 1.3e-7 on the f16 kernel.
 //
 //   warp 0      weight producer: two boxes of 128 rows x 128 bytes and their scale blocks per stage
 //   warp 1      copies the stage's scales to tensor memory (tcgen05.cp) and issues the MMAs
@@ -43,10 +47,11 @@ constexpr int kNativeDigits = 8;
 constexpr int kNativeWorkerWarps = 8;
 constexpr int kNativeFirstWorker = 4;
 constexpr int kNativeThreads = (kNativeFirstWorker + kNativeWorkerWarps) * 32;
-constexpr int kNativeXBytes = 5 * (kNativeRows * kNativeDigits * 128 + 2048);  // ring of digit tiles
+constexpr int kNativeXBytes = 4 * (2 * kNativeRows * kNativeDigits * 128 + 2048);  // ring of digit tiles
 constexpr int kNativeMaxXSlots = 8;
 constexpr int kNativeSmemBytes = kWeightStages * kTiles * kTileStageBytes + kNativeXBytes + 1024;
-constexpr int kNativeAccumulator = 128;          // columns of one tile's accumulators
+constexpr int kNativeAccumulator = 128;          // columns of one tile's accumulators ...
+constexpr int kNativeRest = 64;                  // ... of which those of the second eight digits start here
 constexpr int kNativeScaleColumn = 256;          // tensor memory behind the accumulators: scales
 constexpr int kNativeScaleColumns = 48;          // of one stage: 16 per tile, 16 for the activations
 
@@ -59,6 +64,8 @@ struct NativeBarriers {
     uint64_t done;
     uint64_t tmem_ready;
     uint32_t tmem_base;
+    uint32_t rest[kNativeMaxXSlots];  // byte w: warp w of the slot's team wrote the second eight digits
+    int rest_used;
     int failed;
 };
 
@@ -128,6 +135,78 @@ __device__ __forceinline__ float native_peer_float(const float* local, int rank)
     return value;
 }
 
+// The 2^23 binade, whose low bits are the integer that was added, and what turns them into the integer plus 4 in
+// every octal digit.
+constexpr float kBinade = 12582912.0f;
+constexpr uint32_t kToOctal = 0x924924u - 0x4B400000u;
+
+// Eight digits + 4 -> e2m1: below 4 the sign bit and 4 - digit, from 4 on digit - 4 (codes 0 .. 4 are 0, 0.5,
+// .. 2).  `first`: the first digits of numbers, which go up to 4.
+__device__ __forceinline__ uint32_t e2m1_digits(uint32_t octal, bool first) {
+    const uint32_t four = first ? (octal & 0x88888888u) >> 1 : 0u;
+    const uint32_t negative = (~(octal | four) & 0x44444444u) >> 2;
+    return (((octal ^ (3u * negative)) & 0x33333333u) | four) + 9u * negative;
+}
+
+// Eight e2m1 digits of sixteen numbers (each an integer plus 4 in every octal digit), a digit every `pitch` bytes.
+__device__ __forceinline__ void store_digits(const uint32_t (&digits)[16], unsigned char* out, int pitch) {
+#pragma unroll
+    for (int j = 0; j < kNativeDigits; ++j) {
+        uint32_t word[2];
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            uint32_t octal = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int shift = 4 * i - 3 * j;
+                const uint32_t moved = shift >= 0 ? digits[8 * w + i] << (shift & 31) : digits[8 * w + i] >> ((-shift) & 31);
+                octal |= moved & ((j == kNativeDigits - 1 ? 15u : 7u) << (4 * i));
+            }
+            word[w] = e2m1_digits(octal, j == kNativeDigits - 1);
+        }
+        *reinterpret_cast<uint2*>(out + j * pitch) = make_uint2(word[0], word[1]);
+    }
+}
+
+// The digits of what those of sixteen f16 that are below `on_grid` leave on the grid 1 / up, in multiples of 2^-23
+// of it; one or two of them as a rule, so one after the other, all digits of a number at once.
+__device__ __noinline__ void store_rest(uint4 lo, uint4 hi, uint32_t on_grid, float up, unsigned char* out, int pitch) {
+    const uint32_t half[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    uint32_t below = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        below |= ((half[i] & 0x7fffu) < on_grid ? 1u : 0u) << (2 * i);
+        below |= (((half[i] >> 16) & 0x7fffu) < on_grid ? 2u : 0u) << (2 * i);
+    }
+    uint32_t word[kNativeDigits][2] = {};
+#pragma unroll 1
+    while (below != 0) {
+        const int i = __ffs(below) - 1;
+        below &= below - 1;
+        uint32_t pair = half[0];
+#pragma unroll
+        for (int other = 1; other < 8; ++other) {
+            pair = (i >> 1) == other ? half[other] : pair;
+        }
+        const float x = __half2float(__ushort_as_half(static_cast<unsigned short>((i & 1) ? pair >> 16 : pair))) * up;
+        uint32_t octal = __float_as_uint(fmaf(x - rintf(x), 8388608.0f, kBinade)) + kToOctal;
+        octal = (octal & 0xfffu) | (octal & 0xfff000u) << 4;  // three bits each -> a nibble each
+        octal = (octal & 0x003f003fu) | (octal & 0x0fc00fc0u) << 2;
+        octal = (octal & 0x07070707u) | (octal & 0x38383838u) << 1;
+        const uint32_t codes = e2m1_digits(octal, false);
+#pragma unroll
+        for (int j = 0; j < kNativeDigits; ++j) {
+            const uint32_t digit = ((codes >> (4 * j)) & 15u) << (4 * (i & 7));
+            word[j][0] |= i < 8 ? digit : 0u;
+            word[j][1] |= i < 8 ? 0u : digit;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kNativeDigits; ++j) {
+        *reinterpret_cast<uint2*>(out + j * pitch) = make_uint2(word[j][0], word[j][1]);
+    }
+}
+
 // bf16 rows [batch][K] in and [batch][N] out.  A K split is a thread-block cluster that sums its slices, in
 // slice order, through distributed shared memory: CTA s finishes the rows s, s + splits, ...
 template <bool kSwiglu>
@@ -153,7 +232,9 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
     const int rows_shift = p.batch <= 2 ? 1 : p.batch <= 4 ? 2 : 3;
     const int R = 1 << rows_shift;
     const int N = kNativeDigits * R;
-    const int x_slot_bytes = N * 128 + 2048;  // digit tile [K / 32][N][16 bytes], then its scale blocks
+    // digit tile [K / 32][N][16 bytes], its scale blocks, and the tile of the second eight digits
+    const int x_slot_bytes = 2 * N * 128 + 2048;
+    const int x_rest = N * 128 + 2048;
     const int x_slots = min(kNativeMaxXSlots, kNativeXBytes / x_slot_bytes);
     // a stage has 16 R blocks of 16 activations: one per lane of `team` warps
     const int team = R / 2;
@@ -199,7 +280,9 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
         for (int s = 0; s < kNativeMaxXSlots; ++s) {
             mbar_init(&bars.x_full[s], team);
             mbar_init(&bars.x_empty[s], 1);
+            bars.rest[s] = 0;
         }
+        bars.rest_used = 0;
         mbar_init(&bars.done, 1);
         mbar_init(&bars.tmem_ready, 1);
         bars.failed = status_is_set(p.status) ? 1 : 0;
@@ -248,6 +331,7 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
         bool ok = true;
         int xs = 0;
         uint32_t x_parity = 0;
+        uint32_t rest_started = 0;
         for (int index = 0; index < num_stages; ++index) {
             const int slot = index % kWeightStages;
             ok = native_wait(&bars.w_checked[slot], (index / kWeightStages) & 1, &bars, p.status) &&
@@ -256,6 +340,7 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t rest = *reinterpret_cast<volatile uint32_t*>(&bars.rest[xs]);
             if (elect_one()) {
                 const uint32_t scales = tmem_base + kNativeScaleColumn + (index & 1) * kNativeScaleColumns;
                 const uint32_t x_tile = x_base + xs * x_slot_bytes;
@@ -279,6 +364,23 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
                                    scales + 16 * t + 4 * ks, scales + 32 + 4 * ks, (index > 0 || ks > 0) ? 1u : 0u);
                     }
                 }
+                if (rest != 0) {
+                    uint32_t started = rest_started;
+#pragma unroll 1
+                    for (int ks = 0; ks < 4; ++ks) {
+                        if (((rest >> (8 * ((ks * team) >> 2))) & 0xffu) == 0) {  // whose quarter of the stage it is
+                            continue;
+                        }
+                        const uint64_t b_desc = smem_descriptor(x_tile + x_rest + ks * (2 * 16) * N, N * 16, 128);
+#pragma unroll
+                        for (int t = 0; t < kTiles; ++t) {
+                            umma_nvfp4(tmem_base + t * kNativeAccumulator + kNativeRest,
+                                       swizzled_descriptor(w_tile + t * kTileStageBytes + 32 * ks), b_desc, idesc,
+                                       scales + 16 * t + 4 * ks, scales + 32 + 4 * ks, started);
+                        }
+                        started = 1;
+                    }
+                }
                 umma_commit(&bars.w_empty[slot]);
                 umma_commit(&bars.x_empty[xs]);
                 if (index == num_stages - 1) {
@@ -286,6 +388,7 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
                 }
             }
             __syncwarp();
+            rest_started |= rest != 0 ? 1u : 0u;
             if (++xs == x_slots) {
                 xs = 0;
                 x_parity ^= 1;
@@ -347,6 +450,7 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
             hi = at[1];
         };
         bool ok = true;
+        bool rest_used = false;
         uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
         if (e / team < num_stages) {
             fetch(e / team, lo, hi);
@@ -361,34 +465,39 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
                 half[i] = bf16x2_to_f16x2(half[i]);
             }
             uint32_t peak = 0;
+            uint32_t least = 0x7fff7fffu;  // of the magnitudes that are not 0, less one, as signed halves from -32768
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                peak = __vmaxu2(peak, half[i] & 0x7fff7fffu);
+                const uint32_t magnitude = half[i] & 0x7fff7fffu;
+                peak = __vmaxu2(peak, magnitude);
+                least = __vmins2(least, magnitude + 0x7fff7fffu);
             }
             peak = max(peak & 0xffffu, peak >> 16);
+            const int least_magnitude =
+                min(static_cast<int>(static_cast<int16_t>(least & 0xffffu)), static_cast<int>(least) >> 16) + 0x8001;
             // the block's power of two: 2^(exponent - 14) is above every magnitude; below 2^-2 it stays, and
-            // the last digit is then the grid of the smallest f16
-            const uint32_t exponent = max(peak >> 10, 12u);
-            // as an e4m3 scale, 2^7 left to the epilogue; infinity and NaN poison the block, and the one
-            // binade that the scales do not reach (from 2^15) takes the largest of them, 448
-            const bool top = peak >= 0x7800u;
+            // the last digit is then the grid of the smallest f16.  The scales end at 2^8 (2^7 of it is left
+            // to the epilogue): the one binade above takes that scale, and its first digit may be 4.
+            const int exponent = min(max(static_cast<int>(peak >> 10), 12), 29);
+            // an e4m3 scale; NaN poisons the block (an infinity has become 65504 in the conversion)
             const uint32_t scale = peak >= 0x7c00u ? 0x7fu
-                                   : top           ? 0x7eu
-                                   : exponent >= 15u ? (exponent - 14u) << 3
-                                                     : 1u << (exponent - 12u);
-            const float up = __uint_as_float((163u - min(exponent, 30u)) << 23);  // 2^(36 - exponent)
+                                   : exponent >= 15 ? static_cast<uint32_t>(exponent - 14) << 3
+                                                    : 1u << (exponent - 12);
+            const float up = __uint_as_float(static_cast<uint32_t>(163 - exponent) << 23);  // 2^(36 - exponent)
+            // the smallest magnitude whose eight significant bits all lie on the grid of 2^(exponent - 36)
+            const int on_grid = exponent <= 12 ? 0 : max(exponent - 14, 1) << 10;
+            const bool again = __any_sync(0xffffffffu, least_magnitude < on_grid);
+            rest_used |= again;
+            // multiples of 2^(exponent - 36)
             uint32_t digits[16];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const float2 two = __half22float2(*reinterpret_cast<const __half2*>(&half[i]));
-                // x as a multiple of 2^(exponent - 36), in the low bits of the 2^23 binade; the constant
-                // adds 4 to every octal digit
-                digits[2 * i] = __float_as_uint(fmaf(two.x, up, 12582912.0f)) + (0x924924u - 0x4B400000u);
-                digits[2 * i + 1] = __float_as_uint(fmaf(two.y, up, 12582912.0f)) + (0x924924u - 0x4B400000u);
-                if (top) {
-                    constexpr float kUp = 4194304.0f / (448.0f * 128.0f);
-                    digits[2 * i] = static_cast<uint32_t>(__float2int_rn(two.x * kUp)) + 0x924924u;
-                    digits[2 * i + 1] = static_cast<uint32_t>(__float2int_rn(two.y * kUp)) + 0x924924u;
+                digits[2 * i] = __float_as_uint(fmaf(two.x, up, kBinade)) + kToOctal;
+                digits[2 * i + 1] = __float_as_uint(fmaf(two.y, up, kBinade)) + kToOctal;
+                if (peak >= 0x7800u) {  // more than the binade holds
+                    digits[2 * i] = static_cast<uint32_t>(__float2int_rn(two.x * up)) + 0x924924u;
+                    digits[2 * i + 1] = static_cast<uint32_t>(__float2int_rn(two.y * up)) + 0x924924u;
                 }
             }
             const int xs = index % x_slots;
@@ -401,24 +510,16 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
             unsigned char* scale_out = tile + N * 128 + (block >> 2) * 512 + (block & 3);
 #pragma unroll
             for (int j = 0; j < kNativeDigits; ++j) {
-                uint32_t word[2];
-#pragma unroll
-                for (int w = 0; w < 2; ++w) {
-                    uint32_t octal = 0;
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int shift = 4 * i - 3 * j;
-                        const uint32_t moved = shift >= 0 ? digits[8 * w + i] << (shift & 31) : digits[8 * w + i] >> ((-shift) & 31);
-                        octal |= moved & (7u << (4 * i));
-                    }
-                    // digit + 4 -> e2m1: below 4 the sign bit and 4 - digit, else digit - 4 (codes 0 .. 4 are
-                    // 0, 0.5, .. 2)
-                    const uint32_t negative = (~octal & 0x44444444u) >> 2;
-                    word[w] = ((octal ^ (3u * negative)) & 0x33333333u) + 9u * negative;
-                }
                 const int n = j * R + row;
-                *reinterpret_cast<uint2*>(out + j * R * 16) = make_uint2(word[0], word[1]);
                 scale_out[(n & 31) * 16 + (n >> 5) * 4] = static_cast<unsigned char>(scale);
+            }
+            store_digits(digits, out, R * 16);
+            if (again) {
+                store_rest(make_uint4(half[0], half[1], half[2], half[3]), make_uint4(half[4], half[5], half[6], half[7]),
+                           static_cast<uint32_t>(on_grid), up, out + x_rest, R * 16);
+            }
+            if (lane == 0) {
+                reinterpret_cast<volatile uint8_t*>(&bars.rest[xs])[e % team] = again ? 1 : 0;
             }
             fence_proxy_async();
             __syncwarp();
@@ -426,6 +527,11 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
                 mbar_arrive(&bars.x_full[xs]);
             }
         }
+        if (rest_used && lane == 0) {
+            *reinterpret_cast<volatile int*>(&bars.rest_used) = 1;
+        }
+        __syncwarp();
+        asm volatile("bar.sync 1, %0;" ::"n"(kNativeWorkerWarps * 32) : "memory");
         // ---------------- epilogue ----------------
         // Warp e: output rows 32 (e % 4) .. + 31 of both tiles, activation rows (e / 4) R / 2 .. .
         ok = native_wait(&bars.done, 0, &bars, p.status);
@@ -441,20 +547,32 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
             for (int i = 0; i < kTokens; ++i) {
                 v0[i] = v1[i] = 0.0f;
             }
-            float weight = 128.0f / 2097152.0f;  // 2^7 8^-7
+            const auto add_digits = [&](uint32_t columns, float weight) {  // `weight` of the lowest digit
 #pragma unroll
-            for (int j = 0; j < kNativeDigits; ++j) {
-                uint32_t r0[8], r1[8];  // (the columns behind this warp's rows are other rows and digits)
-                tmem_load8_issue(address + j * R, r0);
-                tmem_load8_issue(address + kNativeAccumulator + j * R, r1);
-                tmem_load_wait();
+                for (int first = 0; first < kNativeDigits; first += 4) {
+                    uint32_t r0[4][8], r1[4][8];  // (the columns behind this warp's rows are other rows and digits)
 #pragma unroll
-                for (int i = 0; i < kTokens; ++i) {
-                    v0[i] = fmaf(__uint_as_float(r0[i]), weight, v0[i]);
-                    v1[i] = fmaf(__uint_as_float(r1[i]), weight, v1[i]);
+                    for (int j = 0; j < 4; ++j) {
+                        tmem_load8_issue(columns + (first + j) * R, r0[j]);
+                        tmem_load8_issue(columns + kNativeAccumulator + (first + j) * R, r1[j]);
+                    }
+                    tmem_load_wait();
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                        for (int i = 0; i < kTokens; ++i) {
+                            v0[i] = fmaf(__uint_as_float(r0[j][i]), weight, v0[i]);
+                            v1[i] = fmaf(__uint_as_float(r1[j][i]), weight, v1[i]);
+                        }
+                        weight *= 8.0f;
+                    }
                 }
-                weight *= 8.0f;
+            };
+            constexpr float kLowest = 128.0f / 2097152.0f;  // 2^7 8^-7
+            if (*reinterpret_cast<volatile int*>(&bars.rest_used) != 0) {
+                add_digits(address + kNativeRest, kLowest / 8388608.0f);
             }
+            add_digits(address, kLowest);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             const int tokens = min(p.batch - first_token, R / 2);
             if (p.splits > 1) {

@@ -850,3 +850,54 @@ def test_four_bit_swiglu_matches_oracle(cuda, ops):
                      dev(torch, x), out, batch)
     torch.cuda.synchronize()
     assert_rms_close(synth.bf16_value(host(out)), want, "four-bit SwiGLU")
+
+
+def dequantize(packed, scales):
+    values = np.array([0, 0.5, 1, 1.5, 2, 3, 4, 6, 0, -0.5, -1, -1.5, -2, -3, -4, -6])
+    codes = np.stack([packed & 15, packed >> 4], axis=-1).reshape(packed.shape[0], -1)
+    return values[codes] * np.repeat(synth.e4m3_decode(scales).astype(np.float64), 16, axis=1)
+
+
+@pytest.mark.parametrize("out_features,in_features", [(5120, 4096), (34816, 512)], ids=["k_slices", "one_slice"])
+@pytest.mark.parametrize("batch", [1, 2, 3, 4, 5, 8])
+def test_four_bit_projection_keeps_small_activations_beside_large(cuda, ops, out_features, in_features, batch):
+    """Every block of sixteen holds one large activation (up to f16's largest binade) where the weights are 0,
+    and small ones elsewhere: the outputs are sums of the small ones alone, which f16 operands hold exactly.
+    Bound: half a bf16 step of the result, and one rounding of 2^-24 of the magnitudes per 64 features."""
+    torch = cuda
+    rng = synth.generator(43, f"beside.{out_features}.{batch}")
+    packed, scales, _ = synth.nvfp4_matrix(43, "beside", out_features, in_features)
+    packed[:, 2::8] &= 0x0F  # feature 5 of every block
+    swizzled = synth.swizzle_block_scales(scales, out_features, in_features)
+    small = rng.uniform(0.002, 0.004, (batch, in_features)) * 2.0 ** rng.integers(-4, 3, (batch, in_features))
+    values = (small * rng.choice([-1.0, 1.0], small.shape)).astype(np.float32)
+    values[:, 5::16] = rng.choice([4096.0, -30000.0, 59904.0, -65280.0, 65504.0], (batch, in_features // 16))
+    x = synth.bf16_bits(values)
+    x[:, 0::64] = synth.bf16_bits(np.zeros((batch, in_features // 64), dtype=np.float32))
+    exact = synth.bf16_value(x).astype(np.float64)
+    exact[:, 5::16] = 0.0
+    weights = dequantize(packed, scales)
+    want = exact @ weights.T
+    magnitudes = np.abs(exact) @ np.abs(weights).T
+    got, _ = run_gemv(torch, ops, packed, scales, swizzled, 1.0, x, out_features, in_features, batch)
+    bound = 2.0 ** -8 * np.abs(want) + (in_features / 64) * 2.0 ** -24 * magnitudes
+    assert np.all(np.abs(got - want) <= bound)
+
+
+@pytest.mark.parametrize("in_features", [4096, 17408])
+def test_four_bit_projection_rounds_no_more_than_the_f16_kernel(cuda, ops, in_features):
+    """Every block of sixteen features is there twice with opposite weights, shuffled over K: the exact result is
+    0, and a call returns its own rounding.  Nine rows run on the f16 kernel, eight of them in four bits."""
+    torch = cuda
+    out_features, blocks = 5120, in_features // 16
+    packed, scales, _ = synth.nvfp4_matrix(46, "rounding", out_features, in_features // 2)
+    order = synth.generator(46, "order").permutation(blocks)
+    packed = packed.reshape(out_features, blocks // 2, 8)
+    packed = np.concatenate([packed, packed ^ 0x88], axis=1)[:, order].reshape(out_features, in_features // 2)
+    scales = np.ascontiguousarray(np.concatenate([scales, scales], axis=1)[:, order])
+    x = synth.normal_bf16(46, "x", (9, blocks // 2, 16))
+    x = np.ascontiguousarray(np.concatenate([x, x], axis=1)[:, order].reshape(9, in_features))
+    swizzled = synth.swizzle_block_scales(scales, out_features, in_features)
+    four, _ = run_gemv(torch, ops, packed, scales, swizzled, 1.0, x[:8], out_features, in_features, 8)
+    wide, _ = run_gemv(torch, ops, packed, scales, swizzled, 1.0, x, out_features, in_features, 9)
+    assert np.any(four != 0) and np.sqrt(np.mean(np.square(four))) <= np.sqrt(np.mean(np.square(wide[:8])))
