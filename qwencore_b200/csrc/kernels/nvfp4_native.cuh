@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
                         if (i < tokens && out_row < p.out_features) {
                             float value = (t == 0 ? v0[i] : v1[i]) * p.inverse_scale[0];
                             if (kSwiglu) {
-                                value = __fdividef(value, 1.0f + __expf(-value)) * (v1[i] * p.inverse_scale[1]);
+                                value = value / (1.0f + __expf(-value)) * (v1[i] * p.inverse_scale[1]);
                             }
                             p.y[static_cast<size_t>(first_token + i) * p.out_features + out_row] =
                                 __float2bfloat16(value);
@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
                 }
                 value *= p.inverse_scale[0];
                 if (kSwiglu) {
-                    value = __fdividef(value, 1.0f + __expf(-value)) * (up * p.inverse_scale[1]);
+                    value = value / (1.0f + __expf(-value)) * (up * p.inverse_scale[1]);
                 }
                 p.y[static_cast<size_t>(token) * p.out_features + out_row] = __float2bfloat16(value);
             }

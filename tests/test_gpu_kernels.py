@@ -901,3 +901,24 @@ def test_four_bit_projection_rounds_no_more_than_the_f16_kernel(cuda, ops, in_fe
     four, _ = run_gemv(torch, ops, packed, scales, swizzled, 1.0, x[:8], out_features, in_features, 8)
     wide, _ = run_gemv(torch, ops, packed, scales, swizzled, 1.0, x, out_features, in_features, 9)
     assert np.any(four != 0) and np.sqrt(np.mean(np.square(four))) <= np.sqrt(np.mean(np.square(wide[:8])))
+
+
+def test_four_bit_swiglu_divides_like_the_other_kernels(cuda, ops):
+    """gate values around -88: 1 + exp(88) is beyond 2^126, where a fast division gives 0 instead of the quotient."""
+    torch = cuda
+    out_features, in_features, batch = 4096, 4096, 2
+    gate = np.full((out_features, in_features // 2), 0x22, dtype=np.uint8)  # 1.0 everywhere
+    scales = np.full((out_features, in_features // 16), 0x38, dtype=np.uint8)
+    swizzled = synth.swizzle_block_scales(scales, out_features, in_features)
+    x = synth.bf16_bits(np.stack([np.full(in_features, -88.0 / 4096, dtype=np.float32),
+                                  np.full(in_features, -87.5 / 4096, dtype=np.float32)]))
+    linear = ops.Linear(dev(torch, gate), dev(torch, swizzled), 1.0, out_features, in_features)
+    up = ops.Linear(dev(torch, gate), dev(torch, swizzled), 2.0 ** -20, out_features, in_features)
+    out = bf16_out(torch, batch, out_features)
+    ops.swiglu_w4a16(linear, up, dev(torch, x), out, batch)
+    torch.cuda.synchronize()
+    value = synth.bf16_value(x).astype(np.float64).sum(-1)
+    want = value / (1.0 + np.exp(-value)) * value * 2.0 ** 20
+    got = synth.bf16_value(host(out)).astype(np.float64)
+    # exp of fp32 arguments near 88: 88 * 2^-24 of the argument's rounding, and a bf16 result
+    assert np.all(np.abs(got - want[:, None]) <= 0.01 * np.abs(want)[:, None])
