@@ -121,7 +121,9 @@ __device__ __forceinline__ void copy_scales(uint32_t tmem, uint64_t desc) {
     asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem), "l"(desc) : "memory");
 }
 
+// (.aligned: the whole warp at once, and every warp gets here from a region that ends with one lane at work)
 __device__ __forceinline__ void native_cluster_sync() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

@@ -922,3 +922,31 @@ def test_four_bit_swiglu_divides_like_the_other_kernels(cuda, ops):
     got = synth.bf16_value(host(out)).astype(np.float64)
     # exp of fp32 arguments near 88: 88 * 2^-24 of the argument's rounding, and a bf16 result
     assert np.all(np.abs(got - want[:, None]) <= 0.01 * np.abs(want)[:, None])
+
+
+@pytest.mark.parametrize("batch", [1, 8])
+@pytest.mark.parametrize("kind", ["matrix", "pair", "head"])
+def test_four_bit_projection_with_a_hint_stores_the_same_bytes(cuda, ops, batch, kind):
+    """A K split (a cluster) and a whole K that name what follows: a large matrix, a pair, a vocabulary head."""
+    torch = cuda
+    from qwencore_b200 import abi
+    x = dev(torch, synth.normal_bf16(44, "x", (batch, 5120)))
+
+    def linear(name, out_features, in_features):
+        packed, _, swizzled = synth.nvfp4_matrix(44, name, out_features, in_features)
+        return ops.Linear(dev(torch, packed), dev(torch, swizzled), 8.0, out_features, in_features)
+
+    after, after_up = linear("after", 5120, 6144), linear("after_up", 5120, 6144)
+    table = torch.zeros((16384, 5120), dtype=torch.uint8, device="cuda")
+    for out_features in (5128, 34816):
+        now = linear("now", out_features, 5120)
+        plain, hinted = bf16_out(torch, batch, out_features), bf16_out(torch, batch, out_features)
+        now.forward_w4a16(x, plain, batch)
+        if kind == "head":
+            assert abi.lib.qwc_nvfp4_prefetch_next(table.data_ptr(), None, None, None, 16384, 5120, 2) == 0
+        else:
+            ops.prefetch_next(after, after_up if kind == "pair" else None)
+        now.forward_w4a16(x, hinted, batch)
+        torch.cuda.synchronize()
+        assert np.array_equal(host(hinted), host(plain))
+    assert abi.lib.qwc_device_status() == 0
