@@ -536,7 +536,8 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
         asm volatile("bar.sync 1, %0;" ::"n"(kNativeWorkerWarps * 32) : "memory");
         // ---------------- epilogue ----------------
         // Warp e: output rows 32 (e % 4) .. + 31 of both tiles, activation rows (e / 4) R / 2 .. .
-        ok = native_wait(&bars.done, 0, &bars, p.status);
+        ok = native_wait(&bars.done, 0, &bars, p.status) &&
+             __all_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&bars.failed) == 0);
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars.tmem_base);

@@ -950,3 +950,30 @@ def test_four_bit_projection_with_a_hint_stores_the_same_bytes(cuda, ops, batch,
         torch.cuda.synchronize()
         assert np.array_equal(host(hinted), host(plain))
     assert abi.lib.qwc_device_status() == 0
+
+
+@pytest.mark.parametrize("out_features,in_features", [(5120, 4096), (34816, 512)], ids=["k_slices", "one_slice"])
+@pytest.mark.parametrize("swiglu", [False, True], ids=["plain", "swiglu"])
+def test_four_bit_projection_stores_nothing_once_a_wait_has_given_up(cuda, ops, out_features, in_features, swiglu):
+    """With the status word set (as an earlier kernel leaves it), as the other projection kernels do."""
+    torch = cuda
+    from qwencore_b200 import abi
+    packed, _, swizzled = synth.nvfp4_matrix(45, "status", out_features, in_features)
+    linear = ops.Linear(dev(torch, packed), dev(torch, swizzled), 8.0, out_features, in_features)
+    x = dev(torch, synth.normal_bf16(45, "x", (3, in_features)))
+    out = dev(torch, np.full((3, out_features), 0x1234, dtype=np.uint16))
+    torch.cuda.synchronize()
+    assert abi.lib.qwc_device_status_set(0x103) == 0
+    try:
+        if swiglu:
+            ops.swiglu_w4a16(linear, linear, x, out, 3)
+        else:
+            linear.forward_w4a16(x, out, 3)
+        torch.cuda.synchronize()
+        assert abi.lib.qwc_device_status() == 0x103
+        assert np.all(host(out) == 0x1234)
+    finally:
+        assert abi.lib.qwc_device_status_reset() == 0
+    linear.forward_w4a16(x, out, 3)
+    torch.cuda.synchronize()
+    assert np.isfinite(synth.bf16_value(host(out))).all()
