@@ -128,13 +128,16 @@ __device__ __forceinline__ void native_cluster_sync() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// A float of another CTA of the cluster, at the place where this CTA has `local`.
-__device__ __forceinline__ float native_peer_float(const float* local, int rank) {
-    uint32_t remote;
-    float value;
+// A word of another CTA of the cluster, at the place where this CTA has `local`.
+__device__ __forceinline__ uint32_t native_peer_word(const void* local, int rank) {
+    uint32_t remote, value;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(local)), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(value) : "r"(remote) : "memory");
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(value) : "r"(remote) : "memory");
     return value;
+}
+
+__device__ __forceinline__ float native_peer_float(const float* local, int rank) {
+    return __uint_as_float(native_peer_word(local, rank));
 }
 
 // The 2^23 binade, whose low bits are the integer that was added, and what turns them into the integer plus 4 in
@@ -615,8 +618,12 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
         const int t = worker >> 7;
         const int out_row = kSwiglu ? pair * kTileRows + (worker & 127)
                                     : (pair * kTiles + t) * kTileRows + (worker & 127);
-        if (worker >= 0 && (!kSwiglu || t == 0) && out_row < p.out_features &&
-            *reinterpret_cast<volatile int*>(&bars.failed) == 0) {
+        if (worker >= 0 && (!kSwiglu || t == 0) && out_row < p.out_features) {
+            uint32_t gave_up = 0;  // a CTA that did has no sums: nobody of its cluster stores
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                gave_up |= r < p.splits ? native_peer_word(&bars.failed, r) : 0u;
+            }
             for (int token = slice; token < p.batch; token += p.splits) {
                 const float* park =
                     reinterpret_cast<const float*>(weight_ring) + (t * kNativeRows + token) * kTileRows + (worker & 127);
@@ -636,7 +643,9 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
                 if (kSwiglu) {
                     value = value / (1.0f + __expf(-value)) * (up * p.inverse_scale[1]);
                 }
-                p.y[static_cast<size_t>(token) * p.out_features + out_row] = __float2bfloat16(value);
+                if (gave_up == 0) {
+                    p.y[static_cast<size_t>(token) * p.out_features + out_row] = __float2bfloat16(value);
+                }
             }
         }
         native_cluster_sync();  // nobody leaves while a peer may still read its shared memory
