@@ -337,7 +337,8 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
         int xs = 0;
         uint32_t x_parity = 0;
         uint32_t rest_started = 0;
-        for (int index = 0; index < num_stages; ++index) {
+        int index = 0;
+        for (; index < num_stages; ++index) {
             const int slot = index % kWeightStages;
             ok = native_wait(&bars.w_checked[slot], (index / kWeightStages) & 1, &bars, p.status) &&
                  native_wait(&bars.x_full[xs], x_parity, &bars, p.status);
@@ -398,6 +399,15 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
                 xs = 0;
                 x_parity ^= 1;
             }
+        }
+        if (!ok && index > 0) {
+            // the MMAs that were issued still read shared memory and write tensor memory: this warp waits for
+            // the last of them (0.2 ms at most) before the CTA gives either back
+            const long long start = clock64();
+            while (!mbar_try_wait(&bars.w_empty[(index - 1) % kWeightStages], ((index - 1) / kWeightStages) & 1) &&
+                   clock64() - start < 400000ll) {
+            }
+            __syncwarp();
         }
     } else if (warp < kNativeFirstWorker) {
         // ---------------- signs of the weight scales ----------------
