@@ -72,6 +72,15 @@ struct NextProjection {
 void set_next_projection(const NextProjection& next);
 NextProjection take_next_projection();
 
+// Rows in memory as bf16: which kernel a projection of `batch` rows runs on (nvfp4_gemv.cu: dispatch), and into
+// how many K slices the two kernels that start from a ring of weight stages cut it.  A launch that has been told
+// what follows asks L2 for the stages that those slices begin with.
+inline bool runs_in_four_bits(int out_features, int in_features, int batch) {
+    return batch <= 8 && static_cast<long long>(out_features) * in_features >= 16ll * 1000 * 1000;
+}
+int native_splits(int out_features, int in_features, bool swiglu);          // nvfp4_native.cuh
+int umma_splits(int out_features, int in_features, bool swiglu, bool fp8);  // nvfp4_umma.cu
+
 // Process-wide shape selection (see qwc_configure in the C ABI).
 struct Shape {
     int delta_value_heads;

@@ -1319,18 +1319,36 @@ LaunchShape shape_of(int out_features, int in_features, bool swiglu, bool fp8, b
     return shape;
 }
 
+// What the projection that the caller named next will start with: on staged activations ...
+LaunchShape staged_shape(const NextProjection& hint) {
+    // kinds 3 and 4: a matrix / a SwiGLU pair that will run as a regular K split (qwc_nvfp4_w4a16_split,
+    // the latency-mode projections)
+    return shape_of(hint.out_features, hint.in_features, hint.kind == 1 || hint.kind == 4, hint.kind == 2,
+                    hint.kind == 3 || hint.kind == 4);
+}
+
+// ... and on rows in memory, of which there are as many as now.
+LaunchShape rows_shape(const NextProjection& hint, int batch) {
+    LaunchShape shape = staged_shape(hint);
+    if (hint.kind <= 2) {
+        shape.splits = runs_in_four_bits(hint.out_features, hint.in_features, batch) && hint.kind != 2
+                           ? native_splits(hint.out_features, hint.in_features, hint.kind == 1)
+                           : umma_splits(hint.out_features, hint.in_features, hint.kind == 1, hint.kind == 2);
+        shape.ctas = shape.pair_tiles * shape.splits;
+    }
+    return shape;
+}
+
 // The caller's hint about the projection that follows (one use).
-void take_hint(StreamKParams& p, CUtensorMap& next_map0, CUtensorMap& next_map1) {
+template <typename Plan>
+void take_hint(StreamKParams& p, CUtensorMap& next_map0, CUtensorMap& next_map1, Plan&& plan) {
     p.next.valid = 0;
     const NextProjection hint = take_next_projection();
     if (hint.packed[0] != nullptr && hint.out_features > 0 && hint.in_features > 0) {
         const bool next_fp8 = hint.kind == 2;
         const bool next_swiglu = hint.kind == 1 || hint.kind == 4;
         const int next_row_bytes = next_fp8 ? hint.in_features : hint.in_features / 2;
-        // kinds 3 and 4: a matrix / a SwiGLU pair that will run as a regular K split (qwc_nvfp4_w4a16_split,
-        // the latency-mode projections)
-        const LaunchShape next =
-            shape_of(hint.out_features, hint.in_features, next_swiglu, next_fp8, hint.kind == 3 || hint.kind == 4);
+        const LaunchShape next = plan(hint);
         if (next.units > 0 &&
             encode_weight_map(&next_map0, hint.packed[0], hint.out_features, next_row_bytes) == cudaSuccess &&
             encode_weight_map(&next_map1, hint.packed[next_swiglu ? 1 : 0], hint.out_features, next_row_bytes) ==
@@ -1399,7 +1417,7 @@ cudaError_t launch_streamk(StreamKParams p, const void* packed0, const void* pac
         return opted == nullptr ? cudaErrorInvalidDevice : *opted;
     }
     CUtensorMap next_map0 = map0, next_map1 = map1;
-    take_hint(p, next_map0, next_map1);
+    take_hint(p, next_map0, next_map1, staged_shape);
     p.status = status_ptr();
     if (p.status == nullptr) {
         return cudaErrorInvalidValue;
@@ -1421,33 +1439,20 @@ cudaError_t launch_streamk(StreamKParams p, const void* packed0, const void* pac
     return cudaLaunchKernelEx(&config, kernel, map0, map1, next_map0, next_map1, p);
 }
 
-}  // namespace
+using NativeKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
+                              const StreamKParams);
+const NativeKernel native_kernels[2] = {nvfp4_native_kernel<false>, nvfp4_native_kernel<true>};
 
-// bf16 rows in, bf16 rows out, at most kNativeRows of them (the reference's signature; see nvfp4_gemv.cu).
-cudaError_t launch_nvfp4_native(const void* packed0, const void* scales0, const void* packed1, const void* scales1,
-                                const __nv_bfloat16* x, __nv_bfloat16* y, int out_features, int in_features, int batch,
-                                float inverse_scale0, float inverse_scale1, bool swiglu, cudaStream_t stream) {
-    StreamKParams p = {};
-    p.scales[0] = static_cast<const uint8_t*>(scales0);
-    p.scales[1] = static_cast<const uint8_t*>(swiglu ? scales1 : scales0);
-    p.x_rows = x;
-    p.y = y;
-    p.inverse_scale[0] = inverse_scale0;
-    p.inverse_scale[1] = inverse_scale1;
-    p.out_features = out_features;
-    p.in_features = in_features;
-    p.batch = batch;
-    using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
-                            const StreamKParams);
-    static const Kernel kernels[2] = {nvfp4_native_kernel<false>, nvfp4_native_kernel<true>};
-    struct Setup {
-        cudaError_t opted;
-        int clusters[9];  // of each size, resident at once (a cluster must sit inside one GPC)
-    };
-    static PerDevice<Setup> setup_per_device;
-    const Setup* setup = setup_per_device.get([]() {
-        Setup s = {};
-        for (const Kernel kernel : kernels) {
+struct NativeSetup {
+    cudaError_t opted;
+    int clusters[9];  // of each size, resident at once (a cluster must sit inside one GPC)
+};
+
+const NativeSetup* native_setup() {
+    static PerDevice<NativeSetup> per_device;
+    return per_device.get([]() {
+        NativeSetup s = {};
+        for (const NativeKernel kernel : native_kernels) {
             s.opted = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNativeSmemBytes);
             if (s.opted != cudaSuccess) {
                 return s;
@@ -1466,13 +1471,55 @@ cudaError_t launch_nvfp4_native(const void* packed0, const void* scales0, const 
             attribute[0].val.clusterDim.z = 1;
             probe.attrs = attribute;
             probe.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&s.clusters[size], kernels[0], &probe) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveClusters(&s.clusters[size], native_kernels[0], &probe) != cudaSuccess) {
                 s.clusters[size] = 0;
                 (void)cudaGetLastError();
             }
         }
         return s;
     });
+}
+
+}  // namespace
+
+int native_splits(int out_features, int in_features, bool swiglu) {
+    const NativeSetup* setup = native_setup();
+    const int rows_per_pair = swiglu ? kTileRows : kTiles * kTileRows;
+    const int pair_tiles = (out_features + rows_per_pair - 1) / rows_per_pair;
+    const int stages_in_k = in_features / (kChunkK * kStageChunks);
+    // Stages one after the other on the busiest SM, plus what a wave costs beside its stages and a
+    // cluster beside its slices (in stages).
+    int splits = 1;
+    double best = 1e30;
+    for (int size = 1; setup != nullptr && size <= 8 && size <= stages_in_k; ++size) {
+        if (setup->clusters[size] <= 0) {
+            continue;
+        }
+        const int waves = (pair_tiles + setup->clusters[size] - 1) / setup->clusters[size];
+        const double cost = waves * ((stages_in_k + size - 1) / size + 3.0) + (size > 1 ? 1.0 : 0.0) + 0.2 * size;
+        if (cost < best) {
+            best = cost;
+            splits = size;
+        }
+    }
+    return splits;
+}
+
+// bf16 rows in, bf16 rows out, at most kNativeRows of them (the reference's signature; see nvfp4_gemv.cu).
+cudaError_t launch_nvfp4_native(const void* packed0, const void* scales0, const void* packed1, const void* scales1,
+                                const __nv_bfloat16* x, __nv_bfloat16* y, int out_features, int in_features, int batch,
+                                float inverse_scale0, float inverse_scale1, bool swiglu, cudaStream_t stream) {
+    StreamKParams p = {};
+    p.scales[0] = static_cast<const uint8_t*>(scales0);
+    p.scales[1] = static_cast<const uint8_t*>(swiglu ? scales1 : scales0);
+    p.x_rows = x;
+    p.y = y;
+    p.inverse_scale[0] = inverse_scale0;
+    p.inverse_scale[1] = inverse_scale1;
+    p.out_features = out_features;
+    p.in_features = in_features;
+    p.batch = batch;
+    const NativeSetup* setup = native_setup();
     if (setup == nullptr || setup->opted != cudaSuccess) {
         (void)take_next_projection();
         return setup == nullptr ? cudaErrorInvalidDevice : setup->opted;
@@ -1481,21 +1528,7 @@ cudaError_t launch_nvfp4_native(const void* packed0, const void* scales0, const 
     p.pair_tiles = (out_features + rows_per_pair - 1) / rows_per_pair;
     p.stages_in_k = in_features / (kChunkK * kStageChunks);
     p.units = p.pair_tiles * p.stages_in_k;
-    // Stages one after the other on the busiest SM, plus what a wave costs beside its stages and a
-    // cluster beside its slices (in stages).
-    p.splits = 1;
-    double best = 1e30;
-    for (int size = 1; size <= 8 && size <= p.stages_in_k; ++size) {
-        if (setup->clusters[size] <= 0) {
-            continue;
-        }
-        const int waves = (p.pair_tiles + setup->clusters[size] - 1) / setup->clusters[size];
-        const double cost = waves * ((p.stages_in_k + size - 1) / size + 3.0) + (size > 1 ? 1.0 : 0.0) + 0.2 * size;
-        if (cost < best) {
-            best = cost;
-            p.splits = size;
-        }
-    }
+    p.splits = native_splits(out_features, in_features, swiglu);
     CUtensorMap map0, map1;
     cudaError_t encoded = encode_weight_map(&map0, packed0, out_features, in_features / 2);
     if (encoded == cudaSuccess) {
@@ -1506,7 +1539,7 @@ cudaError_t launch_nvfp4_native(const void* packed0, const void* scales0, const 
         return encoded;
     }
     CUtensorMap next_map0 = map0, next_map1 = map1;
-    take_hint(p, next_map0, next_map1);
+    take_hint(p, next_map0, next_map1, [batch](const NextProjection& hint) { return rows_shape(hint, batch); });
     p.status = status_ptr();
     if (p.status == nullptr) {
         return cudaErrorInvalidValue;
@@ -1525,7 +1558,7 @@ cudaError_t launch_nvfp4_native(const void* packed0, const void* scales0, const 
     attributes[1].val.clusterDim.z = 1;
     config.attrs = attributes;
     config.numAttrs = p.splits > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&config, kernels[swiglu ? 1 : 0], map0, map1, next_map0, next_map1, p);
+    return cudaLaunchKernelEx(&config, native_kernels[swiglu ? 1 : 0], map0, map1, next_map0, next_map1, p);
 }
 
 namespace {

@@ -736,10 +736,80 @@ int sm_count_umma() {
     return sms;
 }
 
-}  // namespace
+constexpr int kSmemBytes =
+    kWeightStages * kTiles * kTileStageBytes + (kXStages + kXStages * kRawBuffers) * 32 * kChunkK * 2 + 1024;
+using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
+                        const UmmaParams);
+const Kernel kernels[12] = {
+    nvfp4_umma_kernel<false, false, 16, false>, nvfp4_umma_kernel<false, false, 32, false>,
+    nvfp4_umma_kernel<false, true, 16, false>,  nvfp4_umma_kernel<false, true, 32, false>,
+    nvfp4_umma_kernel<true, false, 16, false>,  nvfp4_umma_kernel<true, false, 32, false>,
+    nvfp4_umma_kernel<false, false, 16, true>,  nvfp4_umma_kernel<false, false, 32, true>,
+    nvfp4_umma_kernel<false, true, 16, true>,   nvfp4_umma_kernel<false, true, 32, true>,
+    nvfp4_umma_kernel<true, false, 16, true>,   nvfp4_umma_kernel<true, false, 32, true>};
 
+// Once per device: the kernels' shared memory, and how many clusters of each size are resident at once (a
+// cluster must sit inside one GPC, so the driver is asked).
+struct UmmaSetup {
+    cudaError_t opted;
+    int clusters[9];
+};
 
-namespace {
+const UmmaSetup* umma_setup() {
+    static PerDevice<UmmaSetup> per_device;
+    return per_device.get([]() {
+        UmmaSetup s = {};
+        for (const Kernel kernel : kernels) {
+            s.opted = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+            if (s.opted != cudaSuccess) {
+                return s;
+            }
+        }
+        s.clusters[1] = sm_count_umma();
+        for (int size = 2; size <= 8; ++size) {
+            cudaLaunchConfig_t probe = {};
+            probe.gridDim = dim3(size * 64);
+            probe.blockDim = dim3(kThreads);
+            probe.dynamicSmemBytes = kSmemBytes;
+            cudaLaunchAttribute attribute[1];
+            attribute[0].id = cudaLaunchAttributeClusterDimension;
+            attribute[0].val.clusterDim.x = size;
+            attribute[0].val.clusterDim.y = 1;
+            attribute[0].val.clusterDim.z = 1;
+            probe.attrs = attribute;
+            probe.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&s.clusters[size], kernels[7], &probe) != cudaSuccess) {
+                s.clusters[size] = 0;
+                (void)cudaGetLastError();
+            }
+        }
+        return s;
+    });
+}
+
+// K split: the slices of a row group form a cluster.  The cost of a plan is its waves times the chunks per
+// slice, plus a term for the reduction.
+int plan_splits(const UmmaSetup& setup, int out_features, int in_features, bool swiglu, bool fp8) {
+    const int rows_per_group = swiglu ? kTileRows : kTiles * kTileRows;
+    const int row_groups = (out_features + rows_per_group - 1) / rows_per_group;
+    const int chunks = in_features / kChunkK;
+    const int stage_chunks = fp8 ? 1 : kStageChunks;
+    int best = 1;
+    double best_cost = 1e30;
+    for (int size = 1; size <= 8; ++size) {
+        const int clusters = setup.clusters[size];
+        if (clusters <= 0 || (size > 1 && chunks / size < 2 * stage_chunks)) {
+            continue;
+        }
+        const int waves = (row_groups + clusters - 1) / clusters;
+        const double cost = waves * (static_cast<double>((chunks + size - 1) / size) + 6.0) + 1.5 * (size - 1);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = size;
+        }
+    }
+    return best;
+}
 
 // Fills the launch-dependent fields of p (its operand pointers and mode are the caller's) and launches.
 cudaError_t launch_umma(UmmaParams p, const void* x, int out_features, int in_features, int batch, bool swiglu,
@@ -779,88 +849,14 @@ cudaError_t launch_umma(UmmaParams p, const void* x, int out_features, int in_fe
             return cudaErrorInvalidValue;
         }
     }
-    const int smem_bytes =
-        kWeightStages * kTiles * kTileStageBytes + (kXStages + kXStages * kRawBuffers) * 32 * kChunkK * 2 + 1024;
-    using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
-                            const CUtensorMap, const UmmaParams);
-    static const Kernel kernels[12] = {
-        nvfp4_umma_kernel<false, false, 16, false>, nvfp4_umma_kernel<false, false, 32, false>,
-        nvfp4_umma_kernel<false, true, 16, false>,  nvfp4_umma_kernel<false, true, 32, false>,
-        nvfp4_umma_kernel<true, false, 16, false>,  nvfp4_umma_kernel<true, false, 32, false>,
-        nvfp4_umma_kernel<false, false, 16, true>,  nvfp4_umma_kernel<false, false, 32, true>,
-        nvfp4_umma_kernel<false, true, 16, true>,   nvfp4_umma_kernel<false, true, 32, true>,
-        nvfp4_umma_kernel<true, false, 16, true>,   nvfp4_umma_kernel<true, false, 32, true>};
-    static PerDevice<cudaError_t> opted_per_device;
-    const cudaError_t* opted_found = opted_per_device.get([smem_bytes]() {
-        for (const Kernel kernel : kernels) {
-            const cudaError_t error =
-                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-            if (error != cudaSuccess) {
-                return error;
-            }
-        }
-        return cudaSuccess;
-    });
-    if (opted_found == nullptr) {
+    const UmmaSetup* setup = umma_setup();
+    if (setup == nullptr) {
         return cudaErrorInvalidDevice;
     }
-    if (*opted_found != cudaSuccess) {
-        return *opted_found;
+    if (setup->opted != cudaSuccess) {
+        return setup->opted;
     }
-    // K split: the slices of a row group form a cluster, and a cluster must sit inside one GPC, so
-    // the number of clusters resident at once is asked of the driver per cluster size.  The cost of
-    // a plan is its waves times the chunks per slice, plus a term for the reduction.
-    struct Residency {
-        int clusters[9];
-    };
-    static PerDevice<Residency> residency_per_device;
-    const Residency* residency_found = residency_per_device.get([smem_bytes]() {
-        Residency r = {};
-        for (int size = 1; size <= 8; ++size) {
-            cudaLaunchConfig_t probe = {};
-            probe.gridDim = dim3(size * 64);
-            probe.blockDim = dim3(kThreads);
-            probe.dynamicSmemBytes = smem_bytes;
-            cudaLaunchAttribute attribute[1];
-            attribute[0].id = cudaLaunchAttributeClusterDimension;
-            attribute[0].val.clusterDim.x = size;
-            attribute[0].val.clusterDim.y = 1;
-            attribute[0].val.clusterDim.z = 1;
-            probe.attrs = attribute;
-            probe.numAttrs = 1;
-            int clusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&clusters, kernels[7], &probe) != cudaSuccess) {
-                clusters = 0;
-                (void)cudaGetLastError();
-            }
-            r.clusters[size] = clusters;
-        }
-        return r;
-    });
-    if (residency_found == nullptr) {
-        return cudaErrorInvalidDevice;
-    }
-    const Residency& residency = *residency_found;
-    const auto plan_splits = [&](int row_groups, int features_in, bool fp8) {
-        const int chunks = features_in / kChunkK;
-        const int stage_chunks = fp8 ? 1 : kStageChunks;
-        int best = 1;
-        double best_cost = 1e30;
-        for (int size = 1; size <= 8; ++size) {
-            const int clusters = size == 1 ? sm_count_umma() : residency.clusters[size];
-            if (clusters <= 0 || (size > 1 && chunks / size < 2 * stage_chunks)) {
-                continue;
-            }
-            const int waves = (row_groups + clusters - 1) / clusters;
-            const double cost = waves * (static_cast<double>((chunks + size - 1) / size) + 6.0) + 1.5 * (size - 1);
-            if (cost < best_cost) {
-                best_cost = cost;
-                best = size;
-            }
-        }
-        return best;
-    };
-    const int splits = plan_splits(p.row_groups, in_features, p.fp8 != 0);
+    const int splits = plan_splits(*setup, out_features, in_features, swiglu, p.fp8 != 0);
     p.splits = splits;
     // The caller's hint about the projection that follows (one use): its plan is made the way its own
     // launch will make it, so that this launch's CTAs ask for the boxes that launch starts with.
@@ -880,7 +876,9 @@ cudaError_t launch_umma(UmmaParams p, const void* x, int out_features, int in_fe
             p.next.swiglu = next_swiglu ? 1 : 0;
             p.next.nvfp4 = next_fp8 ? 0 : 1;
             p.next.out_features = hint.out_features;
-            p.next.splits = plan_splits(next_groups, hint.in_features, next_fp8);
+            p.next.splits = !next_fp8 && runs_in_four_bits(hint.out_features, hint.in_features, batch)
+                                ? native_splits(hint.out_features, hint.in_features, next_swiglu)
+                                : plan_splits(*setup, hint.out_features, hint.in_features, next_swiglu, next_fp8);
             p.next.ctas = next_groups * p.next.splits;
             p.next.stages_in_k = hint.in_features / (kChunkK * (next_fp8 ? 1 : kStageChunks));
             p.next.group_blocks = hint.in_features / 64;
@@ -895,7 +893,7 @@ cudaError_t launch_umma(UmmaParams p, const void* x, int out_features, int in_fe
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(p.row_groups * splits);
     config.blockDim = dim3(kThreads);
-    config.dynamicSmemBytes = smem_bytes;
+    config.dynamicSmemBytes = kSmemBytes;
     config.stream = stream;
     cudaLaunchAttribute attribute[2];
     attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -911,6 +909,11 @@ cudaError_t launch_umma(UmmaParams p, const void* x, int out_features, int in_fe
 }
 
 }  // namespace
+
+int umma_splits(int out_features, int in_features, bool swiglu, bool fp8) {
+    const UmmaSetup* setup = umma_setup();
+    return setup == nullptr ? 1 : plan_splits(*setup, out_features, in_features, swiglu, fp8);
+}
 
 cudaError_t launch_nvfp4_umma(const void* packed0, const void* scales0, const void* packed1, const void* scales1,
                               const void* x, void* y, int out_features, int in_features, int batch, float inverse0,
