@@ -324,12 +324,16 @@ __global__ void __launch_bounds__(kThreads, kLanes == 8 ? 7 : 4) delta_decode_in
 }
 
 int sm_count_delta() {
-    int device = 0, value = 0;
-    if (cudaGetDevice(&device) == cudaSuccess &&
-        cudaDeviceGetAttribute(&value, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && value > 0) {
+    static PerDevice<int> count_per_device;  // (a call of one row is bound by the host)
+    const int* found = count_per_device.get([]() {
+        int device = 0, value = 0;
+        if (cudaGetDevice(&device) != cudaSuccess ||
+            cudaDeviceGetAttribute(&value, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || value <= 0) {
+            value = 148;
+        }
         return value;
-    }
-    return 148;
+    });
+    return found == nullptr ? 148 : *found;
 }
 
 // Row splits so that the grid has at least two CTAs per SM
