@@ -41,7 +41,8 @@ namespace cg = cooperative_groups;
 
 namespace qwc {
 
-// tcgen05 paths (nvfp4_umma.cu): NVFP4 projections, and the e4m3 vocabulary head.
+// tcgen05 paths: NVFP4 projections in four bits (nvfp4_native.cuh; the launcher is in nvfp4_streamk.cu), in f16,
+// and the e4m3 vocabulary head (both nvfp4_umma.cu).
 cudaError_t launch_nvfp4_native(const void* packed0, const void* scales0, const void* packed1, const void* scales1,
                                 const __nv_bfloat16* x, __nv_bfloat16* y, int out_features, int in_features, int batch,
                                 float inverse_scale0, float inverse_scale1, bool swiglu, cudaStream_t stream);
@@ -658,11 +659,7 @@ template <int MODE>
 cudaError_t dispatch(const GemvParams& p, cudaStream_t stream) {
     const int wide_tiles = ((p.out_features + 127) / 128) * 4;
     const bool wide = MODE == kNvfp4 && wide_tiles >= 2 * sm_count();
-    // The tcgen05 kernel streams weights faster than the mma.sync one at every batch size but has a
-    // longer start-up (TMEM allocation, first TMA round trip, cluster reduction): it takes over
-    // above eight rows, and below that for vocabulary heads of 60 MB and more.
-    const bool large = static_cast<long long>(p.out_features) * p.in_features >= 60ll * 1000 * 1000;
-    // its stores are 16 bytes wide and its activation fetch is a tiled TMA copy
+    // the tcgen05 kernels' stores are 16 bytes wide and its activation fetch is a tiled TMA copy
     const bool aligned = p.out_features % 8 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0 &&
                          (reinterpret_cast<uintptr_t>(p.x) & 15) == 0 &&
                          ((reinterpret_cast<uintptr_t>(p.packed[0]) | reinterpret_cast<uintptr_t>(p.packed[1]) |
@@ -678,8 +675,13 @@ cudaError_t dispatch(const GemvParams& p, cudaStream_t stream) {
                                    p.in_features, p.batch, p.inverse_scale[0], p.inverse_scale[1],
                                    MODE == kNvfp4Swiglu, stream);
     }
-    if (p.batch <= 8 && !(large && aligned)) {
-        (void)take_next_projection();  // only the tcgen05 kernel acts on the hint; it is good for one launch
+    // The f16 tcgen05 kernel streams weights faster than the mma.sync one at every batch size but has a
+    // longer start-up (TMEM allocation, first TMA round trip, cluster reduction): it takes over
+    // above eight rows, and below that for vocabulary heads of 60 MB and more.
+    const bool large_head =
+        MODE == kFp8Rows && static_cast<long long>(p.out_features) * p.in_features >= 60ll * 1000 * 1000;
+    if (p.batch <= 8 && !(large_head && aligned)) {
+        (void)take_next_projection();  // only the tcgen05 kernels act on the hint; it is good for one launch
         return launch<1, 1, MODE>(p, stream);
     }
     if (MODE == kFp8Rows && aligned) {

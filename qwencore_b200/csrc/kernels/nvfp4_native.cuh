@@ -62,7 +62,6 @@ struct NativeBarriers {
     uint64_t x_full[kNativeMaxXSlots];
     uint64_t x_empty[kNativeMaxXSlots];
     uint64_t done;
-    uint64_t tmem_ready;
     uint32_t tmem_base;
     uint32_t rest[kNativeMaxXSlots];  // byte w: warp w of the slot's team wrote the second eight digits
     int rest_used;
@@ -289,7 +288,6 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
         }
         bars.rest_used = 0;
         mbar_init(&bars.done, 1);
-        mbar_init(&bars.tmem_ready, 1);
         bars.failed = status_is_set(p.status) ? 1 : 0;
         bars.tmem_base = 0;
         mbar_fence_init();
@@ -324,9 +322,6 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) {
-            mbar_arrive(&bars.tmem_ready);
-        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars.tmem_base);
         // A and B e2m1 (1), scales e4m3, fp32 accumulators, M = 128
