@@ -351,13 +351,14 @@ int splits_for(int batch, int v_heads) {
 using DeltaKernel = void (*)(int8_t*, float*, const uint32_t*, const float*, const float*, const float*, const float*,
                              const float*, const float*, float*, int, int, int*, const GatedNorm);
 
-// Four lanes per row (123 registers) while every CTA is resident at once with them, four per SM; eight (71
-// registers, seven CTAs per SM) beyond.  Measured (us, layers that L2 does not hold, four / eight lanes): 48
-// heads at 1 row 3.62 / 4.90, at 9 rows (432 CTAs) 8.28 / 12.00, at 12 rows (576) 8.70 / 12.54; 32 heads at 32
-// rows (1024 CTAs, two waves of the first) 14.55 / 13.97.
+// Four lanes per row (123 registers) while every CTA is resident at once with them, four per SM, or hardly more;
+// eight (71 registers, seven CTAs per SM) beyond.  Measured (us, layers that L2 does not hold, four / eight
+// lanes): 48 heads at 1 row 3.62 / 4.90, at 9 rows (432 CTAs) 8.28 / 12.00, at 12 rows (576) 8.70 / 12.54; 32 heads
+// at 20 rows (640) 11.7 / 12.7, at 22 rows (704) 12.6 / 12.9, at 23 rows (736) 13.1 / 13.0, at 32 rows (1024) 14.6 /
+// 14.0; 48 heads at 15 rows (720) 12.9 / 12.9.
 template <bool kEarly>
 DeltaKernel kernel_for(int ctas) {
-    return ctas <= 4 * sm_count_delta() ? delta_decode_int8_kernel<kEarly, 4> : delta_decode_int8_kernel<kEarly, 8>;
+    return 4 * ctas <= 19 * sm_count_delta() ? delta_decode_int8_kernel<kEarly, 4> : delta_decode_int8_kernel<kEarly, 8>;
 }
 
 }  // namespace

@@ -367,7 +367,7 @@ def test_delta_decode_int8_matches_oracle(cuda, ops, batch, v_heads):
         assert np.array_equal(scales[slot], case["scales"][slot])
 
 
-@pytest.mark.parametrize("batch,v_heads", [(18, 32), (19, 32), (12, 48), (13, 48), (1, 32), (2, 32), (3, 48)],
+@pytest.mark.parametrize("batch,v_heads", [(21, 32), (22, 32), (14, 48), (15, 48), (1, 32), (2, 32), (3, 48)],
                          ids=["last_four_lanes", "first_eight_lanes", "last_four_lanes_h48", "first_eight_lanes_h48",
                               "row_split_16", "row_split_8", "row_split_4"])
 @pytest.mark.parametrize("exponent", [0, -100, 92], ids=["unit_q", "tiny_q", "huge_q"])
@@ -392,7 +392,7 @@ def test_delta_decode_both_forms(cuda, ops, batch, v_heads, exponent):
     assert np.allclose(scales, want_scales, rtol=1e-5, atol=0)
 
 
-@pytest.mark.parametrize("batch,v_heads", [(3, 32), (19, 32)], ids=["four_lanes", "eight_lanes"])
+@pytest.mark.parametrize("batch,v_heads", [(3, 32), (24, 32)], ids=["four_lanes", "eight_lanes"])
 @pytest.mark.parametrize("vector", ["k", "q"])
 def test_delta_dot_products_keep_small_elements_beside_an_outlier(cuda, ops, batch, v_heads, vector):
     """k (then q) holds a 1 where every state row's code is 0, and elements of 1e-5 to 1e-8 elsewhere: the dot
@@ -421,7 +421,7 @@ def test_delta_dot_products_keep_small_elements_beside_an_outlier(cuda, ops, bat
     assert np.all(np.abs(out - want) <= bound)
 
 
-@pytest.mark.parametrize("batch", [3, 19], ids=["four_lanes", "eight_lanes"])
+@pytest.mark.parametrize("batch", [3, 24], ids=["four_lanes", "eight_lanes"])
 @pytest.mark.parametrize("value", [np.nan, np.inf])
 def test_delta_non_finite_key_stays_in_its_head(cuda, ops, value, batch):
     v_heads = 32
