@@ -75,8 +75,22 @@ NextProjection take_next_projection();
 // Rows in memory as bf16: which kernel a projection of `batch` rows runs on (nvfp4_gemv.cu: dispatch), and into
 // how many K slices the two kernels that start from a ring of weight stages cut it.  A launch that has been told
 // what follows asks L2 for the stages that those slices begin with.
-inline bool runs_in_four_bits(int out_features, int in_features, int batch) {
-    return batch <= 8 && static_cast<long long>(out_features) * in_features >= 16ll * 1000 * 1000;
+//
+// Four bits up to eight rows, unless the matrix is so small that the kernel's start-up shows.  Measured (us at 1,
+// 4 and 8 rows, other kernel / four bits, activations of a dozen launches): 8192 x 2048 (16.8 M) 5.7, 5.9, 6.0 /
+// 6.2, 6.4, 7.4; 4096 x 4096 6.6, 6.9, 7.2 / 6.2, 7.1, 7.7; 20480 x 1024 (21 M) 6.4, 6.5, 6.5 / 5.4, 5.9, 6.5;
+// 10240 x 2048 7.7, 7.7, 7.8 / 6.5, 7.4, 8.1; 5120 x 4096 8.1, 8.2, 8.3 / 6.8, 7.4, 8.2; 6144 x 4096 (25 M) 8.6,
+// 8.7, 8.8 / 7.2, 7.8, 8.8; 65536 x 512 (34 M, two stages) 9.6, 9.7, 9.9 / 9.0, 9.1, 10.5.  A SwiGLU pair streams
+// twice the bytes per output and gains at every size tried: 8192 x 2048 10.6, 10.8, 10.9 / 7.8, 8.7, 10.1, 34816 x
+// 512 11.1, 11.5, 11.5 / 8.6, 9.0, 10.2.  Above eight rows the digits take longer than the weights (34816 x 5120 at
+// 16 rows 24.6 / 30.3).
+inline bool runs_in_four_bits(int out_features, int in_features, int batch, bool swiglu) {
+    const long long weights = static_cast<long long>(out_features) * in_features;
+    if (swiglu) {
+        return batch <= 8 && weights >= 16ll * 1000 * 1000;
+    }
+    return batch <= 4 ? weights >= 20ll * 1000 * 1000
+                      : batch <= 8 && weights >= 24ll * 1000 * 1000 && in_features >= 1024;
 }
 int native_splits(int out_features, int in_features, bool swiglu);          // nvfp4_native.cuh
 int umma_splits(int out_features, int in_features, bool swiglu, bool fp8);  // nvfp4_umma.cu

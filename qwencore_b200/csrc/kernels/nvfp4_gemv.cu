@@ -666,11 +666,8 @@ cudaError_t dispatch(const GemvParams& p, cudaStream_t stream) {
                            reinterpret_cast<uintptr_t>(p.scales[0]) | reinterpret_cast<uintptr_t>(p.scales[1])) & 15) == 0 &&
                          (MODE != kFp8Rows || ((reinterpret_cast<uintptr_t>(p.y_f32) & 15) == 0 &&
                                                (reinterpret_cast<uintptr_t>(p.row_scales) & 15) == 0));
-    // Up to eight rows both operands enter the tensor cores in four bits (nvfp4_native.cuh), unless the
-    // matrix is so small that its start-up shows.  Measured (us, mma.sync or f16 tcgen05 / four bits):
-    // 1040 x 512 at 1 and 8 rows 3.1, 3.8 / 3.8, 4.7; 5120 x 4096 8.1, 8.2 / 6.1, 7.4; 34816 x 5120 25.7,
-    // 24.5 / 20.7, 21.6; above eight rows the digits take longer than the weights (16: 24.6 / 30.3).
-    if (MODE != kFp8Rows && aligned && runs_in_four_bits(p.out_features, p.in_features, p.batch)) {
+    // Both operands in four bits (nvfp4_native.cuh): the rule and its figures are in common.cuh.
+    if (MODE != kFp8Rows && aligned && runs_in_four_bits(p.out_features, p.in_features, p.batch, MODE == kNvfp4Swiglu)) {
         return launch_nvfp4_native(p.packed[0], p.scales[0], p.packed[1], p.scales[1], p.x, p.y, p.out_features,
                                    p.in_features, p.batch, p.inverse_scale[0], p.inverse_scale[1],
                                    MODE == kNvfp4Swiglu, stream);

@@ -876,7 +876,7 @@ cudaError_t launch_umma(UmmaParams p, const void* x, int out_features, int in_fe
             p.next.swiglu = next_swiglu ? 1 : 0;
             p.next.nvfp4 = next_fp8 ? 0 : 1;
             p.next.out_features = hint.out_features;
-            p.next.splits = !next_fp8 && runs_in_four_bits(hint.out_features, hint.in_features, batch)
+            p.next.splits = !next_fp8 && runs_in_four_bits(hint.out_features, hint.in_features, batch, next_swiglu)
                                 ? native_splits(hint.out_features, hint.in_features, next_swiglu)
                                 : plan_splits(*setup, hint.out_features, hint.in_features, next_swiglu, next_fp8);
             p.next.ctas = next_groups * p.next.splits;

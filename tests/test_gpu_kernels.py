@@ -806,7 +806,7 @@ def test_page_table_apply_edits(cuda, ops):
 # ---------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("out_features,in_features,batch", [(5128, 4096, 1), (5120, 4096, 2), (5120, 4096, 3),
-                                                            (1040, 17408, 5), (5120, 4096, 8), (34816, 512, 7)])
+                                                            (1400, 17408, 5), (5120, 6144, 8), (34816, 1024, 7)])
 @pytest.mark.parametrize("std", [1.0, 3000.0, 1e-3], ids=["unit", "large", "small"])
 def test_four_bit_projection_matches_oracle(cuda, ops, out_features, in_features, batch, std):
     """Every padding of the activation rows, ragged last tiles, one and several K slices, block scales of
@@ -858,7 +858,7 @@ def dequantize(packed, scales):
     return values[codes] * np.repeat(synth.e4m3_decode(scales).astype(np.float64), 16, axis=1)
 
 
-@pytest.mark.parametrize("out_features,in_features", [(5120, 4096), (34816, 512)], ids=["k_slices", "one_slice"])
+@pytest.mark.parametrize("out_features,in_features", [(5120, 6144), (34816, 1024)], ids=["k_slices", "one_slice"])
 @pytest.mark.parametrize("batch", [1, 2, 3, 4, 5, 8])
 def test_four_bit_projection_keeps_small_activations_beside_large(cuda, ops, out_features, in_features, batch):
     """Every block of sixteen holds one large activation (up to f16's largest binade) where the weights are 0,
@@ -884,7 +884,7 @@ def test_four_bit_projection_keeps_small_activations_beside_large(cuda, ops, out
     assert np.all(np.abs(got - want) <= bound)
 
 
-@pytest.mark.parametrize("in_features", [4096, 17408])
+@pytest.mark.parametrize("in_features", [6144, 17408])
 def test_four_bit_projection_rounds_no_more_than_the_f16_kernel(cuda, ops, in_features):
     """Every block of sixteen features is there twice with opposite weights, shuffled over K: the exact result is
     0, and a call returns its own rounding.  Nine rows run on the f16 kernel, eight of them in four bits."""
@@ -952,7 +952,7 @@ def test_four_bit_projection_with_a_hint_stores_the_same_bytes(cuda, ops, batch,
     assert abi.lib.qwc_device_status() == 0
 
 
-@pytest.mark.parametrize("out_features,in_features", [(5120, 4096), (34816, 512)], ids=["k_slices", "one_slice"])
+@pytest.mark.parametrize("out_features,in_features", [(5120, 6144), (34816, 1024)], ids=["k_slices", "one_slice"])
 @pytest.mark.parametrize("swiglu", [False, True], ids=["plain", "swiglu"])
 def test_four_bit_projection_stores_nothing_once_a_wait_has_given_up(cuda, ops, out_features, in_features, swiglu):
     """With the status word set (as an earlier kernel leaves it), as the other projection kernels do."""
