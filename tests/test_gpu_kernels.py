@@ -810,7 +810,7 @@ def test_page_table_apply_edits(cuda, ops):
 @pytest.mark.parametrize("std", [1.0, 3000.0, 1e-3], ids=["unit", "large", "small"])
 def test_four_bit_projection_matches_oracle(cuda, ops, out_features, in_features, batch, std):
     """Every padding of the activation rows, ragged last tiles, one and several K slices, block scales of
-    either sign, blocks whose activations differ by nine orders of magnitude, and saturation at 65504."""
+    either sign, blocks whose activations differ by nine orders of magnitude, f16's largest binade, and a NaN."""
     torch = cuda
     packed, scales, _ = synth.nvfp4_matrix(41, "four_bit", out_features, in_features)
     flip = synth.generator(41, "signs").random(scales.shape) < 0.02
@@ -834,6 +834,24 @@ def test_four_bit_projection_matches_oracle(cuda, ops, out_features, in_features
     torch.cuda.synchronize()
     assert np.isnan(synth.bf16_value(host(out))[batch - 1]).all()
     assert np.array_equal(host(out)[: batch - 1], clean[: batch - 1])
+
+
+def test_four_bit_projection_saturates_at_the_largest_f16(cuda, ops):
+    """Rows with values beyond 65504, with an infinity of either sign, and an ordinary one: the infinities become
+    65504 like the rest (only NaN poisons).  Bound: half a bf16 step, one rounding of the magnitudes per 64 features."""
+    torch = cuda
+    out_features, in_features = 5120, 4096
+    packed, scales, swizzled = synth.nvfp4_matrix(47, "saturate", out_features, in_features)
+    x = synth.normal_bf16(47, "x", (4, in_features))
+    x[0, 3::97] = synth.bf16_bits(np.resize(np.array([1e6, -7e4, 65536.0, -3e38], dtype=np.float32), x[0, 3::97].size))
+    x[1, 1000] = synth.bf16_bits(np.array([np.inf], dtype=np.float32))[0]
+    x[2, 17] = synth.bf16_bits(np.array([-np.inf], dtype=np.float32))[0]
+    exact = np.clip(synth.bf16_value(x).astype(np.float64), -65504.0, 65504.0)
+    weights = dequantize(packed, scales)
+    got, _ = run_gemv(torch, ops, packed, scales, swizzled, 1.0, x, out_features, in_features, 4)
+    want = exact @ weights.T
+    bound = 2.0 ** -8 * np.abs(want) + (in_features / 64) * 2.0 ** -24 * (np.abs(exact) @ np.abs(weights).T)
+    assert np.all(np.abs(got - want) <= bound)
 
 
 def test_four_bit_swiglu_matches_oracle(cuda, ops):
