@@ -7,8 +7,9 @@
 // its bytes need from HBM, and the stages in the ring are still to be widened when the last byte has
 // landed.  Here nobody touches a weight: the end of the launch follows the last byte, and what bounds the
 // kernel is the weight stream, between a start and a tail of about 3 us.  Measured (us, bf16 rows in, layers
-// that L2 does not hold, f16 / four bits at one and at eight rows): 34816 x 5120 26.3 / 20.7 (4.9 TB/s) and
-// 24.0 / 22.6, 5120 x 17408 16.5 / 12.9 and 17.0 / 15.1, 12352 x 5120 13.2 / 10.6 and 13.5 / 12.4.
+// that L2 does not hold, a dozen different activations, f16 / four bits at one and at eight rows): 34816 x 5120
+// 22.8 / 18.9 (5.3 TB/s) and 21.0 / 20.4, 5120 x 17408 15.7 / 12.8 and 16.3 / 15.4, 5120 x 6144 10.9 / 7.8 and
+// 11.1 / 9.7.
 //
 // Not above eight rows, and not for staged activations inside a decode step: making digits costs about 25
 // instructions per activation in every CTA, after the activations have arrived.  At sixteen rows that

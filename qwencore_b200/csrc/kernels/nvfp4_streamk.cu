@@ -1489,7 +1489,7 @@ int native_splits(int out_features, int in_features, bool swiglu) {
     const int stages_in_k = in_features / (kChunkK * kStageChunks);
     // Stages one after the other on the busiest SM, plus what a wave costs beside its stages and a
     // cluster beside its slices (in stages).  Forced to 1 .. 8 slices over thirteen shapes (3336 x 5120 to
-    // 34816 x 5120, matrix and pair, one and eight rows), the choice is the fastest or within 3 % of it.
+    // 34816 x 5120, matrix and pair, one and eight rows), the choice is the fastest or within 4 % of it.
     int splits = 1;
     double best = 1e30;
     for (int size = 1; setup != nullptr && size <= 8 && size <= stages_in_k; ++size) {
