@@ -119,6 +119,9 @@ struct StreamKParams {
     // slice (a CTA per tile pair: matrices with about as many pairs as SMs) the CTA finishes its pair
     // itself.  0 splits: equal shares with tickets.
     int splits;
+    uint32_t split_inverse;  // ceil(2^32 / splits): quotients of small numbers without a division
+    int slice_stages;        // stages_in_k / splits ...
+    int slice_rest;          // ... and what is left
     float* split_out;
     // Latency mode (one activation row, weight rows split over ranks): the slices go to every rank's
     // exchange block as tagged words instead (exchange.cuh); split_out is null then.
@@ -178,7 +181,6 @@ struct Barriers {
     uint64_t x_free[kXStages];
     uint64_t d_ready[kAccumulatorBuffers];
     uint64_t d_free[kAccumulatorBuffers];
-    uint64_t tmem_ready;
     uint32_t tmem_base;
     int failed;
 };
@@ -231,6 +233,16 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 // First unit of CTA `cta` when `units` units are shared by `ctas` CTAs.
 __device__ __forceinline__ int share_begin(int units, int cta, int ctas) {
     return static_cast<int>(static_cast<long long>(units) * cta / ctas);
+}
+
+// n / splits for n < 65536 (splits <= 8; the rounding error of the inverse stays below 1 / splits).
+__device__ __forceinline__ int split_quotient(const StreamKParams& p, int n) {
+    return p.splits == 1 ? n : static_cast<int>(__umulhi(static_cast<uint32_t>(n), p.split_inverse));
+}
+
+// stages_in_k * slice / splits
+__device__ __forceinline__ int slice_begin(const StreamKParams& p, int slice) {
+    return p.slice_stages * slice + split_quotient(p, p.slice_rest * slice);
 }
 
 // The CTA whose share holds unit `unit` (ctas <= units, so no share is empty).
@@ -384,19 +396,20 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int ctas = gridDim.x;
     const int S = p.stages_in_k;
     constexpr int stage_chunks = kFp8 ? 1 : kStageChunks;  // 128 bytes per row and stage either way
-    int u_begin, u_end;
+    int u_begin, u_end, pair_first;
     if (kSplitOut) {
-        const int pair = cta / p.splits;
-        const int slice = cta - pair * p.splits;
-        u_begin = pair * S + S * slice / p.splits;
-        u_end = pair * S + S * (slice + 1) / p.splits;
+        // (no divisions: every CTA of a launch stands at this point before its first weight is asked for)
+        pair_first = split_quotient(p, cta);
+        const int slice = cta - pair_first * p.splits;
+        u_begin = pair_first * S + slice_begin(p, slice);
+        u_end = pair_first * S + slice_begin(p, slice + 1);
     } else {
         u_begin = share_begin(p.units, cta, ctas);
         u_end = share_begin(p.units, cta + 1, ctas);
+        pair_first = u_begin / S;
     }
     const int num_units = u_end - u_begin;
     const int total_chunks = num_units * stage_chunks;
-    const int pair_first = u_begin / S;
     const int stage_first = u_begin - pair_first * S;
     const int group_blocks = p.in_features / 64;
     constexpr int x_chunk_bytes = kPad * kChunkK * 2;
@@ -430,24 +443,29 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
     };
-    // The first trip round the weight ring does not wait for the rest of the CTA: the producer's
-    // thread sets up the ring's own barriers and asks for the first stages before the CTA-wide barrier
-    // (weights are never written during a step, so nothing has to be waited for either).
-    const int early_stages = num_units < kWeightStages ? num_units : kWeightStages;
+    // The first stage does not wait for the rest of the CTA: the producer's thread sets up the ring's own
+    // barriers and asks for it before the CTA-wide barrier (weights are never written during a step, so
+    // nothing has to be waited for either).  Only the first: asking takes 0.15 us a stage, and the other
+    // warps, the one that fetches activations among them, stand at the barrier meanwhile.  Nothing else that
+    // takes time lies before that barrier: no division, no look at the status word, tensor memory is
+    // allocated by a warp with nothing else to do.  CTA entry to the end of the barrier 1.5 -> 0.54 us, to the
+    // first MMA 3.2 -> 2.4 us (5120 x 17408 at one row); launches back to back at one row, us: 5120 x 4096
+    // 5.66 -> 5.04, 5120 x 17408 11.9 -> 11.2, 12352 x 5120 9.7 -> 9.2, gate and up 20.3 -> 19.9.
+    constexpr int early_stages = 1;
     if (threadIdx.x == kProducerWarp * 32) {
         for (int s = 0; s < kWeightStages; ++s) {
             mbar_init(&bars.w_full[s], 1);
             mbar_init(&bars.w_empty[s], kFp8 ? kRowWarps : kDequantWarps);  // warps that read a stage
         }
         mbar_fence_init();
-        int pair = pair_first, stage = stage_first;
-        for (int index = 0; index < early_stages; ++index) {
-            issue_stage(index, pair, stage);
-            if (++stage == S) {
-                stage = 0;
-                ++pair;
-            }
-        }
+        issue_stage(0, pair_first, stage_first);
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars.tmem_base)),
+                     "r"(kTmemColumns)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
     if (threadIdx.x == 0) {
         for (int t = 0; t < kTiles; ++t) {
@@ -464,36 +482,20 @@ __global__ void __launch_bounds__(kThreads, 1)
             mbar_init(&bars.d_ready[b], kMmaWarps);
             mbar_init(&bars.d_free[b], kEpilogueWarps);
         }
-        mbar_init(&bars.tmem_ready, 1);
-        bars.failed = status_is_set(p.status) ? 1 : 0;
-        bars.tmem_base = 0;
+        bars.failed = 0;
         mbar_fence_init();
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         QWC_TRACE(1);  // barriers set up
     }
-    // Tensor memory is allocated while the producer already fetches weights; the warps that use it
-    // wait for the address below.
-    uint32_t tmem_base = 0;
-    if (warp == kMmaWarp) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars.tmem_base)),
-                     "r"(kTmemColumns)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) {
-            mbar_arrive(&bars.tmem_ready);
-        }
+    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars.tmem_base);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // (by a thread with nothing to do yet: whoever has to wait from here on looks at the flag)
+    if (threadIdx.x == kThreads - 1 && status_is_set(p.status)) {
+        *reinterpret_cast<volatile int*>(&bars.failed) = 1;
     }
-    bool tmem_ok = true;
-    if (warp != kProducerWarp && warp != kXWarp) {
-        tmem_ok = sk_wait(&bars.tmem_ready, 0, &bars, p.status);
-        tmem_ok = __all_sync(0xffffffffu, tmem_ok);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars.tmem_base);
-    }
+    int issued = early_stages;  // copies the producer of the weights / of the activations has asked for
 
     if (warp < kDequantWarps) {
         // ---------------- dequantise: thread = row ----------------
@@ -505,7 +507,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int row_offset = local_row * kBoxRowBytes;
         const int row_swizzle = local_row & 7;
         const int scale_offset = (local_row & 31) * 16 + (local_row >> 5) * 4;
-        bool ok = tmem_ok;
+        bool ok = true;
         for (int c = set; c < total_chunks && ok; c += kDequantSets) {
             const int wstage = kFp8 ? c : c / kStageChunks;
             const int slot = wstage % kWeightStages;
@@ -607,8 +609,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ---------------- producer: weights and scales ----------------
         bool ok = true;
         int pair = pair_first, stage = stage_first + early_stages;
-        while (stage >= S) {
-            stage -= S;
+        if (stage == S) {
+            stage = 0;
             ++pair;
         }
         for (int index = early_stages; index < num_units && ok; ++index) {
@@ -622,6 +624,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 issue_stage(index, pair, stage);
             }
             __syncwarp();
+            issued = index + 1;
             if (++stage == S) {
                 stage = 0;
                 ++pair;
@@ -643,7 +646,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint64_t desc_stage = static_cast<uint64_t>(kXStageBytes >> 4);
         const uint32_t a_tile = tmem_base + t * kTileColumns;
         const uint32_t d_tile = a_tile + kAccumulatorColumn;
-        bool ok = tmem_ok;
+        bool ok = true;
         int buf = 0, xs = 0;
         uint32_t a_parity = 0, x_parity = 0;
         int stage = stage_first;
@@ -710,6 +713,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ---------------- activation chunks ----------------
         // Everything above starts before the kernel that produces the activations has finished; these
         // loads (and the epilogue's stores) wait for it.
+        issued = 0;
         pdl_wait();
         QWC_TRACE_LANE0(22);  // the previous kernel has finished
         bool ok = true;
@@ -732,6 +736,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                          x_chunk_bytes, &bars.x_full[xs]);
             }
             __syncwarp();
+            issued = c + 1;
             if (in_stage == stage_chunks - 1 && ++stage == S) {
                 stage = 0;
             }
@@ -751,7 +756,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t best_index = UINT32_MAX;
         const bool sampling = kFp8 && p.candidate_values != nullptr;
         float* stash = stash_base + e * kStashWarpFloats + lane;
-        bool ok = tmem_ok;
+        bool ok = true;
 
         // Scales the finished tile pair in the stash, combines (SwiGLU), rounds and stores the activation
         // rows below `batch`.  batch == 0 is the rehearsal (below): every instruction runs, for every
@@ -1105,26 +1110,22 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
     }
 
-    // A CTA that gave up must not return while the stages it asked for before the barrier are still
-    // landing in its shared memory: their thread waits for them, with a limit of 0.2 ms per ring slot
-    // (a stage that was consumed has completed its first phase long ago and the wait falls through).
+    // A CTA that gave up must not return while copies it asked for are still landing in its shared memory:
+    // the warps that asked wait for the last trip round their ring, with a limit of 0.2 ms per slot (a copy
+    // that was consumed has completed its phase long ago and the wait falls through).
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (threadIdx.x == 0) {
         QWC_TRACE(21);  // every role done
     }
     const bool failed = *reinterpret_cast<volatile int*>(&bars.failed) != 0;
-    if (failed && threadIdx.x == kProducerWarp * 32) {
-        for (int slot = 0; slot < early_stages; ++slot) {
+    if (failed && (threadIdx.x == kProducerWarp * 32 || threadIdx.x == kXWarp * 32)) {
+        const bool weights = threadIdx.x == kProducerWarp * 32;
+        const int slots = weights ? kWeightStages : kXStages;
+        for (int i = issued > slots ? issued - slots : 0; i < issued; ++i) {
+            uint64_t* full = weights ? &bars.w_full[i % slots] : &bars.x_full[i % slots];
             const long long start = clock64();
-            while (!mbar_try_wait(&bars.w_full[slot], 0) && clock64() - start < 400000ll) {
-            }
-        }
-    }
-    if (failed && threadIdx.x == kXWarp * 32) {
-        for (int slot = 0; slot < kXStages; ++slot) {
-            const long long start = clock64();
-            while (!mbar_try_wait(&bars.x_full[slot], 0) && clock64() - start < 400000ll) {
+            while (!mbar_try_wait(full, (i / slots) & 1) && clock64() - start < 400000ll) {
             }
         }
     }
@@ -1380,6 +1381,11 @@ cudaError_t launch_streamk(StreamKParams p, const void* packed0, const void* pac
     p.stages_in_k = shape.stages_in_k;
     p.units = shape.units;
     p.splits = shape.splits;
+    if (shape.splits > 0) {
+        p.split_inverse = static_cast<uint32_t>(((1ull << 32) + shape.splits - 1) / shape.splits);
+        p.slice_stages = shape.stages_in_k / shape.splits;
+        p.slice_rest = shape.stages_in_k % shape.splits;
+    }
     unsigned char* base = static_cast<unsigned char*>(workspace);
     p.partials = reinterpret_cast<float*>(base);
     p.tickets = shape.splits > 0 ? nullptr : reinterpret_cast<int*>(base + kPartialBytes);
