@@ -32,6 +32,7 @@ namespace {
 
 constexpr int kDim = kDeltaHeadDim;  // 128 x 128 state per head
 constexpr int kThreads = 128;
+static_assert(kThreads == kDim, "thread i fetches row i of v");
 constexpr int kPartRows = 32;        // rows per bulk copy / per CTA iteration
 constexpr int kMaxParts = kDim / kPartRows;
 
@@ -66,9 +67,6 @@ __global__ void __launch_bounds__(kThreads, kLanes == 8 ? 7 : 4) delta_decode_in
     const float* __restrict__ alpha, const float* __restrict__ beta, const float* __restrict__ kq,
     float* __restrict__ out, int v_heads, int state_capacity, int* status, const GatedNorm norm) {
     pdl_launch_dependents();
-    if (!kEarly) {
-        pdl_wait();
-    }
     __shared__ __align__(128) uint8_t tile[kDim * kDim];
     __shared__ __align__(16) float row_scale[kDim];
     __shared__ float out_rows[kDim];
@@ -76,14 +74,43 @@ __global__ void __launch_bounds__(kThreads, kLanes == 8 ? 7 : 4) delta_decode_in
     __shared__ uint64_t bars[kMaxParts];
     __shared__ int failed;
 
-    if (status_is_set(status)) {
-        return;
-    }
     const int h = blockIdx.x;
     const int b = blockIdx.y;
     const int rows_here = kDim / gridDim.z;
     const int row_begin = blockIdx.z * rows_here;
-    const int slot = state_slots == nullptr ? b : static_cast<int>(state_slots[b]);
+    const int hk = h / (v_heads / kDeltaKeyHeads);
+    const int parts = (rows_here + kPartRows - 1) / kPartRows;
+    const int part_rows = rows_here < kPartRows ? rows_here : kPartRows;
+    if (threadIdx.x == 0) {
+        failed = 0;
+        for (int part = 0; part < parts; ++part) {
+            mbar_init(&bars[part], 1);
+        }
+        mbar_fence_init();
+    }
+    if (!kEarly) {
+        // The slot as it stands now may still be rewritten by an earlier kernel, and so may the state: both are
+        // read for good after the wait.  But usually they stay, and then the tile is in L2 by that time: it
+        // comes in while the kernel before this one writes its last tiles back (eight launches over layers that
+        // L2 does not hold, 32 heads x 32 rows: 119 -> 106 us).
+        if (threadIdx.x == 0) {
+            const uint32_t likely =
+                state_slots == nullptr ? static_cast<uint32_t>(b) : *const_cast<const volatile uint32_t*>(state_slots + b);
+            if (likely < static_cast<uint32_t>(state_capacity)) {
+                const size_t row = (static_cast<size_t>(likely) * v_heads + h) * kDim + row_begin;
+                bulk_prefetch_l2(state + row * kDim, rows_here * kDim);
+                bulk_prefetch_l2(state_scales + row, rows_here * 4);
+            }
+        }
+        pdl_wait();
+    }
+    // (both in flight at once)
+    const int earlier_failure = *reinterpret_cast<const volatile int*>(status);
+    const int slot =
+        state_slots == nullptr ? b : static_cast<int>(*const_cast<const volatile uint32_t*>(state_slots + b));
+    if (earlier_failure != 0) {
+        return;
+    }
     if (static_cast<uint32_t>(slot) >= static_cast<uint32_t>(state_capacity)) {
         // a slot beyond the pool: nothing of this row is read or written, the host learns of it
         // through the status word (the whole CTA takes this branch: the slot is per row)
@@ -92,21 +119,10 @@ __global__ void __launch_bounds__(kThreads, kLanes == 8 ? 7 : 4) delta_decode_in
         }
         return;
     }
-    const int hk = h / (v_heads / kDeltaKeyHeads);
-    const int parts = (rows_here + kPartRows - 1) / kPartRows;
-    const int part_rows = rows_here < kPartRows ? rows_here : kPartRows;
 
     int8_t* S = state + (static_cast<size_t>(slot) * v_heads + h) * (kDim * kDim) + row_begin * kDim;
     float* scales = state_scales + (static_cast<size_t>(slot) * v_heads + h) * kDim + row_begin;
 
-    if (threadIdx.x == 0) {
-        failed = 0;
-        for (int part = 0; part < parts; ++part) {
-            mbar_init(&bars[part], 1);
-        }
-        mbar_fence_init();
-    }
-    __syncthreads();
     if (threadIdx.x == 0) {
         for (int part = 0; part < parts; ++part) {
             const uint32_t bytes = part_rows * kDim;
@@ -120,10 +136,11 @@ __global__ void __launch_bounds__(kThreads, kLanes == 8 ? 7 : 4) delta_decode_in
     if (kEarly) {
         pdl_wait();  // q, k, v and the gates come from the preceding kernel
     }
-    for (int i = threadIdx.x; i < rows_here; i += kThreads) {
-        v_rows[i] = v[(static_cast<size_t>(b) * v_heads + h) * kDim + row_begin + i];
+    // what a thread needs of them, all in flight at once
+    float v_mine = 0.0f;
+    if (threadIdx.x < rows_here) {
+        v_mine = v[(static_cast<size_t>(b) * v_heads + h) * kDim + row_begin + threadIdx.x];
     }
-    __syncthreads();
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -149,6 +166,8 @@ __global__ void __launch_bounds__(kThreads, kLanes == 8 ? 7 : 4) delta_decode_in
     const float a = alpha[static_cast<size_t>(b) * v_heads + h];
     const float bt = beta[static_cast<size_t>(b) * v_heads + h];
     const float kq_token = kq[static_cast<size_t>(b) * kDeltaKeyHeads + hk];
+    v_rows[threadIdx.x] = v_mine;  // a thread per row of the tile at least
+    __syncthreads();
 
     constexpr float kMagic = 12582912.0f;        // 1.5 * 2^23
     constexpr float kMagicBiased = 12583040.0f;  // kMagic + 128
@@ -352,13 +371,13 @@ using DeltaKernel = void (*)(int8_t*, float*, const uint32_t*, const float*, con
                              const float*, const float*, float*, int, int, int*, const GatedNorm);
 
 // Four lanes per row (123 registers) while every CTA is resident at once with them, four per SM, or hardly more;
-// eight (71 registers, seven CTAs per SM) beyond.  Measured (us, layers that L2 does not hold, four / eight
-// lanes): 48 heads at 1 row 3.62 / 4.90, at 9 rows (432 CTAs) 8.28 / 12.00, at 12 rows (576) 8.70 / 12.54; 32 heads
-// at 20 rows (640) 11.7 / 12.7, at 22 rows (704) 12.6 / 12.9, at 23 rows (736) 13.1 / 13.0, at 32 rows (1024) 14.6 /
-// 14.0; 48 heads at 15 rows (720) 12.9 / 12.9.
+// eight (70 registers, seven CTAs per SM) beyond.  Measured (us, layers that L2 does not hold, four / eight
+// lanes): 48 heads at 1 row 3.49 / 4.79, at 9 rows (432 CTAs) 7.24 / 11.2, at 12 rows (576) 7.63 / 11.7; 32 heads
+// at 20 rows (640) 11.1 / 11.7, at 22 rows (704) 11.2 / 11.9, at 23 rows (736) 11.6 / 12.2, at 25 rows (800)
+// 12.5 / 12.0, at 32 rows (1024) 13.6 / 12.8; 48 heads at 16 rows (768) 12.1 / 12.0, at 32 rows (1536) 19.7 / 18.4.
 template <bool kEarly>
 DeltaKernel kernel_for(int ctas) {
-    return 4 * ctas <= 19 * sm_count_delta() ? delta_decode_int8_kernel<kEarly, 4> : delta_decode_int8_kernel<kEarly, 8>;
+    return ctas <= 5 * sm_count_delta() ? delta_decode_int8_kernel<kEarly, 4> : delta_decode_int8_kernel<kEarly, 8>;
 }
 
 }  // namespace

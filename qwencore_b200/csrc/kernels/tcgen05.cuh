@@ -59,11 +59,6 @@ __device__ __forceinline__ void tma_box_prefetch_l2(const CUtensorMap* map, int 
                  : "memory");
 }
 
-// Contiguous bytes into L2; address 16-byte aligned, size a multiple of 16.
-__device__ __forceinline__ void bulk_prefetch_l2(const void* global, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(global), "r"(bytes) : "memory");
-}
-
 // 16 consecutive 32-bit columns of this thread's tensor-memory lane.
 __device__ __forceinline__ void tmem_store16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(

@@ -368,8 +368,8 @@ def test_delta_decode_int8_matches_oracle(cuda, ops, batch, v_heads):
 
 
 @pytest.mark.parametrize("batch,v_heads", [(21, 32), (22, 32), (14, 48), (15, 48), (1, 32), (2, 32), (3, 48)],
-                         ids=["last_four_lanes", "first_eight_lanes", "last_four_lanes_h48", "first_eight_lanes_h48",
-                              "row_split_16", "row_split_8", "row_split_4"])
+                         ids=["ctas_672", "ctas_704", "ctas_672_h48", "ctas_720_h48", "row_split_16", "row_split_8",
+                              "row_split_4"])
 @pytest.mark.parametrize("exponent", [0, -100, 92], ids=["unit_q", "tiny_q", "huge_q"])
 def test_delta_decode_both_forms(cuda, ops, batch, v_heads, exponent):
     """On either side of the line between four and eight lanes per row, with row splits, with a key of zeros
@@ -390,6 +390,38 @@ def test_delta_decode_both_forms(cuda, ops, batch, v_heads, exponent):
     diff = np.abs(state.astype(np.int32) - want_state.astype(np.int32))
     assert diff.max() <= 1 and np.mean(diff > 0) < 1e-4
     assert np.allclose(scales, want_scales, rtol=1e-5, atol=0)
+
+
+@pytest.mark.parametrize("batch,v_heads", [(1, 48), (23, 32), (24, 32)],
+                         ids=["row_split", "last_four_lanes", "first_eight_lanes"])
+@pytest.mark.parametrize("before", [0, 0xFFFFFFFF], ids=["another_slot", "no_slot"])
+def test_delta_slots_and_state_written_just_before_the_call(cuda, ops, batch, v_heads, before):
+    """The kernel looks at a row's slot before the work ahead of it on the stream has ended, to have the tile
+    brought into L2; what counts is what stands there afterwards.  Slots, state and scales are written by copies
+    right before the call: the same bits as with everything in place long before."""
+    torch = cuda
+    from qwencore_b200 import abi
+
+    case = synth.delta_case(13, batch, v_heads)
+    want = run_delta(torch, ops, case, batch, v_heads)
+    shape = abi.get_shape()
+    abi.configure(v_heads, shape[1])
+    try:
+        fresh = [dev(torch, case[name]) for name in ("state", "scales", "slots")]
+        vectors = [dev(torch, case[name]) for name in ("q", "k", "v", "alpha", "beta", "kq")]
+        state, scales = torch.zeros_like(fresh[0]), torch.zeros_like(fresh[1])
+        slots = dev(torch, np.full(batch, before, dtype=np.uint32))
+        out = torch.zeros((batch, v_heads, 128), dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        for target, source in zip((state, scales, slots), fresh):
+            target.copy_(source)
+        ops.delta_decode_slots_packed(state, scales, slots, *vectors, out, case["capacity"], batch)
+        torch.cuda.synchronize()
+    finally:
+        abi.configure(*shape)
+    for got, expected in zip((state, scales, out), want):
+        assert np.array_equal(host(got), expected)
+    assert abi.lib.qwc_device_status() == 0
 
 
 @pytest.mark.parametrize("batch,v_heads", [(3, 32), (24, 32)], ids=["four_lanes", "eight_lanes"])
