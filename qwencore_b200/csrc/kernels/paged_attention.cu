@@ -2,12 +2,11 @@
 //
 // Replaces crates/qwc-cuda/cuda/paged_attention.cu:1913-1958 (qwc_paged_attention_packed_fp8)
 // for decode rows (tile of six packed query heads per KV head).  Semantics follow the
-// reference: Q, K, V and P enter the tensor cores as f16 (e4m3 -> f16 is exact), softmax
-// and accumulation in fp32, optional sigmoid output gate, split-context partials merged
-// by a second kernel (cuda/paged_attention.cu:1464-1574,1736-1823).
+// reference: softmax and accumulation in fp32, optional sigmoid output gate, split-context partials
+// merged by a second kernel (cuda/paged_attention.cu:1464-1574,1736-1823).
 //
-// The op reads every K and V byte of the row's context once and nothing else of size,
-// so it is HBM-bound.  Layout for sm_100a:
+// The op reads every K and V byte of the row's context once and nothing else of
+// size, so it is HBM-bound.  Layout for sm_100a:
 //   * a persistent grid of one CTA per SM.  The rows of a ragged batch differ in context by
 //     orders of magnitude, so the work is cut on the device into equal shares: the 16-token
 //     units of all (row, kv head) pairs are laid end to end, CTA c owns positions
@@ -15,137 +14,315 @@
 //     CTA's share (its partial is merged by the second kernel).  Every CTA streams the same
 //     number of bytes whatever the contexts are, and the launch shape depends only on the SM
 //     count, so the step stays capturable in a CUDA graph;
-//   * inside a CTA one producer warp and eight consumer warps.  KV moves in 4 KiB units (16
-//     tokens x 256 B of one kv head: a whole 16-token page, or a quarter of a 64-token page)
-//     by bulk-async copies (TMA 1-D) into a 3-stage ring of 8 units (128 tokens, 64 KiB of
-//     K+V per stage) guarded by full/empty mbarriers; the producer runs ahead across task
-//     boundaries, so the ring never drains between tasks;
-//   * each unit lands 16 bytes further than a multiple of 4 KiB.  An MMA column tile is
-//     "token j of 8 different units", so the eight rows an ldmatrix or a fragment load
-//     touches fall in eight different 16-byte bank groups: conflict-free without a
-//     swizzled tensor map;
-//   * QK^T: the six heads of the group are rows of one m16 tile, e4m3 pairs are widened
-//     by the hardware converter straight into B fragments; each warp owns two column tiles
-//     and keeps four independent accumulation chains.  PV: V is transposed on the fly by
-//     ldmatrix.trans on byte pairs and a byte permute; the eight warps split the 256 output
-//     dims, exchanging P through 2 KiB of shared memory.
+//   * nobody converts a cache byte.  K and V go from memory to tcgen05.mma.kind::f8f6f4 as they are
+//     stored: a stage is 128 tokens of one kv head, each unit of 16 tokens (a whole 16-token page, or a quarter
+//     of a 64-token page) two swizzled TMA boxes of 128 bytes per token.  K is the A operand of S^T = K Q^T
+//     (128 tokens x 256 dims, K-major), V the A operand of O^T = V^T P^T (dims x tokens, MN-major);
+//   * queries and probabilities enter as e4m3 digits.  An e4m3 has four significant bits, so a number x is
+//     written as x0 + x1 / 16 + x2 / 256, every digit rounded to nearest from what the digits before it left, and
+//     digit j of head h is column 8 j + h of the B operand: three accumulators per output, added with their
+//     weights in fp32.  A head's query is first brought to [128, 256) by a power of two: a bf16's eight bits are
+//     exact down to 2^-18 of the largest element, and an element below that is off by 2^-26 of the largest.
+//     A probability is kept to 2^-13 of itself (f16, which the kernel used to multiply with: 2^-12), down to
+//     2^-26 of the largest;
+//   * O of one stage is read from tensor memory and added to fp32 registers, where a change of the running
+//     maximum costs one multiplication.
+//
+//   warps 0-3   softmax: thread = token of the stage.  S from tensor memory, maximum over the 128 tokens,
+//               exponentials, digits of P to shared memory
+//   warps 4-11  thread = output dim: digits of the next task's query, the accumulators of O, the result
+//   warp 12     issues the MMAs: S of stage n + 1 before O of stage n
+//   warps 13,14 fetch K and V into rings of three stages, ahead across task boundaries
+//
+// What it took to get there: widening every cache byte to f16 for mma.sync kept the conversion unit 76 % busy
+// and the stage on dependent instructions.  Measured (us, layers that L2 does not hold, before / now):
+// 32 rows in [128, 2048] 26.4 / 23.4, one row of 2048 12.3 / 11.4, three rows of 32768 45.3 / 42.4 (6.1 TB/s while it
+// streams), 32 rows log-uniform to 32768 82.8 / 77.2, 20 rows from 8192 to 32768 134.1 / 121.1 (6.1 TB/s all in all).
+// The new operands alone, on the old plan and merge, gave 26.4 / 25.5 and 82.9 / 82.6: what had been hidden behind
+// the conversions was the plan, the merge and CTAs that ended early (SplitPlan, reduce_partitions_kernel).
 //
 // Cache memory must hold finite e4m3 codes in every allocated page (a zero-initialised
 // pool, as the reference allocates it): positions past the context are masked by
 // zero probabilities, not skipped.
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace qwc {
 namespace {
 
-constexpr int kConsumerWarps = 8;
-constexpr int kConsumerThreads = kConsumerWarps * 32;
-constexpr int kThreads = kConsumerThreads + 32;  // + the producer warp
+constexpr int kSoftmaxWarps = 4;
+constexpr int kOutputWarps = 8;
+constexpr int kFirstOutputWarp = kSoftmaxWarps;
+constexpr int kMmaWarp = kFirstOutputWarp + kOutputWarps;
+constexpr int kKeyWarp = kMmaWarp + 1;
+constexpr int kValueWarp = kMmaWarp + 2;
+constexpr int kQueryWarp = kMmaWarp + 3;
+constexpr int kPlanWarp = kMmaWarp + 4;
+constexpr int kListReaders = kPlanWarp;  // every warp before it reads the task lists
+constexpr int kThreads = (kPlanWarp + 1) * 32;
 constexpr int kUnitTokens = 16;
-constexpr int kUnitBytes = kUnitTokens * kHeadDim;  // 4096
-constexpr int kUnitPitch = kUnitBytes + 16;         // staggered landing offset
 constexpr int kStageUnits = 8;
+constexpr int kStageTokens = kStageUnits * kUnitTokens;
+constexpr int kBoxBytes = kUnitTokens * 128;            // half the dims of a unit
+constexpr int kHalfBytes = kStageUnits * kBoxBytes;     // ... of a stage
+constexpr int kStageBytes = 2 * kHalfBytes;             // K or V of a stage
 constexpr int kStages = 3;
-constexpr int kStageBytes = kStageUnits * kUnitPitch;    // per K or V
+constexpr int kDigits = 3;
+constexpr int kColumns = 32;                            // digit j of head h is column 8 j + h; the rest is zero
+constexpr int kQueryBytes = kColumns * kHeadDim;        // B operand of S, K-major core matrices
+constexpr int kProbabilityBytes = kColumns * kStageTokens;  // B operand of O, MN-major core matrices
+constexpr int kTmemColumns = 256;
+constexpr int kScoreColumn = 0;                         // two buffers
+constexpr int kOutputColumn = 2 * kColumns;             // two buffers of two halves of the dims
 constexpr int kPartialFloats = 2;
 constexpr size_t kPartialBytes = 2 * sizeof(float) + kHeadDim * sizeof(__half);  // 520
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr int kMaxCtaTasks = 64;      // list capacity; the plan keeps a CTA far below it
-constexpr int kPlanMinPadding = 16;   // units a task costs beyond its tokens (query load, epilogue, merge)
-constexpr int kPlanPaddingDivisor = 24;  // padding = share / this at least: bounds the tasks of one CTA
+constexpr int kMaxListTasks = 96;     // tasks of one chunk; the plan keeps it below
+constexpr int kPlanMinPadding = 4;    // units a task costs beyond its tokens
+constexpr int kPlanPaddingDivisor = 64;  // padding = share / this at least: bounds the tasks of one chunk
+constexpr int kChunksPerSm = 4;       // one large chunk and three small ones
+constexpr int kDynamicShare = 192;    // units per SM from which on the line is cut into chunks of two sizes ...
+constexpr int kThreeSmallShare = 480;  // ... with three small ones instead of two
 constexpr int kPlanRows = 256;        // rows whose prefix fits the shared-memory table
 
 struct Task {
     int row;
     int kv_head;
     int part;
+    int last;  // no piece of the pair after this one
     int unit_begin;
     int units;
     int context;  // tokens of the row, cut at the block table's capacity
 };
 
 struct Smem {
-    uint8_t k[kStages][kStageBytes];
+    uint8_t k[kStages][kStageBytes];  // [half of the dims][token][128 bytes], 128-byte swizzle
     uint8_t v[kStages][kStageBytes];
-    uint2 p[kStageUnits][32];       // P as A fragments: [pv k-step][lane]
-    float warp_max[kConsumerWarps][8];
-    float warp_sum[kConsumerWarps][8];
-    uint64_t full[kStages];
-    uint64_t empty[kStages];
-    int first_unit[kPlanRows + 1];  // prefix sum of the rows' units (a row without context counts one)
-    Task tasks[kMaxCtaTasks];
-    int task_count;
-    int issued;                     // stages the producer has put in flight
-    int consumed;                   // stages the consumers have finished
-    int failed;                     // a consumer's wait gave up
-    int producer_failed;            // the producer's wait gave up (written by the producer only)
-    int leave[2];                   // what one consumer thread saw of the two flags before the barrier of stage n & 1
+    uint8_t p[2][kProbabilityBytes];  // [column / 16][token][16]
+    uint8_t q[2][kQueryBytes];        // [dim / 16][column][16]
+    uint64_t k_full[kStages], k_empty[kStages];
+    uint64_t v_full[kStages], v_empty[kStages];
+    uint64_t q_ready[2], q_free[2];   // of a task's query
+    uint64_t s_ready[2], s_free[2];   // of a stage: scores in tensor memory
+    uint64_t max_ready[2];            // the four warps' maxima
+    uint64_t p_ready[2], p_free[2];   // probabilities in shared memory
+    uint64_t o_ready[2], o_free[2];   // outputs in tensor memory
+    uint64_t t_ready[2], t_free[2];   // of a task: sums and maxima
+    float warp_max[2][kSoftmaxWarps][8];
+    float rescale[4][8];              // what a stage multiplies the sums of the stages before it with
+    float query_scale[2][8];
+    float task_sum[2][kSoftmaxWarps][8];
+    float task_max[2][8];
+    uint64_t list_ready[2], list_free[2];  // of a chunk: its tasks
+    uint64_t list_wanted;           // every copy of the newest chunk has been asked for
+    uint64_t claim_ready;
+    ulonglong2 claim;               // what the hardware answered
+    unsigned long long first_unit[kPlanRows + 1];  // (as Positions) prefix sum of the rows' units (a row without context counts one)
+    Task tasks[2][kMaxListTasks];
+    int task_count[2];              // -1: there is nothing left
+    uint32_t tmem_base;
+    int failed;                     // a wait gave up
 };
 
-__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
-    const __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&h);
+static_assert(sizeof(Smem) + 1024 <= 232448, "shared memory of a CTA");
+
+// (out of line, as in the projection kernels: a wait that is already satisfied costs one test)
+__device__ __noinline__ bool att_wait_slow(uint64_t* bar, uint32_t parity, Smem& sm, int* status) {
+    const long long start = clock64();
+    for (;;) {
+#pragma unroll 1
+        for (int spin = 0; spin < 64; ++spin) {
+            if (mbar_try_wait(bar, parity)) {
+                return true;
+            }
+        }
+        if (*reinterpret_cast<volatile int*>(&sm.failed) != 0) {
+            return false;
+        }
+        if (clock64() - start > 40000000ll) {
+            break;
+        }
+    }
+    atomicCAS(status, 0, kStatusAttentionPageWait);
+    *reinterpret_cast<volatile int*>(&sm.failed) = 1;
+    return false;
 }
 
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t address) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(address));
+// For a converged warp: the same answer in every lane.
+__device__ __forceinline__ bool att_wait(uint64_t* bar, uint32_t parity, Smem& sm, int* status) {
+    const bool ok = mbar_try_wait(bar, parity) || att_wait_slow(bar, parity, sm, status);
+    return __all_sync(0xffffffffu, ok);
 }
 
-// low / high 16 bits of a word holding two e4m3 pairs -> two f16x2
-__device__ __forceinline__ void cvt_e4m3x4(uint32_t word, uint32_t& lo, uint32_t& hi) {
-    asm("{\n"
-        ".reg .b16 a, b;\n"
-        "mov.b32 {a, b}, %2;\n"
-        "cvt.rn.f16x2.e4m3x2 %0, a;\n"
-        "cvt.rn.f16x2.e4m3x2 %1, b;\n"
+// Operand of 128-byte rows with the 128-byte swizzle, eight rows (1 KiB) to an atom: K-major (a row is a token, its
+// bytes the dims that are contracted) as well as MN-major (a row is a token that is contracted, its bytes the dims
+// of the output).
+__device__ __forceinline__ uint64_t swizzled_descriptor(uint32_t address) {
+    const uint64_t lo = ((address >> 4) & 0x3FFFu) | (1ull << 16);
+    const uint64_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);
+    return lo | (hi << 32);
+}
+
+// D[128][N] (+)= A[128][32] x B[N][32], e4m3 from shared memory, fp32 accumulate.
+__device__ __forceinline__ void umma_fp8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                         uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+__device__ __forceinline__ uint32_t float2_to_e4m3x2(float lo, float hi) {
+    uint16_t out;
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(out) : "f"(hi), "f"(lo));
+    return out;
+}
+
+// The next digit of two numbers, and sixteen times what it leaves.
+__device__ __forceinline__ uint32_t take_digit(float& lo, float& hi) {
+    const uint32_t digit = float2_to_e4m3x2(lo, hi);
+    const uint32_t half = cvt_e4m3x2_to_f16x2(digit);
+    const float2 value = __half22float2(*reinterpret_cast<const __half2*>(&half));
+    lo = (lo - value.x) * 16.0f;
+    hi = (hi - value.y) * 16.0f;
+    return digit;
+}
+
+// Largest value of the warp (a NaN counts as nothing).
+__device__ __forceinline__ float warp_highest(float value) {
+    float out;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(out) : "f"(value));
+    return out;
+}
+
+// Asks the hardware for a CTA of this grid that has not started yet: it will not start, and whoever asked does its
+// work.  The answer, 16 bytes, arrives in shared memory.
+__device__ __forceinline__ void claim_chunk(ulonglong2* answer, uint64_t* bar) {
+    asm volatile(
+        "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+            smem_u32(answer)),
+        "r"(smem_u32(bar))
+        : "memory");
+}
+
+// The CTA index in the answer, -1 when all have started (nothing may be asked after that).
+__device__ __forceinline__ int claimed_chunk(const ulonglong2* answer) {
+    int index;
+    asm volatile(
+        "{\n"
+        ".reg .b128 answer;\n"
+        ".reg .pred given;\n"
+        ".reg .b32 x;\n"
+        "ld.shared.b128 answer, [%1];\n"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 given, answer;\n"
+        "mov.b32 x, -1;\n"
+        "@given clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 x, answer;\n"
+        "mov.b32 %0, x;\n"
         "}\n"
-        : "=r"(lo), "=r"(hi)
-        : "r"(word));
+        : "=r"(index)
+        : "r"(smem_u32(answer))
+        : "memory");
+    return index;
 }
 
-__device__ __forceinline__ void consumer_sync() {
-    asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads) : "memory");
+// Three accumulators of a digit each, with their weights.
+__device__ __forceinline__ float combine_digits(uint32_t d0, uint32_t d1, uint32_t d2) {
+    return fmaf(fmaf(__uint_as_float(d2), 0.0625f, __uint_as_float(d1)), 0.0625f, __uint_as_float(d0));
 }
 
-// The split plan.  Both kernels evaluate it from the same inputs.
+// Cache pages as rows of 256 bytes, fetched in boxes of 16 tokens x 128 bytes.  The launcher does not know how many
+// pages the pool has (nor do the kernels of the reference): the map describes as many rows as a coordinate can
+// name, and the block tables say which of them exist.
+cudaError_t encode_cache_map(CUtensorMap* map, const void* cache) {
+    const EncodeTiled encode = tensor_map_encoder();
+    if (encode == nullptr) {
+        return cudaErrorNotSupported;
+    }
+    const cuuint64_t dims[2] = {kHeadDim, 0x7fffffffull};
+    const cuuint64_t strides[1] = {kHeadDim};
+    const cuuint32_t box[2] = {128, kUnitTokens};
+    const cuuint32_t element_strides[2] = {1, 1};
+    const CUresult result =
+        encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(cache), dims, strides, box, element_strides,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return result == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+// The split plan.
 //
 // The (row, kv head) pairs are laid end to end, row-major, on a line of units; a pair takes
 // max(units, 1) + padding positions (the padding stands for what a task costs beyond its tokens).
-// Every CTA owns `share` consecutive positions and works on the tokens that fall inside: all CTAs
-// stream the same amount, whatever the rows' lengths.  The piece of a pair inside CTA c is partial
-// number c - (first CTA that touches the pair); a pair without context is one empty piece.
-//   * padding >= share / kPlanPaddingDivisor, so that a CTA never holds more than
-//     kPlanPaddingDivisor + pairs / CTAs + 2 tasks;
-//   * share >= capacity / (partitions - 1): a row never has more pieces than the workspace has slots;
-//   * share is a whole number of stages.
+// The line is cut into chunks, and a task is the piece of one pair inside one chunk, partial number
+// c - (first chunk that touches the pair); a pair without context is one empty piece.  The last piece of a pair says
+// so in the sign of its sum: the merge kernel needs no plan.
+//   * One equal chunk per SM, up to kDynamicShare units.  Beyond that one large chunk (seven tenths of an SM's share)
+//     and two or, from kThreeSmallShare on, three small ones: a CTA starts with a large chunk and, once it has
+//     asked for its last bytes, takes the next chunk that nobody has.  The SMs do not get the same share of the
+//     memory's bandwidth (40 to 56 GB/s each, others every time): with equal chunks of 350 units the CTAs' ends
+//     lay 53 to 72 us after their first copies.  Measured (us, equal chunks / two small / three small / six small):
+//     share 350 (32 rows, log-uniform to 32768) 79.9 / 77.2 / 78.6 / 83.4, 330 76.0 / 71.8 / 72.8, 612 (20 rows,
+//     8192 to 32768) 128.5 / 123.0 / 121.1 / 126.1, 230 (32 x 4096) 56.3 / 55.2 / 58.2; at 166 (three rows of
+//     32768, forced) 42.8 / - / 52.1.
+//   * padding >= share / kPlanPaddingDivisor, so that a chunk never holds more than kPlanPaddingDivisor + 4 tasks;
+//   * every chunk >= capacity / (partitions - 1): a row never has more pieces than the workspace has slots;
+//   * every chunk is a whole number of stages.
+// Position: uint32_t, unless the block tables could describe a longer line (plan_is_wide).
+template <typename Position>
 struct SplitPlan {
-    long long share;
+    Position large, small;
+    Position line;
     int padding;
 };
 
-__device__ __forceinline__ SplitPlan make_split_plan(long long total_row_units, int rows, int capacity_units,
-                                                     int partitions, int ctas) {
-    const long long by_capacity = partitions > 1 ? (capacity_units + partitions - 2) / (partitions - 1) : 0;
-    long long share = (total_row_units * kKvHeads + ctas - 1) / ctas;
-    share = share > by_capacity ? share : by_capacity;
-    const long long padding_wanted = (share + kPlanPaddingDivisor - 1) / kPlanPaddingDivisor;
-    SplitPlan plan;
-    plan.padding = static_cast<int>(padding_wanted > kPlanMinPadding ? padding_wanted : kPlanMinPadding);
-    const long long line = (total_row_units + static_cast<long long>(rows) * plan.padding) * kKvHeads;
-    share = (line + ctas - 1) / ctas;
-    share = share > by_capacity ? share : by_capacity;
-    plan.share = (share + kStageUnits - 1) / kStageUnits * kStageUnits;
+constexpr int kPlanSlack = 1 << 20;  // more than the padding of a pair can be while positions have 32 bits
+
+template <typename Position>
+__device__ __forceinline__ SplitPlan<Position> make_split_plan(Position total_row_units, int rows, int smallest_chunk,
+                                                               int ctas) {
+    // (shares in floating point, rounded up by more than the arithmetic can be off)
+    const float per_cta = 1.00001f / static_cast<float>(ctas);
+    const Position smallest = static_cast<Position>(smallest_chunk);
+    Position share = static_cast<Position>(static_cast<float>(total_row_units) * kKvHeads * per_cta) + 1;
+    share = share > smallest ? share : smallest;
+    SplitPlan<Position> plan;
+    plan.padding = static_cast<int>(share / kPlanPaddingDivisor) + 1;
+    plan.padding = plan.padding > kPlanMinPadding ? plan.padding : kPlanMinPadding;
+    plan.line = (total_row_units + static_cast<Position>(rows) * plan.padding) * kKvHeads;
+    share = static_cast<Position>(static_cast<float>(plan.line) * per_cta) + 1;
+    const bool dynamic = share >= kDynamicShare;
+    const Position tenth = share / 10;
+    plan.small = !dynamic ? share : share >= kThreeSmallShare ? tenth : tenth + tenth / 2;
+    plan.large = !dynamic ? share : share - (share >= kThreeSmallShare ? 3 : 2) * plan.small;
+    plan.large = ((plan.large > smallest ? plan.large : smallest) + kStageUnits - 1) / kStageUnits * kStageUnits;
+    plan.small = ((plan.small > smallest ? plan.small : smallest) + kStageUnits - 1) / kStageUnits * kStageUnits;
     return plan;
 }
 
+// The chunk that holds a position of the line ...
+template <typename Position>
+__device__ __forceinline__ int chunk_of(const SplitPlan<Position>& plan, Position position, int ctas) {
+    const Position small_begin = plan.large * ctas;
+    return position < small_begin ? static_cast<int>(position / plan.large)
+                                  : ctas + static_cast<int>((position - small_begin) / plan.small);
+}
+
+// ... and where a chunk begins.
+template <typename Position>
+__device__ __forceinline__ Position chunk_begin(const SplitPlan<Position>& plan, int chunk, int ctas) {
+    return chunk < ctas ? plan.large * chunk : plan.large * ctas + plan.small * (chunk - ctas);
+}
+
 // first position of pair (row, kv head); units_before = units of the rows before it
-__device__ __forceinline__ long long pair_position(const SplitPlan& plan, int row, int kv_head, long long units_before,
-                                                   int row_units) {
-    return (units_before + static_cast<long long>(row) * plan.padding) * kKvHeads +
-           static_cast<long long>(kv_head) * (row_units + plan.padding);
+template <typename Position>
+__device__ __forceinline__ Position pair_position(const SplitPlan<Position>& plan, int row, int kv_head,
+                                                  Position units_before, Position row_units) {
+    return (units_before + static_cast<Position>(row) * plan.padding) * kKvHeads +
+           static_cast<Position>(kv_head) * (row_units + plan.padding);
 }
 
 // A context longer than the block table can describe is cut at the table's capacity.
@@ -157,554 +334,807 @@ __device__ __forceinline__ int units_of_context(uint32_t context, int capacity_u
 // Units a row occupies on the plan's line: a row without context still gets one task (it stores zeros).
 __device__ __forceinline__ int plan_units(int units) { return units > 0 ? units : 1; }
 
-template <bool kSplit>
+template <bool kSplit, typename Position>
 __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
+    const __grid_constant__ CUtensorMap key_map, const __grid_constant__ CUtensorMap value_map,
     const __nv_bfloat16* __restrict__ query, const __nv_bfloat16* __restrict__ query_gate_projection,
-    const uint8_t* __restrict__ key_cache, const uint8_t* __restrict__ value_cache,
     const uint32_t* __restrict__ block_tables, const uint32_t* __restrict__ context_lengths,
     const float* __restrict__ key_scales, const float* __restrict__ value_scales,
     __nv_bfloat16* __restrict__ output, __half* __restrict__ staged_output, int padded_rows,
     float* __restrict__ partial_stats, __half* __restrict__ partial_out, int rows, int max_blocks, int row_base,
-    int page_size, int gate_stride, int partitions, float softmax_scale, int* status) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
+    int page_size, int gate_stride, int partitions, int smallest_chunk, int ctas, float softmax_scale, int* status) {
+    extern __shared__ unsigned char smem_raw[];
+    Smem& sm = *reinterpret_cast<Smem*>(smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
 
     pdl_launch_dependents();
-    if (status_is_set(status)) {
-        return;
-    }
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const int g = lane >> 2;
-    const int t = lane & 3;
     const int units_per_page = page_size / kUnitTokens;
     const int capacity_units = max_blocks * units_per_page;
 
-    // ---- plan: task size, the rows' task counts, this CTA's task list ---------------------
     // Stale bytes of a partly filled stage are multiplied by zero probabilities, so they
-    // must be finite: clear the value ring once (every later byte comes from the cache).
+    // must be finite: clear the value ring once (every later byte comes from the cache).  The columns of a
+    // query that belong to no digit stay zero.
     for (int i = threadIdx.x; i < kStages * kStageBytes / 16; i += kThreads) {
         reinterpret_cast<uint4*>(&sm.v[0][0])[i] = make_uint4(0, 0, 0, 0);
     }
-    pdl_wait();  // context lengths, tables, query and the cache rows of this step come from earlier kernels
-    if (warp == 0) {
-        if (lane == 0) {
-            sm.failed = 0;
-            sm.producer_failed = 0;
-            sm.leave[0] = 0;
-            sm.leave[1] = 0;
-            sm.consumed = 0;
-            sm.issued = 0;
-            for (int s = 0; s < kStages; ++s) {
-                mbar_init(&sm.full[s], 1);
-                mbar_init(&sm.empty[s], kConsumerWarps);
-            }
-            mbar_fence_init();
+    for (int i = threadIdx.x; i < 2 * kQueryBytes / 16; i += kThreads) {
+        reinterpret_cast<uint4*>(&sm.q[0][0])[i] = make_uint4(0, 0, 0, 0);
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
+                     "r"(kTmemColumns)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+    if (threadIdx.x == kKeyWarp * 32) {
+        for (int i = 0; i < kStages; ++i) {
+            mbar_init(&sm.k_full[i], 1);
+            mbar_init(&sm.k_empty[i], 1);
+            mbar_init(&sm.v_full[i], 1);
+            mbar_init(&sm.v_empty[i], 1);
         }
-        int count = 0;
-        if (!kSplit) {
-            // whole (row, kv head) pairs, dealt round: c, c + grid, ...
-            for (int index = lane; index < kMaxCtaTasks; index += 32) {
-                const long long id = static_cast<long long>(blockIdx.x) + static_cast<long long>(index) * gridDim.x;
-                if (id < static_cast<long long>(rows) * kKvHeads) {
-                    const int row = static_cast<int>(id / kKvHeads);
-                    const uint32_t row_context = context_lengths[row_base + row];
-                    Task task;
-                    task.context = static_cast<int>(min(row_context, static_cast<uint32_t>(capacity_units) * kUnitTokens));
-                    task.row = row_base + row;
-                    task.kv_head = static_cast<int>(id % kKvHeads);
-                    task.part = 0;
-                    task.unit_begin = 0;
-                    task.units = units_of_context(row_context, capacity_units);
-                    sm.tasks[index] = task;
-                    ++count;
-                }
-            }
-            count = __reduce_add_sync(0xffffffffu, count);
-        } else {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&sm.q_ready[i], 1);
+            mbar_init(&sm.q_free[i], 1 + kSoftmaxWarps);
+            mbar_init(&sm.s_ready[i], 1);
+            mbar_init(&sm.s_free[i], kSoftmaxWarps);
+            mbar_init(&sm.max_ready[i], kSoftmaxWarps);
+            mbar_init(&sm.p_ready[i], kSoftmaxWarps);
+            mbar_init(&sm.p_free[i], 1);
+            mbar_init(&sm.o_ready[i], 2);  // the MMAs, and the thread that issued them (it passes on what it waited for)
+            mbar_init(&sm.o_free[i], kOutputWarps);
+            mbar_init(&sm.t_ready[i], kSoftmaxWarps);
+            mbar_init(&sm.t_free[i], kOutputWarps);
+            mbar_init(&sm.list_ready[i], 1);
+            mbar_init(&sm.list_free[i], kListReaders);
+        }
+        mbar_init(&sm.list_wanted, 1);
+        mbar_init(&sm.claim_ready, 1);
+        sm.failed = 0;
+        mbar_fence_init();
+    }
+    fence_proxy_async();
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sm.tmem_base);
+    bool ok = true;
+    int t = 0;  // tasks and ...
+    int n = 0;  // ... stages so far, over all chunks
+
+    if (warp == kPlanWarp || warp == 0) {
+        // ---------------- plan: the tasks of one chunk after the other ------------------------------
+        // (Warp 0 walks through the first list too, into scratch, before the wait for the kernels ahead and on
+        // whatever the context lengths are then: when the plan is made, its instructions are in the cache.)
+        const bool rehearsal = warp == 0;
+        if (!rehearsal) {
+            pdl_wait();  // context lengths, tables, query and the cache rows of this step come from earlier kernels
+        }
+        Position* const first_unit =
+            rehearsal ? reinterpret_cast<Position*>(sm.p[0]) : reinterpret_cast<Position*>(sm.first_unit);
+        const int earlier_failure = *reinterpret_cast<const volatile int*>(status);
+        SplitPlan<Position> plan = {};
+        if (kSplit) {
             // prefix of the rows' units: a warp scan per 32 rows
-            int carry = 0;
+            Position carry = 0;
+#pragma unroll 1
             for (int base = 0; base < rows; base += 32) {
                 const int r = base + lane;
-                const int mine = r < rows ? plan_units(units_of_context(context_lengths[row_base + r], capacity_units)) : 0;
-                int inclusive = mine;
+                const Position mine =
+                    r < rows ? plan_units(units_of_context(__ldcg(context_lengths + row_base + r), capacity_units)) : 0;
+                Position inclusive = mine;
 #pragma unroll
                 for (int offset = 1; offset < 32; offset <<= 1) {
-                    const int other = __shfl_up_sync(0xffffffffu, inclusive, offset);
+                    const Position other = __shfl_up_sync(0xffffffffu, inclusive, offset);
                     if (lane >= offset) {
                         inclusive += other;
                     }
                 }
                 if (r < rows) {
-                    sm.first_unit[r] = carry + inclusive - mine;
+                    first_unit[r] = carry + inclusive - mine;
                 }
                 carry += __shfl_sync(0xffffffffu, inclusive, 31);
             }
             if (lane == 0) {
-                sm.first_unit[rows] = carry;
+                first_unit[rows] = carry;
             }
             __syncwarp();
-            const SplitPlan plan = make_split_plan(carry, rows, capacity_units, partitions, gridDim.x);
-            const long long low = static_cast<long long>(blockIdx.x) * plan.share;
-            const long long high = low + plan.share;
-            // the pieces of this CTA, in (row, kv head) order: 32 rows at a time, a lane per row
-            for (int base = 0; base < rows; base += 32) {
-                const int r = base + lane;
-                Task mine[kKvHeads];
-                int found = 0;
-                if (r < rows) {
-                    const uint32_t row_context = context_lengths[row_base + r];
-                    const int row_units = units_of_context(row_context, capacity_units);
-                    const int occupied = plan_units(row_units);
-#pragma unroll
-                    for (int kv = 0; kv < kKvHeads; ++kv) {
-                        const long long start = pair_position(plan, r, kv, sm.first_unit[r], occupied);
-                        if (start < high && start + occupied > low) {
-                            const long long begin = low > start ? low - start : 0;
-                            const long long end = high - start < occupied ? high - start : occupied;
-                            Task task;
-                            task.context =
-                                static_cast<int>(min(row_context, static_cast<uint32_t>(capacity_units) * kUnitTokens));
-                            task.row = row_base + r;
-                            task.kv_head = kv;
-                            task.part = static_cast<int>(blockIdx.x - start / plan.share);
-                            task.unit_begin = static_cast<int>(begin);
-                            task.units = max(0, min(static_cast<int>(end), row_units) - static_cast<int>(begin));
-                            mine[found++] = task;
-                        }
+            plan = make_split_plan(carry, rows, smallest_chunk, ctas);
+        }
+        int chunk = earlier_failure != 0 ? -1 : static_cast<int>(blockIdx.x);
+        int claims = 0;
+#pragma unroll 1
+        for (int m = 0; ok; ++m) {
+            Task* const tasks = rehearsal ? reinterpret_cast<Task*>(sm.p[1]) : sm.tasks[m & 1];
+            int count = 0;
+            if (chunk < 0) {
+                count = -1;
+            } else if (!kSplit) {
+                // whole (row, kv head) pairs, dealt round: c, c + grid, ...
+                for (int id = chunk + lane * ctas; id < rows * kKvHeads; id += 32 * ctas) {
+                    const int index = (id - chunk) / ctas;
+                    const uint32_t row_context = __ldcg(context_lengths + row_base + id / kKvHeads);
+                    if (index < kMaxListTasks) {
+                        Task task;
+                        task.context =
+                            static_cast<int>(min(row_context, static_cast<uint32_t>(capacity_units) * kUnitTokens));
+                        task.row = row_base + id / kKvHeads;
+                        task.kv_head = id % kKvHeads;
+                        task.part = 0;
+                        task.last = 1;
+                        task.unit_begin = 0;
+                        task.units = units_of_context(row_context, capacity_units);
+                        tasks[index] = task;
+                    }
+                    ++count;
+                }
+                count = static_cast<int>(__reduce_add_sync(0xffffffffu, count));
+            } else {
+                const Position low = chunk_begin(plan, chunk, ctas);
+                const Position high = chunk_begin(plan, chunk + 1, ctas);
+                // the pieces inside the chunk, in (row, kv head) order: 32 pairs at a time
+#pragma unroll 1
+                for (int base = 0; base < rows * kKvHeads; base += 32) {
+                    const int r = (base + lane) / kKvHeads;
+                    const int kv = (base + lane) % kKvHeads;
+                    bool inside = false;
+                    Position start = high, occupied = 0;
+                    if (r < rows) {
+                        occupied = first_unit[r + 1] - first_unit[r];
+                        start = pair_position(plan, r, kv, first_unit[r], occupied);
+                        inside = start < high && start + occupied > low;
+                    }
+                    const uint32_t found = __ballot_sync(0xffffffffu, inside);
+                    const int index = count + __popc(found & ((1u << lane) - 1u));
+                    if (inside && index < kMaxListTasks) {
+                        const uint32_t row_context = __ldcg(context_lengths + row_base + r);
+                        const int row_units = units_of_context(row_context, capacity_units);
+                        const Position begin = low > start ? low - start : 0;
+                        const Position end = high - start < occupied ? high - start : occupied;
+                        Task task;
+                        task.context =
+                            static_cast<int>(min(row_context, static_cast<uint32_t>(capacity_units) * kUnitTokens));
+                        task.row = row_base + r;
+                        task.kv_head = kv;
+                        task.part = start < low ? chunk - chunk_of(plan, start, ctas) : 0;
+                        task.last = end == occupied;
+                        task.unit_begin = static_cast<int>(begin);
+                        task.units = max(0, min(static_cast<int>(end), row_units) - static_cast<int>(begin));
+                        tasks[index] = task;
+                    }
+                    count += __popc(found);
+                    if (__all_sync(0xffffffffu, start >= high)) {
+                        break;
                     }
                 }
-                int before = found;  // exclusive prefix over the lanes
-#pragma unroll
-                for (int offset = 1; offset < 32; offset <<= 1) {
-                    const int other = __shfl_up_sync(0xffffffffu, before, offset);
-                    if (lane >= offset) {
-                        before += other;
-                    }
-                }
-                const int all = __shfl_sync(0xffffffffu, before, 31);
-                before -= found;
-#pragma unroll
-                for (int i = 0; i < kKvHeads; ++i) {
-                    if (i < found && count + before + i < kMaxCtaTasks) {
-                        sm.tasks[count + before + i] = mine[i];
-                    }
-                }
-                count += all;
             }
-            if (count > kMaxCtaTasks) {
+            __syncwarp();
+            if (rehearsal) {
+                break;
+            }
+            if (count > kMaxListTasks) {
                 // cannot happen while the launcher's check of rows against the SM count holds
                 if (lane == 0) {
                     atomicCAS(status, 0, kStatusAttentionPlanOverflow);
                 }
-                count = 0;
+                count = -1;
+            }
+            if (lane == 0) {
+                sm.task_count[m & 1] = count;
+                mbar_arrive(&sm.list_ready[m & 1]);
+            }
+            __syncwarp();
+            if (count < 0) {
+                break;
+            }
+            // The next chunk is claimed once the last bytes of this one have been asked for (an answer takes 0.2
+            // us, the ring holds three stages); what lies past the end of the line is claimed too (it would
+            // start, and find nothing to do).
+            chunk = -1;
+            ok = att_wait(&sm.list_free[(m + 1) & 1], (((m + 1) >> 1) & 1) ^ 1, sm, status) &&
+                 att_wait(&sm.list_wanted, m & 1, sm, status);
+            while (gridDim.x > ctas && ok) {
+                if (lane == 0) {
+                    fence_proxy_async();  // the answer before this one has been read
+                    mbar_arrive_expect_tx(&sm.claim_ready, 16);
+                    claim_chunk(&sm.claim, &sm.claim_ready);
+                }
+                __syncwarp();
+                ok = att_wait(&sm.claim_ready, claims & 1, sm, status);
+                ++claims;
+                chunk = ok ? claimed_chunk(&sm.claim) : -1;
+                __syncwarp();
+                if (chunk < 0 || chunk_begin(plan, chunk, ctas) < plan.line) {
+                    break;
+                }
             }
         }
-        if (lane == 0) {
-            sm.task_count = count;
-        }
     }
-    fence_proxy_async();
-    __syncthreads();
-    const int task_count = sm.task_count;
 
-    if (warp == kConsumerWarps) {
-        // ---------------- producer ----------------------------------------------------------
-        int n = 0;  // stages issued so far
-        bool ok = true;
-        for (int ti = 0; ti < task_count && ok; ++ti) {
-            const Task task = sm.tasks[ti];
-            const uint32_t* table = block_tables + static_cast<size_t>(task.row) * max_blocks;
-            const int stages = (task.units + kStageUnits - 1) / kStageUnits;
-            for (int st = 0; st < stages && ok; ++st, ++n) {
-                const int slot = n % kStages;
-                const int first = task.unit_begin + st * kStageUnits;
-                const int count = min(kStageUnits, task.units - st * kStageUnits);
-                // the page id is fetched before the wait for a free slot, which is the longer of the two
-                const uint32_t physical = lane < count ? table[(first + lane) / units_per_page] : 0u;
-                ok = mbar_wait_bounded(&sm.empty[slot], ((n / kStages) & 1) ^ 1, kStatusAttentionPageWait, status);
-                // one lane reads the consumers' flag for the whole warp: the decision to leave is uniform
-                const int consumers_left =
-                    __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&sm.failed), 0);
-                ok = __all_sync(0xffffffffu, ok) && consumers_left == 0;
+    if (warp == kKeyWarp || warp == kValueWarp) {
+        // ---------------- K or V: two lanes per unit, one for each half of the dims -----------------
+        const bool keys = warp == kKeyWarp;
+        uint64_t* const full = keys ? sm.k_full : sm.v_full;
+        uint64_t* const empty = keys ? sm.k_empty : sm.v_empty;
+        uint8_t* const ring = keys ? &sm.k[0][0] : &sm.v[0][0];
+        const CUtensorMap* const map = keys ? &key_map : &value_map;
+        const int unit = lane >> 1;
+        const int half = lane & 1;
+        pdl_wait();
+        for (int m = 0; ok; ++m) {
+            ok = att_wait(&sm.list_ready[m & 1], (m >> 1) & 1, sm, status);
+            const int count = ok ? sm.task_count[m & 1] : -1;
+            if (count < 0) {
+                break;
+            }
+            for (int i = 0; i < count && ok; ++i) {
+                const Task task = sm.tasks[m & 1][i];
+                const uint32_t* table = block_tables + static_cast<size_t>(task.row) * max_blocks;
+                const int stages = (task.units + kStageUnits - 1) / kStageUnits;
+                for (int st = 0; st < stages; ++st, ++n) {
+                    const int slot = n % kStages;
+                    const int first = task.unit_begin + st * kStageUnits;
+                    const int units = min(kStageUnits, task.units - st * kStageUnits);
+                    // the page id is fetched before the wait for a free slot, which is the longer of the two
+                    const uint32_t physical = unit < units ? table[(first + unit) / units_per_page] : 0u;
+                    ok = att_wait(&empty[slot], ((n / kStages) & 1) ^ 1, sm, status);
+                    if (!ok) {
+                        break;
+                    }
+                    if (lane == 0) {
+                        mbar_arrive_expect_tx(&full[slot], static_cast<uint32_t>(units) * 2 * kBoxBytes);
+                    }
+                    __syncwarp();
+                    if (unit < units) {
+                        const int row = (static_cast<int>(physical) * kKvHeads + task.kv_head) * page_size +
+                                        (first + unit) % units_per_page * kUnitTokens;
+                        tma_box_g2s(ring + slot * kStageBytes + half * kHalfBytes + unit * kBoxBytes, map, half * 128, row,
+                                    &full[slot]);
+                    }
+                    __syncwarp();
+                }
+            }
+            __syncwarp();
+            if (lane == 0 && ok) {
+if (keys) {
+                    mbar_arrive(&sm.list_wanted);
+                }
+                                mbar_arrive(&sm.list_free[m & 1]);
+            }
+        }
+        if (!ok) {
+            // copies that were asked for may still be landing in this CTA's shared memory: wait for the last trip
+            // round the ring, 0.2 ms per slot at most
+            for (int i = n > kStages ? n - kStages : 0; i < n; ++i) {
+                const long long start = clock64();
+                while (!mbar_try_wait(&full[i % kStages], (i / kStages) & 1) && clock64() - start < 400000ll) {
+                }
+            }
+            __syncwarp();
+        }
+    } else if (warp == kMmaWarp) {
+        // ---------------- tensor-core issue ---------------------------------------------------
+        const uint32_t idesc_scores = (1u << 4) | (static_cast<uint32_t>(kColumns >> 3) << 17) | (8u << 24);
+        const uint32_t idesc_output = idesc_scores | (1u << 15) | (1u << 16);  // both operands MN-major
+        const uint32_t k_base = smem_u32(&sm.k[0][0]), v_base = smem_u32(&sm.v[0][0]);
+        const uint32_t q_base = smem_u32(&sm.q[0][0]), p_base = smem_u32(&sm.p[0][0]);
+        // O of stage m
+        const auto issue_output = [&](int m) {
+            const int slot = m % kStages;
+            const int buffer = m & 1;
+            const bool ready = att_wait(&sm.p_ready[buffer], (m >> 1) & 1, sm, status) &&
+                               att_wait(&sm.v_full[slot], (m / kStages) & 1, sm, status) &&
+                               att_wait(&sm.o_free[buffer], ((m >> 1) & 1) ^ 1, sm, status);
+            if (!ready) {
+                return false;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one()) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const uint32_t d = tmem_base + kOutputColumn + (2 * buffer + half) * kColumns;
+#pragma unroll
+                    for (int ks = 0; ks < kStageTokens / 32; ++ks) {
+                        // 32 tokens: four atoms of V; P: columns in chunks of 16, a chunk's tokens 16 bytes apart
+                        umma_fp8(d, swizzled_descriptor(v_base + slot * kStageBytes + half * kHalfBytes + ks * 4096),
+                                 smem_descriptor(p_base + buffer * kProbabilityBytes + ks * 512, 128, kStageTokens * 16),
+                                 idesc_output, ks > 0 ? 1u : 0u);
+                    }
+                }
+                umma_commit(&sm.v_empty[slot]);
+                umma_commit(&sm.p_free[buffer]);
+                umma_commit(&sm.o_ready[buffer]);
+                mbar_arrive(&sm.o_ready[buffer]);
+            }
+            __syncwarp();
+            return true;
+        };
+        int issued = 0;  // O of this many stages
+        for (int m = 0; ok; ++m) {
+            ok = att_wait(&sm.list_ready[m & 1], (m >> 1) & 1, sm, status);
+            const int count = ok ? sm.task_count[m & 1] : -1;
+            if (count < 0) {
+                break;
+            }
+            for (int i = 0; i < count && ok; ++i) {
+                const int stages = (sm.tasks[m & 1][i].units + kStageUnits - 1) / kStageUnits;
+                ok = att_wait(&sm.q_ready[t & 1], (t >> 1) & 1, sm, status);
+                for (int st = 0; st < stages && ok; ++st) {
+                    const int slot = n % kStages;
+                    const int buffer = n & 1;
+                    ok = att_wait(&sm.k_full[slot], (n / kStages) & 1, sm, status) &&
+                         att_wait(&sm.s_free[buffer], ((n >> 1) & 1) ^ 1, sm, status);
+                    if (!ok) {
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (elect_one()) {
+                        const uint32_t d = tmem_base + kScoreColumn + buffer * kColumns;
+#pragma unroll
+                        for (int half = 0; half < 2; ++half) {
+#pragma unroll
+                            for (int ks = 0; ks < 4; ++ks) {
+                                umma_fp8(d, swizzled_descriptor(k_base + slot * kStageBytes + half * kHalfBytes + ks * 32),
+                                         smem_descriptor(q_base + (t & 1) * kQueryBytes + (half * 4 + ks) * 32 * kColumns,
+                                                         kColumns * 16, 128),
+                                         idesc_scores, (half > 0 || ks > 0) ? 1u : 0u);
+                            }
+                        }
+                        umma_commit(&sm.k_empty[slot]);
+                        umma_commit(&sm.s_ready[buffer]);
+                        if (st == stages - 1) {
+                            umma_commit(&sm.q_free[t & 1]);
+                        }
+                    }
+                    __syncwarp();
+                    ++n;
+                    if (issued < n - 1) {
+                        ok = issue_output(issued);
+                        issued += ok ? 1 : 0;
+                    }
+                }
+                if (stages == 0 && ok) {
+                    // Nothing to multiply.  What is pending goes now: after a few tasks like this one the next query
+                    // waits for the softmax warps, they for the output warps, and these for it.
+                    if (issued < n) {
+                        ok = issue_output(issued);
+                        issued += ok ? 1 : 0;
+                    }
+                    if (lane == 0) {
+                        mbar_arrive(&sm.q_free[t & 1]);
+                    }
+                    __syncwarp();
+                }
+                ++t;
+            }
+            // (the next chunk may be a while in coming)
+            if (ok && issued < n) {
+                ok = issue_output(issued);
+                issued += ok ? 1 : 0;
+            }
+            __syncwarp();
+            if (lane == 0 && ok) {
+                mbar_arrive(&sm.list_free[m & 1]);
+            }
+        }
+        if (!ok && n > 0) {
+            // the MMAs that were issued still read shared memory and write tensor memory: wait for the last of
+            // them (0.2 ms at most) before the CTA gives either back
+            const long long start = clock64();
+            while (!(mbar_try_wait(&sm.k_empty[(n - 1) % kStages], ((n - 1) / kStages) & 1) &&
+                     (issued == 0 || mbar_try_wait(&sm.v_empty[(issued - 1) % kStages], ((issued - 1) / kStages) & 1))) &&
+                   clock64() - start < 400000ll) {
+            }
+            __syncwarp();
+        }
+    } else if (warp < kSoftmaxWarps) {
+        // ---------------- softmax: thread = token ---------------------------------------------
+        const uint32_t s_lane = tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + kScoreColumn;
+        const int token = threadIdx.x;
+        pdl_wait();
+        for (int m = 0; ok; ++m) {
+            ok = att_wait(&sm.list_ready[m & 1], (m >> 1) & 1, sm, status);
+            const int count = ok ? sm.task_count[m & 1] : -1;
+            if (count < 0) {
+                break;
+            }
+            for (int i = 0; i < count && ok; ++i) {
+                const Task task = sm.tasks[m & 1][i];
+                const int stages = (task.units + kStageUnits - 1) / kStageUnits;
+                ok = att_wait(&sm.q_ready[t & 1], (t >> 1) & 1, sm, status);
                 if (!ok) {
                     break;
                 }
-                if (lane == 0) {
-                    mbar_arrive_expect_tx(&sm.full[slot], static_cast<uint32_t>(count) * 2 * kUnitBytes);
-                }
-                __syncwarp();
-                if (lane < count) {
-                    const int unit = first + lane;
-                    const size_t offset = ((static_cast<size_t>(physical) * kKvHeads + task.kv_head) * page_size +
-                                           static_cast<size_t>(unit % units_per_page) * kUnitTokens) *
-                                          kHeadDim;
-                    bulk_g2s(&sm.k[slot][lane * kUnitPitch], key_cache + offset, kUnitBytes, &sm.full[slot]);
-                    bulk_g2s(&sm.v[slot][lane * kUnitPitch], value_cache + offset, kUnitBytes, &sm.full[slot]);
+                const float k_scale = key_scales ? key_scales[task.kv_head] : 1.0f;
+                float score_scale[kGqaGroup], running_max[kGqaGroup], running_sum[kGqaGroup];
+#pragma unroll
+                for (int h = 0; h < kGqaGroup; ++h) {
+                    score_scale[h] = softmax_scale * k_scale * kLog2e * sm.query_scale[t & 1][h];
+                    running_max[h] = -INFINITY;  // log2 domain, the same in all threads
+                    running_sum[h] = 0.0f;       // this thread's tokens only
                 }
                 __syncwarp();
                 if (lane == 0) {
-                    *reinterpret_cast<volatile int*>(&sm.issued) = n + 1;
+                    mbar_arrive(&sm.q_free[t & 1]);  // (the scales have been read)
                 }
-            }
-        }
-        if (!ok && lane == 0) {
-            *reinterpret_cast<volatile int*>(&sm.producer_failed) = 1;
-        }
-    } else {
-        // ---------------- consumers ---------------------------------------------------------
-        const uint32_t v_base = smem_u32(&sm.v[0][0]);
-        int n = 0;  // stages consumed so far
-        bool ok = true;
-        // bf16 words of this lane's query fragments (head g of the task's group; rows 6, 7 are padding)
-        uint2 q_raw[16];
-        auto load_query = [&](const Task& next) {
-            const int head = next.kv_head * kGqaGroup + g;
-            const __nv_bfloat16* qp = query + (static_cast<size_t>(next.row) * kQueryHeads + head) * kHeadDim;
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const int unit = 2 * t + (m & 1) + 8 * (m >> 1);
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    q_raw[m * 4 + s] = g < kGqaGroup ? *reinterpret_cast<const uint2*>(qp + 16 * unit + 4 * s)
-                                                     : make_uint2(0u, 0u);
-                }
-            }
-        };
-        if (task_count > 0) {
-            load_query(sm.tasks[0]);
-        }
-        for (int ti = 0; ti < task_count && ok; ++ti) {
-            const Task task = sm.tasks[ti];
-            const int row = task.row;
-            const int kv_head = task.kv_head;
-            const int context = task.context;
-
-            // Query A fragments for the 16 k-steps.  K fragment reads take 16-byte bank group
-            // u(t, m) = 2t + (m & 1) + 8 (m >> 1) of a token row in load m, so k-step (m, s)
-            // contracts dims 16 u + 4 s .. + 3 for t = 0..3: Q uses the same permutation.
-            // The raw bf16 words were fetched while the previous task was computed.
-            uint32_t qa[16][2];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                qa[i][0] = pack_half2(__uint_as_float(q_raw[i].x << 16), __uint_as_float(q_raw[i].x & 0xffff0000u));
-                qa[i][1] = pack_half2(__uint_as_float(q_raw[i].y << 16), __uint_as_float(q_raw[i].y & 0xffff0000u));
-            }
-            if (ti + 1 < task_count) {
-                load_query(sm.tasks[ti + 1]);  // in flight during this task
-            }
-            const float k_scale = key_scales ? key_scales[kv_head] : 1.0f;
-            const float score_scale = softmax_scale * k_scale * kLog2e;
-
-            float oacc[2][2][4];
-#pragma unroll
-            for (int a = 0; a < 2; ++a) {
-#pragma unroll
-                for (int b = 0; b < 2; ++b) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        oacc[a][b][c] = 0.0f;
+                for (int st = 0; st < stages; ++st, ++n) {
+                    const int buffer = n & 1;
+                    const uint32_t parity = (n >> 1) & 1;
+                    ok = att_wait(&sm.s_ready[buffer], parity, sm, status);
+                    if (!ok) {
+                        break;
                     }
-                }
-            }
-            float running_max = -INFINITY;  // log2 domain, shared by all warps
-            float running_sum = 0.0f;       // this warp's tokens only
-
-            const int stages = (task.units + kStageUnits - 1) / kStageUnits;
-            for (int st = 0; st < stages; ++st, ++n) {
-                const int slot = n % kStages;
-                if (*reinterpret_cast<volatile int*>(&sm.failed) != 0 ||
-                    !mbar_wait_bounded(&sm.full[slot], (n / kStages) & 1, kStatusAttentionPageWait, status)) {
-                    *reinterpret_cast<volatile int*>(&sm.failed) = 1;  // acted on after the next barrier, by all
-                }
-                const int first_token = (task.unit_begin + st * kStageUnits) * kUnitTokens;
-                const int units_here = task.units - st * kStageUnits;
-
-                // ---- S = Q K^T for this warp's two column tiles (tokens 2w, 2w + 1 of each unit)
-                float acc[2][2][4];
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    uint32_t d01[16], d2[8];
+                    tmem_load16_issue(s_lane + buffer * kColumns, d01);
+                    tmem_load8_issue(s_lane + buffer * kColumns + 16, d2);
+                    tmem_load_wait();
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&sm.s_free[buffer]);
+                    }
+                    const bool valid = (task.unit_begin + st * kStageUnits) * kUnitTokens + token < task.context &&
+                                       token < (task.units - st * kStageUnits) * kUnitTokens;
+                    float score[kGqaGroup];
+                    float mine = -INFINITY;
 #pragma unroll
-                for (int a = 0; a < 2; ++a) {
+                    for (int h = 0; h < kGqaGroup; ++h) {
+                        score[h] = valid ? combine_digits(d01[h], d01[8 + h], d2[h]) * score_scale[h] : -INFINITY;
+                        const float highest = warp_highest(score[h]);
+                        mine = lane == h ? highest : mine;
+                    }
+                    if (lane < 8) {
+                        sm.warp_max[buffer][warp][lane] = mine;
+                    }
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&sm.max_ready[buffer]);
+                    }
+                    ok = att_wait(&sm.max_ready[buffer], parity, sm, status);
+                    if (!ok) {
+                        break;
+                    }
+                    float probability[kGqaGroup], factor[kGqaGroup];
 #pragma unroll
-                    for (int b = 0; b < 2; ++b) {
+                    for (int h = 0; h < kGqaGroup; ++h) {
+                        float new_max = running_max[h];
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            acc[a][b][c] = 0.0f;
+                        for (int w = 0; w < kSoftmaxWarps; ++w) {
+                            new_max = fmaxf(new_max, sm.warp_max[buffer][w][h]);
+                        }
+                        factor[h] = new_max == -INFINITY ? 1.0f : exp2f(running_max[h] - new_max);
+                        probability[h] = new_max == -INFINITY ? 0.0f : exp2f(score[h] - new_max);
+                        running_sum[h] = fmaf(running_sum[h], factor[h], probability[h]);
+                        running_max[h] = new_max;
+                        probability[h] *= 256.0f;
+                    }
+                    uint32_t words[2 * kDigits];
+#pragma unroll
+                    for (int j = 0; j < kDigits; ++j) {
+                        const uint32_t pair0 = take_digit(probability[0], probability[1]);
+                        const uint32_t pair1 = take_digit(probability[2], probability[3]);
+                        words[2 * j] = pair0 | pair1 << 16;
+                        words[2 * j + 1] = take_digit(probability[4], probability[5]);
+                    }
+                    ok = att_wait(&sm.p_free[buffer], parity ^ 1, sm, status);
+                    if (!ok) {
+                        break;
+                    }
+                    *reinterpret_cast<uint4*>(&sm.p[buffer][token * 16]) = make_uint4(words[0], words[1], words[2], words[3]);
+                    *reinterpret_cast<uint4*>(&sm.p[buffer][(kStageTokens + token) * 16]) = make_uint4(words[4], words[5], 0u, 0u);
+                    // (four buffers: these words of stage n + 4 come after O of stage n + 2, which comes after the
+                    // output warps have read stage n)
+                    if (token == 0) {
+#pragma unroll
+                        for (int h = 0; h < kGqaGroup; ++h) {
+                            sm.rescale[n & 3][h] = factor[h];
                         }
                     }
-                }
-                const uint8_t* krow = &sm.k[slot][g * kUnitPitch + (2 * warp) * kHeadDim];
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const int unit = 2 * t + (m & 1) + 8 * (m >> 1);
-                    const uint4 raw0 = *reinterpret_cast<const uint4*>(krow + 16 * unit);
-                    const uint4 raw1 = *reinterpret_cast<const uint4*>(krow + kHeadDim + 16 * unit);
-                    const uint32_t words[2][4] = {{raw0.x, raw0.y, raw0.z, raw0.w}, {raw1.x, raw1.y, raw1.z, raw1.w}};
-#pragma unroll
-                    for (int s = 0; s < 4; ++s) {
-#pragma unroll
-                        for (int tile = 0; tile < 2; ++tile) {
-                            uint32_t b0, b1;
-                            cvt_e4m3x4(words[tile][s], b0, b1);
-                            mma_f16_16816(acc[tile][s & 1], qa[m * 4 + s][0], 0u, qa[m * 4 + s][1], 0u, b0, b1);
-                        }
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&sm.p_ready[buffer]);
                     }
                 }
-                // acc[tile][.][0], [1]: head g, tokens (unit 2t, j) and (unit 2t + 1, j), j = 2w + tile
-                float sc[2][2];
-                float local_max = -INFINITY;
-#pragma unroll
-                for (int tile = 0; tile < 2; ++tile) {
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int token = first_token + (2 * t + e) * kUnitTokens + 2 * warp + tile;
-                        const bool valid = token < context && (2 * t + e) < units_here;
-                        sc[tile][e] = valid ? (acc[tile][0][e] + acc[tile][1][e]) * score_scale : -INFINITY;
-                        local_max = fmaxf(local_max, sc[tile][e]);
-                    }
-                }
-                local_max = fmaxf(local_max, __shfl_xor_sync(0xffffffffu, local_max, 1));
-                local_max = fmaxf(local_max, __shfl_xor_sync(0xffffffffu, local_max, 2));
-                if (t == 0) {
-                    sm.warp_max[warp][g] = local_max;
-                }
-                // The flags can change at any moment (the producer raises its own asynchronously), so a
-                // consumer that read them for itself after the barrier could leave while another stays and
-                // waits at the next barrier for ever.  One thread samples them before the barrier into the
-                // word of this stage; every consumer acts on that word only.  A failure that thread 0 has
-                // not seen yet is acted on one stage later.
-                if (threadIdx.x == 0) {
-                    sm.leave[n & 1] = *reinterpret_cast<volatile int*>(&sm.failed) |
-                                      *reinterpret_cast<volatile int*>(&sm.producer_failed);
-                }
-                consumer_sync();
-                ok = *reinterpret_cast<volatile int*>(&sm.leave[n & 1]) == 0;
                 if (!ok) {
-                    break;  // the same word for every consumer: they leave together
+                    break;
                 }
-
-                float new_max = running_max;
-#pragma unroll
-                for (int w = 0; w < kConsumerWarps; ++w) {
-                    new_max = fmaxf(new_max, sm.warp_max[w][g]);
+                ok = att_wait(&sm.t_free[t & 1], ((t >> 1) & 1) ^ 1, sm, status);
+                if (!ok) {
+                    break;
                 }
-                const float rescale = new_max == -INFINITY ? 1.0f : exp2f(running_max - new_max);
-                running_max = new_max;
-                float row_sum = 0.0f;
-                uint32_t pfrag[2];
+                float mine = 0.0f;
 #pragma unroll
-                for (int tile = 0; tile < 2; ++tile) {
-                    const float p0 = new_max == -INFINITY ? 0.0f : exp2f(sc[tile][0] - new_max);
-                    const float p1 = new_max == -INFINITY ? 0.0f : exp2f(sc[tile][1] - new_max);
-                    row_sum += p0 + p1;
-                    pfrag[tile] = pack_half2(p0, p1);
-                }
-                running_sum = running_sum * rescale + row_sum;
-                // PV k-step kk contracts tokens j = 2 kk and 2 kk + 1 of the eight units: this warp's two tiles.
-                sm.p[warp][lane] = make_uint2(pfrag[0], pfrag[1]);
-#pragma unroll
-                for (int a = 0; a < 2; ++a) {
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        oacc[a][b][0] *= rescale;
-                        oacc[a][b][1] *= rescale;
+                for (int h = 0; h < kGqaGroup; ++h) {
+                    const float sum = warp_sum(running_sum[h]);
+                    mine = lane == h ? sum : mine;
+                    if (token == 0) {
+                        sm.task_max[t & 1][h] = running_max[h];
                     }
                 }
-                consumer_sync();
-
-                // ---- O += P V for this warp's 32 output dims --------------------------------
-                const uint32_t v_slot = v_base + slot * kStageBytes;
-                const int matrix = lane >> 3;
-                const uint32_t v_lane = v_slot + (lane & 7) * kUnitPitch + (matrix & 1) * kHeadDim +
-                                        (2 * warp + (matrix >> 1)) * 16;
-#pragma unroll
-                for (int kk = 0; kk < kStageUnits; ++kk) {
-                    const uint2 pa = sm.p[kk][lane];
-                    uint32_t r[4];
-                    ldmatrix_x4_trans(r, v_lane + 2 * kk * kHeadDim);
-#pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        // bytes (b0, b2 | b1, b3): low pair feeds the even dim, high pair the odd dim
-                        const uint32_t lo_tokens = __byte_perm(r[2 * half], 0, 0x3120);
-                        const uint32_t hi_tokens = __byte_perm(r[2 * half + 1], 0, 0x3120);
-                        uint32_t even0, odd0, even1, odd1;
-                        cvt_e4m3x4(lo_tokens, even0, odd0);
-                        cvt_e4m3x4(hi_tokens, even1, odd1);
-                        mma_f16_16816(oacc[half][0], pa.x, 0u, pa.y, 0u, even0, even1);
-                        mma_f16_16816(oacc[half][1], pa.x, 0u, pa.y, 0u, odd0, odd1);
-                    }
+                if (lane < 8) {
+                    sm.task_sum[t & 1][warp][lane] = mine;
                 }
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive(&sm.empty[slot]);
+                    mbar_arrive(&sm.t_ready[t & 1]);
                 }
+                ++t;
             }
-            if (!ok) {
+            __syncwarp();
+            if (lane == 0 && ok) {
+                mbar_arrive(&sm.list_free[m & 1]);
+            }
+        }
+    } else if (warp == kQueryWarp) {
+        // ---------------- query digits: eight dims per lane, one head after the other ----------------
+        pdl_wait();
+        for (int m = 0; ok; ++m) {
+            ok = att_wait(&sm.list_ready[m & 1], (m >> 1) & 1, sm, status);
+            const int count = ok ? sm.task_count[m & 1] : -1;
+            if (count < 0) {
                 break;
             }
-
-            // ---- combine the warps' sums, normalise, write --------------------------------
-            running_sum += __shfl_xor_sync(0xffffffffu, running_sum, 1);
-            running_sum += __shfl_xor_sync(0xffffffffu, running_sum, 2);
-            if (t == 0) {
-                sm.warp_sum[warp][g] = running_sum;
-            }
-            consumer_sync();
-            float total = 0.0f;
+            for (int i = 0; i < count && ok; ++i) {
+                const Task task = sm.tasks[m & 1][i];
+                const uint2* at_lane = reinterpret_cast<const uint2*>(
+                    query + (static_cast<size_t>(task.row) * kQueryHeads + task.kv_head * kGqaGroup) * kHeadDim + 8 * lane);
+                uint2 raw[kGqaGroup][2];  // (rows start on 8-byte boundaries)
 #pragma unroll
-            for (int w = 0; w < kConsumerWarps; ++w) {
-                total += sm.warp_sum[w][g];
-            }
-            consumer_sync();  // the sums are read before the next task overwrites them
-            if (g < kGqaGroup) {
-                const float v_scale = value_scales ? value_scales[kv_head] : 1.0f;
-                const float inverse = total > 0.0f ? v_scale / total : 0.0f;
-                const int head = kv_head * kGqaGroup + g;
-                const size_t pair = static_cast<size_t>(row - row_base) * kQueryHeads + head;
-                if (kSplit) {
-                    const size_t slot_index = pair * partitions + task.part;
-                    if (warp == 0 && t == 0) {
-                        float* stats = partial_stats + slot_index * kPartialFloats;
-                        stats[0] = running_max;
-                        stats[1] = total;
+                for (int h = 0; h < kGqaGroup; ++h) {
+                    raw[h][0] = at_lane[h * (kHeadDim / 4)];
+                    raw[h][1] = at_lane[h * (kHeadDim / 4) + 1];
+                }
+                ok = att_wait(&sm.q_free[t & 1], ((t >> 1) & 1) ^ 1, sm, status);
+                if (!ok) {
+                    break;
+                }
+#pragma unroll
+                for (int h = 0; h < kGqaGroup; ++h) {
+                    const uint32_t pairs[4] = {raw[h][0].x, raw[h][0].y, raw[h][1].x, raw[h][1].y};
+                    uint32_t highest = 0;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        highest = max(highest, max(pairs[j] & 0x7fffu, (pairs[j] >> 16) & 0x7fffu));
                     }
-                    __half* po = partial_out + slot_index * kHeadDim;
+                    highest = __reduce_max_sync(0xffffffffu, highest);
+                    // largest magnitude to [128, 256).  With an infinity in the head only the infinities count, and
+                    // the scores become infinities (or NaN) when they are scaled back; a NaN is an e4m3 NaN.
+                    const uint32_t exponent = max(highest >> 7, 8u);
+                    const bool infinite = highest >= 0x7f80u;
+                    const float up = __uint_as_float((261u - exponent) << 23);
+                    uint32_t bytes[kDigits][2];
 #pragma unroll
-                    for (int a = 0; a < 2; ++a) {
-                        const int d = 16 * (2 * warp + a) + 4 * t;
-                        const uint2 packed = make_uint2(pack_half2(oacc[a][0][0] * inverse, oacc[a][1][0] * inverse),
-                                                        pack_half2(oacc[a][0][1] * inverse, oacc[a][1][1] * inverse));
-                        *reinterpret_cast<uint2*>(po + d) = packed;
-                    }
-                } else {
-                    __nv_bfloat16* op = output + (static_cast<size_t>(row) * kQueryHeads + head) * kHeadDim;
-                    const __nv_bfloat16* gp = query_gate_projection
-                                                  ? query_gate_projection + static_cast<size_t>(row) * gate_stride +
-                                                        head * (2 * kHeadDim) + kHeadDim
-                                                  : nullptr;
-#pragma unroll
-                    for (int a = 0; a < 2; ++a) {
-                        const int d = 16 * (2 * warp + a) + 4 * t;
-                        float values[4] = {oacc[a][0][0] * inverse, oacc[a][1][0] * inverse, oacc[a][0][1] * inverse,
-                                           oacc[a][1][1] * inverse};
-                        if (gp != nullptr) {
-                            const uint2 graw = *reinterpret_cast<const uint2*>(gp + d);
-                            const float gates[4] = {__uint_as_float(graw.x << 16), __uint_as_float(graw.x & 0xffff0000u),
-                                                    __uint_as_float(graw.y << 16), __uint_as_float(graw.y & 0xffff0000u)};
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                values[i] *= 1.0f / (1.0f + __expf(-gates[i]));
-                            }
+                    for (int j = 0; j < 4; ++j) {
+                        float lo = __uint_as_float(pairs[j] << 16), hi = __uint_as_float(pairs[j] & 0xffff0000u);
+                        if (infinite) {
+                            lo = isnan(lo) ? lo : isinf(lo) ? copysignf(1.0f, lo) : 0.0f;
+                            hi = isnan(hi) ? hi : isinf(hi) ? copysignf(1.0f, hi) : 0.0f;
+                        } else {
+                            lo *= up;
+                            hi *= up;
                         }
-                        __nv_bfloat162 lo = __floats2bfloat162_rn(values[0], values[1]);
-                        __nv_bfloat162 hi = __floats2bfloat162_rn(values[2], values[3]);
-                        uint2 packed;
-                        packed.x = *reinterpret_cast<uint32_t*>(&lo);
-                        packed.y = *reinterpret_cast<uint32_t*>(&hi);
+#pragma unroll
+                        for (int d = 0; d < kDigits; ++d) {
+                            const uint32_t digit = take_digit(lo, hi);
+                            bytes[d][j >> 1] = (j & 1) ? bytes[d][j >> 1] | digit << 16 : digit;
+                        }
+                    }
+                    uint8_t* const at = &sm.q[t & 1][(lane >> 1) * 16 * kColumns + h * 16 + (lane & 1) * 8];
+#pragma unroll
+                    for (int d = 0; d < kDigits; ++d) {
+                        *reinterpret_cast<uint2*>(at + d * 128) = make_uint2(bytes[d][0], bytes[d][1]);
+                    }
+                    if (lane == 0) {
+                        sm.query_scale[t & 1][h] = infinite ? INFINITY : __uint_as_float((exponent - 7u) << 23);
+                    }
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&sm.q_ready[t & 1]);
+                }
+                ++t;
+            }
+            __syncwarp();
+            if (lane == 0 && ok) {
+                mbar_arrive(&sm.list_free[m & 1]);
+            }
+        }
+    } else if (warp < kMmaWarp) {
+        // ---------------- outputs: thread = dim -----------------------------------------------
+        const int o_warp = warp - kFirstOutputWarp;
+        const int half = o_warp >> 2;
+        const int dim = half * 128 + (o_warp & 3) * 32 + lane;
+        const uint32_t o_lane = tmem_base + (static_cast<uint32_t>((o_warp & 3) * 32) << 16) + kOutputColumn + half * kColumns;
+        pdl_wait();
+        for (int m = 0; ok; ++m) {
+            ok = att_wait(&sm.list_ready[m & 1], (m >> 1) & 1, sm, status);
+            const int count = ok ? sm.task_count[m & 1] : -1;
+            if (count < 0) {
+                break;
+            }
+            for (int i = 0; i < count && ok; ++i) {
+                const Task task = sm.tasks[m & 1][i];
+                const int row = task.row;
+                const int kv_head = task.kv_head;
+                const int stages = (task.units + kStageUnits - 1) / kStageUnits;
+                float total[kGqaGroup];
+#pragma unroll
+                for (int h = 0; h < kGqaGroup; ++h) {
+                    total[h] = 0.0f;
+                }
+                for (int st = 0; st < stages; ++st, ++n) {
+                    const int buffer = n & 1;
+                    ok = att_wait(&sm.o_ready[buffer], (n >> 1) & 1, sm, status);
+                    if (!ok) {
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    uint32_t d01[16], d2[8];
+                    tmem_load16_issue(o_lane + 2 * buffer * kColumns, d01);
+                    tmem_load8_issue(o_lane + 2 * buffer * kColumns + 16, d2);
+                    float factor[kGqaGroup];
+#pragma unroll
+                    for (int h = 0; h < kGqaGroup; ++h) {
+                        factor[h] = sm.rescale[n & 3][h];
+                    }
+                    tmem_load_wait();
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&sm.o_free[buffer]);
+                    }
+#pragma unroll
+                    for (int h = 0; h < kGqaGroup; ++h) {
+                        total[h] = fmaf(total[h], factor[h], combine_digits(d01[h], d01[8 + h], d2[h]));
+                    }
+                }
+                if (!ok) {
+                    break;
+                }
+                ok = att_wait(&sm.t_ready[t & 1], (t >> 1) & 1, sm, status);
+                if (!ok) {
+                    break;
+                }
+                // (the probabilities were multiplied with 256)
+                const float v_scale = (value_scales ? value_scales[kv_head] : 1.0f) * 0.00390625f;
+#pragma unroll
+                for (int h = 0; h < kGqaGroup; ++h) {
+                    float denominator = 0.0f;
+#pragma unroll
+                    for (int w = 0; w < kSoftmaxWarps; ++w) {
+                        denominator += sm.task_sum[t & 1][w][h];
+                    }
+                    const float inverse = denominator > 0.0f ? v_scale / denominator : 0.0f;
+                    const float value = total[h] * inverse;
+                    const int head = kv_head * kGqaGroup + h;
+                    const size_t pair = static_cast<size_t>(row - row_base) * kQueryHeads + head;
+                    if (kSplit) {
+                        const size_t slot = pair * partitions + task.part;
+                        if (dim == 0) {
+                            float* stats = partial_stats + slot * kPartialFloats;
+                            stats[0] = sm.task_max[t & 1][h];
+                            // the last piece of a pair carries a sign
+                        stats[1] = task.last ? __uint_as_float(__float_as_uint(denominator) | 0x80000000u) : fabsf(denominator);
+                        }
+                        partial_out[slot * kHeadDim + dim] = __float2half_rn(value);
+                    } else {
+                        float gated = value;
+                        if (query_gate_projection != nullptr) {
+                            const float gate = __bfloat162float(query_gate_projection[static_cast<size_t>(row) * gate_stride +
+                                                                                      head * (2 * kHeadDim) + kHeadDim + dim]);
+                            gated *= 1.0f / (1.0f + __expf(-gate));
+                        }
+                        const __nv_bfloat16 rounded = __float2bfloat16(gated);
                         if (output != nullptr) {
-                            *reinterpret_cast<uint2*>(op + d) = packed;
+                            output[(static_cast<size_t>(row) * kQueryHeads + head) * kHeadDim + dim] = rounded;
                         }
                         if (staged_output != nullptr) {
-                            // the same values as f16 in the operand layout of the output projection
-                            const int feature = head * kHeadDim + d;
-                            *reinterpret_cast<uint2*>(staged_output +
-                                                      (static_cast<size_t>(feature >> 3) * padded_rows + row) * 8 +
-                                                      (feature & 7)) =
-                                make_uint2(bf16x2_to_f16x2(packed.x), bf16x2_to_f16x2(packed.y));
+                            // the same value as f16 in the operand layout of the output projection
+                            const int feature = head * kHeadDim + dim;
+                            staged_output[(static_cast<size_t>(feature >> 3) * padded_rows + row) * 8 + (feature & 7)] =
+                                __float2half_rn(fminf(fmaxf(__bfloat162float(rounded), -65504.0f), 65504.0f));
                         }
                     }
                 }
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&sm.t_free[t & 1]);
+                }
+                ++t;
+            }
+            __syncwarp();
+            if (lane == 0 && ok) {
+                mbar_arrive(&sm.list_free[m & 1]);
             }
         }
-        if (threadIdx.x == 0) {
-            sm.consumed = n;
-        }
     }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    // After a failed wait the CTA must not return while copies it issued are still landing:
-    // one thread waits (bounded) for the stages that were put in flight and never consumed.
-    if (threadIdx.x == 0 && (sm.failed | sm.producer_failed) != 0) {
-        for (int i = sm.consumed; i < sm.issued; ++i) {
-            mbar_wait_bounded(&sm.full[i % kStages], (i / kStages) & 1, kStatusAttentionPageWait, status);
-        }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemColumns) : "memory");
     }
 }
 
 // Log-sum-exp merge of the partitions, output gate, bf16 store (as cuda/paged_attention.cu:1736-1823).
-// One CTA of four warps per (row, head): the longest row of a ragged batch has dozens of partials,
-// and a single warp walking them is a chain of dependent memory round trips.  Warp w takes the
-// partials w, w + 4, ... (eight dims per lane), the four sums meet in shared memory in warp order.
-constexpr int kMergeWarps = 4;
+// One CTA per (row, head): the longest row of a ragged batch has dozens of partials, and a single warp walking them
+// is a chain of dependent memory round trips.  Warp w takes the partials w, w + 8, ... (eight dims per lane), the
+// sums meet in shared memory in warp order.  A pair's partials lie side by side and the sign of the sum marks the
+// last one; the slots behind it were never written.  Statistics and outputs are asked for together, before that
+// mark is known.  (The kernel used to make the
+// attention kernel's plan again, a microsecond and a half of dependent arithmetic: from the end of the wait to the
+// last store 4.4 us, now 1.6.)
+constexpr int kMergeWarps = 8;
+constexpr int kMergeDepth = 4;
 
 __global__ void __launch_bounds__(kMergeWarps * 32) reduce_partitions_kernel(
     const float* __restrict__ partial_stats, const __half* __restrict__ partial_out,
-    const __nv_bfloat16* __restrict__ query_gate_projection, const uint32_t* __restrict__ context_lengths,
-    __nv_bfloat16* __restrict__ output, __half* __restrict__ staged_output, int padded_rows, int rows, int partitions,
-    int row_base, int gate_stride, int capacity_units, int plan_ctas) {
+    const __nv_bfloat16* __restrict__ query_gate_projection, __nv_bfloat16* __restrict__ output,
+    __half* __restrict__ staged_output, int padded_rows, int partitions, int row_base, int gate_stride) {
     pdl_launch_dependents();  // the output projection may start streaming its weights
-    pdl_wait();
     __shared__ float sums[kMergeWarps][kHeadDim];
     __shared__ float denominators[kMergeWarps];
     const int pair = blockIdx.x;  // (row, head)
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    // The same plan as the attention kernel made: this pair has `used` partials, the rest of its
-    // slots were never written.
-    const int plan_row = pair / kQueryHeads;
-    long long total_units = 0, units_before = 0;
-    for (int r = lane; r < rows; r += 32) {
-        const int units = plan_units(units_of_context(context_lengths[row_base + r], capacity_units));
-        total_units += units;
-        units_before += r < plan_row ? units : 0;
-    }
-#pragma unroll
-    for (int offset = 16; offset > 0; offset >>= 1) {
-        total_units += __shfl_xor_sync(0xffffffffu, total_units, offset);
-        units_before += __shfl_xor_sync(0xffffffffu, units_before, offset);
-    }
-    const SplitPlan plan = make_split_plan(total_units, rows, capacity_units, partitions, plan_ctas);
-    const int occupied = plan_units(units_of_context(context_lengths[row_base + plan_row], capacity_units));
-    const long long start = pair_position(plan, plan_row, (pair % kQueryHeads) / kGqaGroup, units_before, occupied);
-    const int used = static_cast<int>((start + occupied - 1) / plan.share - start / plan.share) + 1;
-    const float* stats = partial_stats + static_cast<size_t>(pair) * partitions * kPartialFloats;
-    // every warp finds the maximum over all partials (lanes side by side) ...
-    float maximum = -INFINITY;
-    for (int p = lane; p < used; p += 32) {
-        const float2 pair_stats = *reinterpret_cast<const float2*>(stats + 2 * p);
-        if (pair_stats.y > 0.0f) {
-            maximum = fmaxf(maximum, pair_stats.x);
-        }
-    }
-#pragma unroll
-    for (int offset = 16; offset > 0; offset >>= 1) {
-        maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, offset));
-    }
-    // ... and sums its own quarter of them, four outputs in flight at a time
-    float denominator = 0.0f;
-    float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    const int row = row_base + pair / kQueryHeads;
+    const int head = pair % kQueryHeads;
+    const float2* stats = reinterpret_cast<const float2*>(partial_stats) + static_cast<size_t>(pair) * partitions;
     const __half* outs = partial_out + static_cast<size_t>(pair) * partitions * kHeadDim + 8 * lane;
-    for (int first = warp; first < used; first += 4 * kMergeWarps) {
-        uint4 raw[4];
-        float weight[4];
+    pdl_wait();
+    uint4 raw[kMergeDepth];
+    float2 raw_stats[kMergeDepth];
+    const auto fetch = [&](int first, int end) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < kMergeDepth; ++j) {
             const int p = first + j * kMergeWarps;
-            weight[j] = 0.0f;
+            raw_stats[j] = make_float2(-INFINITY, 0.0f);
             raw[j] = make_uint4(0, 0, 0, 0);
-            if (p < used) {
-                const float2 pair_stats = *reinterpret_cast<const float2*>(stats + 2 * p);
-                weight[j] = pair_stats.y > 0.0f ? pair_stats.y * exp2f(pair_stats.x - maximum) : 0.0f;
+            if (p < end) {
+                raw_stats[j] = stats[p];
                 raw[j] = *reinterpret_cast<const uint4*>(outs + static_cast<size_t>(p) * kHeadDim);
             }
         }
+    };
+    fetch(warp, partitions);
+    // every warp looks for the last partial and finds the maximum over all of them (lanes side by side) ...
+    float maximum = -INFINITY;
+    int used = partitions;
+    for (int base = 0; base < used; base += 32) {
+        const float2 mine = base + lane < partitions ? stats[base + lane] : make_float2(-INFINITY, 0.0f);
+        const uint32_t marks = __ballot_sync(0xffffffffu, (__float_as_uint(mine.y) >> 31) != 0);
+        if (marks != 0) {
+            used = base + __ffs(marks);
+        }
+        if (base + lane < used && fabsf(mine.y) > 0.0f) {
+            maximum = fmaxf(maximum, mine.x);
+        }
+    }
+    maximum = warp_highest(maximum);
+    // ... and adds up its own
+    float denominator = 0.0f;
+    float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    for (int first = warp; first < used; first += kMergeDepth * kMergeWarps) {
+        if (first != warp) {
+            fetch(first, used);
+        }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            denominator += weight[j];
+        for (int j = 0; j < kMergeDepth; ++j) {
+            const float sum = fabsf(raw_stats[j].y);
+            const bool present = first + j * kMergeWarps < used;
+            const float weight = present && sum > 0.0f ? sum * exp2f(raw_stats[j].x - maximum) : 0.0f;
+            denominator += weight;
             const __half2* h = reinterpret_cast<const __half2*>(&raw[j]);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const float2 f = __half22float2(h[i]);
-                acc[2 * i] += weight[j] * f.x;
-                acc[2 * i + 1] += weight[j] * f.y;
+                if (present) {  // (a slot that was never written may hold anything)
+                    acc[2 * i] += weight * f.x;
+                    acc[2 * i + 1] += weight * f.y;
+                }
             }
         }
     }
@@ -716,56 +1146,41 @@ __global__ void __launch_bounds__(kMergeWarps * 32) reduce_partitions_kernel(
         denominators[warp] = denominator;
     }
     __syncthreads();
-    if (warp != 0) {
-        return;
-    }
+    // a thread per dim
+    const int dim = threadIdx.x;
+    float total = 0.0f;
     denominator = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        acc[i] = 0.0f;
-    }
 #pragma unroll
     for (int w = 0; w < kMergeWarps; ++w) {
         denominator += denominators[w];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            acc[i] += sums[w][8 * lane + i];
-        }
+        total += sums[w][dim];
     }
     const float inverse = denominator > 0.0f ? 1.0f / denominator : 0.0f;
-    const int row = row_base + pair / kQueryHeads;
-    const int head = pair % kQueryHeads;
-    float gates[8] = {1.0f, 1.0f, 1.0f, 1.0f, 1.0f, 1.0f, 1.0f, 1.0f};
+    float gate = 1.0f;
     if (query_gate_projection != nullptr) {
-        const uint4 graw = *reinterpret_cast<const uint4*>(
-            query_gate_projection + static_cast<size_t>(row) * gate_stride + head * (2 * kHeadDim) + kHeadDim + 8 * lane);
-        const uint32_t words[4] = {graw.x, graw.y, graw.z, graw.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            gates[2 * i] = 1.0f / (1.0f + __expf(-__uint_as_float(words[i] << 16)));
-            gates[2 * i + 1] = 1.0f / (1.0f + __expf(-__uint_as_float(words[i] & 0xffff0000u)));
-        }
+        gate = __bfloat162float(
+            query_gate_projection[static_cast<size_t>(row) * gate_stride + head * (2 * kHeadDim) + kHeadDim + dim]);
+        gate = 1.0f / (1.0f + __expf(-gate));
     }
-    uint32_t packed[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        __nv_bfloat162 v = __floats2bfloat162_rn(acc[2 * i] * inverse * gates[2 * i],
-                                                  acc[2 * i + 1] * inverse * gates[2 * i + 1]);
-        packed[i] = *reinterpret_cast<uint32_t*>(&v);
-    }
+    const __nv_bfloat16 rounded = __float2bfloat16(total * inverse * gate);
     if (output != nullptr) {
-        *reinterpret_cast<uint4*>(output + (static_cast<size_t>(row) * kQueryHeads + head) * kHeadDim + 8 * lane) =
-            make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        output[(static_cast<size_t>(row) * kQueryHeads + head) * kHeadDim + dim] = rounded;
     }
     if (staged_output != nullptr) {
-        // the same values as f16 in the operand layout of the output projection: this lane's eight
-        // dims are one K core
-        const int core = head * (kHeadDim / 8) + lane;
-        *reinterpret_cast<uint4*>(staged_output + (static_cast<size_t>(core) * padded_rows + row) * 8) =
-            make_uint4(bf16x2_to_f16x2(packed[0]), bf16x2_to_f16x2(packed[1]), bf16x2_to_f16x2(packed[2]),
-                       bf16x2_to_f16x2(packed[3]));
+        // the same value as f16 in the operand layout of the output projection
+        const int feature = head * kHeadDim + dim;
+        staged_output[(static_cast<size_t>(feature >> 3) * padded_rows + row) * 8 + (feature & 7)] =
+            __float2half_rn(fminf(fmaxf(__bfloat162float(rounded), -65504.0f), 65504.0f));
     }
 }
+static_assert(kMergeWarps * 32 == kHeadDim, "a thread per dim");
+
+using AttentionKernel = void (*)(const CUtensorMap, const CUtensorMap, const __nv_bfloat16*, const __nv_bfloat16*,
+                                 const uint32_t*, const uint32_t*, const float*, const float*, __nv_bfloat16*, __half*,
+                                 int, float*, __half*, int, int, int, int, int, int, int, int, float, int*);
+const AttentionKernel attention_kernels[3] = {paged_attention_packed_kernel<false, uint32_t>,
+                                              paged_attention_packed_kernel<true, uint32_t>,
+                                              paged_attention_packed_kernel<true, unsigned long long>};
 
 cudaError_t launch_attention(const void* query, const void* query_gate_projection, const void* key_cache,
                              const void* value_cache, const void* block_tables, const void* context_lengths,
@@ -790,17 +1205,17 @@ cudaError_t launch_attention(const void* query, const void* query_gate_projectio
     if (status == nullptr) {
         return cudaErrorInvalidValue;
     }
-    const size_t shared = sizeof(Smem);
+    const size_t shared = sizeof(Smem) + 1024;
     static PerDevice<cudaError_t> opted_per_device;
     const cudaError_t* opted = opted_per_device.get([shared]() {
-        const cudaError_t direct =
-            cudaFuncSetAttribute(paged_attention_packed_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(shared));
-        if (direct != cudaSuccess) {
-            return direct;
+        for (const AttentionKernel kernel : attention_kernels) {
+            const cudaError_t error =
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared));
+            if (error != cudaSuccess) {
+                return error;
+            }
         }
-        return cudaFuncSetAttribute(paged_attention_packed_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(shared));
+        return cudaSuccess;
     });
     if (opted == nullptr) {
         return cudaErrorInvalidDevice;
@@ -808,49 +1223,56 @@ cudaError_t launch_attention(const void* query, const void* query_gate_projectio
     if (*opted != cudaSuccess) {
         return *opted;
     }
-    // One CTA per SM, whatever the batch: the task list is cut on the device.  A CTA's list holds
-    // kMaxCtaTasks entries; the plan gives it at most kPlanPaddingDivisor + 2 plus one per row and
-    // kv head and CTA (undivided rows: one per row and kv head and CTA).
+    // One CTA per SM at a time, whatever the batch: the task lists are cut on the device.  A list holds
+    // kMaxListTasks entries; the plan gives a chunk at most kPlanPaddingDivisor + 4 (undivided rows: one per row
+    // and kv head and CTA).
     int device = 0, sms = 0;
     if (cudaGetDevice(&device) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) {
         return cudaErrorInvalidDevice;
     }
-    if ((rows * kKvHeads + sms - 1) / sms + kPlanPaddingDivisor + 2 > kMaxCtaTasks) {
+    if ((rows * kKvHeads + sms - 1) / sms + kPlanPaddingDivisor + 4 > kMaxListTasks) {
         return cudaErrorInvalidValue;
     }
-    const dim3 grid(sms);
-    const int padded_rows = row_base + rows <= 16 ? 16 : 32;  // of the staged output
-    if (partitions == 1) {
-        return qwc::launch_chained(paged_attention_packed_kernel<false>, dim3(grid), dim3(kThreads), shared, stream, 
-            static_cast<const __nv_bfloat16*>(query), static_cast<const __nv_bfloat16*>(query_gate_projection),
-            static_cast<const uint8_t*>(key_cache), static_cast<const uint8_t*>(value_cache),
-            static_cast<const uint32_t*>(block_tables), static_cast<const uint32_t*>(context_lengths), key_scales,
-            value_scales, static_cast<__nv_bfloat16*>(output), static_cast<__half*>(staged_output), padded_rows,
-            nullptr, nullptr, rows, max_blocks, row_base, page_size, gate_stride, 1, softmax_scale, status);
+    CUtensorMap key_map, value_map;
+    cudaError_t encoded = encode_cache_map(&key_map, key_cache);
+    if (encoded == cudaSuccess) {
+        encoded = encode_cache_map(&value_map, value_cache);
     }
+    if (encoded != cudaSuccess) {
+        return encoded;
+    }
+    const int padded_rows = row_base + rows <= 16 ? 16 : 32;  // of the staged output
+    const bool split = partitions > 1;
     const size_t partials = static_cast<size_t>(rows) * kQueryHeads * partitions;
-    if (workspace == nullptr || workspace_bytes < partials * kPartialBytes) {
+    if (split && (workspace == nullptr || workspace_bytes < partials * kPartialBytes)) {
         return cudaErrorInvalidValue;
     }
     // partials is a multiple of 24, so the f16 block starts on a 16-byte boundary.
-    float* partial_stats = static_cast<float*>(workspace);
-    __half* partial_out = reinterpret_cast<__half*>(partial_stats + partials * kPartialFloats);
-    const cudaError_t launched = qwc::launch_chained(paged_attention_packed_kernel<true>, dim3(grid), dim3(kThreads), shared, stream, 
+    float* partial_stats = split ? static_cast<float*>(workspace) : nullptr;
+    __half* partial_out = split ? reinterpret_cast<__half*>(partial_stats + partials * kPartialFloats) : nullptr;
+    const long long capacity_units = static_cast<long long>(max_blocks) * (page_size / kUnitTokens);
+    const int smallest_chunk = split ? static_cast<int>((capacity_units + partitions - 2) / (partitions - 1)) : 0;
+    // What the block tables could describe bounds the line: whether its positions fit 32 bits (a large chunk per
+    // SM among them), and whether an SM's share can reach the length from which on chunks have two sizes.
+    const long long longest = (capacity_units + kPlanSlack) * rows * kKvHeads;
+    const bool wide = split && (longest >= (1ll << 31) || static_cast<long long>(smallest_chunk) * sms >= (1ll << 30));
+    const bool may_be_dynamic = split && capacity_units * rows * kKvHeads / sms >= kDynamicShare / 2;
+    const AttentionKernel kernel = attention_kernels[split ? (wide ? 2 : 1) : 0];
+    const cudaError_t launched = qwc::launch_chained(
+        kernel, dim3(may_be_dynamic ? kChunksPerSm * sms : sms), dim3(kThreads), shared, stream, key_map, value_map,
         static_cast<const __nv_bfloat16*>(query), static_cast<const __nv_bfloat16*>(query_gate_projection),
-        static_cast<const uint8_t*>(key_cache), static_cast<const uint8_t*>(value_cache),
         static_cast<const uint32_t*>(block_tables), static_cast<const uint32_t*>(context_lengths), key_scales,
-        value_scales, static_cast<__nv_bfloat16*>(output), nullptr, padded_rows, partial_stats, partial_out, rows,
-        max_blocks, row_base, page_size, gate_stride, partitions, softmax_scale, status);
-    if (launched != cudaSuccess) {
+        value_scales, split ? nullptr : static_cast<__nv_bfloat16*>(output),
+        split ? nullptr : static_cast<__half*>(staged_output), padded_rows, partial_stats, partial_out, rows, max_blocks,
+        row_base, page_size, gate_stride, partitions, smallest_chunk, sms, softmax_scale, status);
+    if (launched != cudaSuccess || !split) {
         return launched;
     }
-    const int pairs = rows * kQueryHeads;
-    return qwc::launch_chained(reduce_partitions_kernel, dim3(pairs), dim3(kMergeWarps * 32), 0, stream, 
-        partial_stats, partial_out, static_cast<const __nv_bfloat16*>(query_gate_projection),
-        static_cast<const uint32_t*>(context_lengths), static_cast<__nv_bfloat16*>(output),
-        static_cast<__half*>(staged_output), padded_rows, rows, partitions, row_base, gate_stride,
-        max_blocks * (page_size / kUnitTokens), sms);
+    return qwc::launch_chained(reduce_partitions_kernel, dim3(rows * kQueryHeads), dim3(kMergeWarps * 32), 0, stream,
+                               partial_stats, partial_out, static_cast<const __nv_bfloat16*>(query_gate_projection),
+                               static_cast<__nv_bfloat16*>(output), static_cast<__half*>(staged_output), padded_rows,
+                               partitions, row_base, gate_stride);
 }
 
 // ---- built-in scratch for callers that cannot allocate ------------------------------------

@@ -290,6 +290,87 @@ def test_packed_attention_sharp_softmax(cuda, ops):
     assert np.max(np.abs(got - want)) <= 0.006 * scale + 0.004
 
 
+@pytest.mark.parametrize("contexts,page_size,partitions", [
+    ([16, 1, 0, 127, 128, 129], 16, 2),          # stages of one unit, of a whole stage and of one unit more
+    ([30000, 33, 0, 31001, 17, 30016, 29999], 16, 40),   # 200 units per SM: large chunks and two small ones each
+    ([60000, 1, 70001, 64, 65000, 60064, 60001], 64, 200),  # 530 units: three small ones
+    ([60000, 70001, 500], 16, 2),                # the workspace has two slots per row: no chunk below a row's length
+], ids=["short", "two_small", "three_small", "two_slots"])
+def test_packed_attention_chunks(cuda, ops, contexts, page_size, partitions):
+    """Every cut of the line into chunks, with rows without context; the slots that no piece is written to hold NaN
+    before the call (rows share their pages: what is tested is the plan)."""
+    torch = cuda
+    case = synth.attention_case(16, [1024], page_size=page_size)
+    contexts = np.asarray(contexts, dtype=np.uint32)
+    blocks = (int(contexts.max()) + page_size - 1) // page_size + 1
+    rng = np.random.default_rng(16)
+    case.update(contexts=contexts, max_blocks=blocks, batch=contexts.size,
+                block_tables=rng.integers(0, case["num_blocks"], (contexts.size, blocks)).astype(np.uint32),
+                query=synth.bf16_bits(rng.standard_normal((contexts.size, 24, 256), dtype=np.float32)))
+    out = bf16_out(torch, contexts.size, 24, 256)
+    workspace = torch.full((ops.packed_workspace_bytes(contexts.size, partitions),), 0xFF, dtype=torch.uint8, device="cuda")
+    ops.gated_packed(dev(torch, case["query"]), None, dev(torch, case["key_cache"]), dev(torch, case["value_cache"]),
+                     dev(torch, case["block_tables"]), dev(torch, contexts), blocks, out, contexts.size, 0, partitions,
+                     workspace, page_size, None, None)
+    torch.cuda.synchronize()
+    got, want = synth.bf16_value(host(out)), attention_oracle(case, page_size)
+    want[contexts == 0] = 0.0  # (the oracle divides by a sum of nothing)
+    check_attention(got, want, "chunks")
+
+
+def test_packed_attention_positions_beyond_32_bits(cuda, ops):
+    """A block table that could describe 134 million tokens, with two slots per row: the plan's positions no longer
+    fit 32 bits."""
+    torch = cuda
+    case = synth.attention_case(17, [700, 3], page_size=64)
+    blocks = 1 << 21
+    tables = torch.zeros((2, blocks), dtype=torch.int32, device="cuda")
+    tables[:, :case["max_blocks"]] = dev(torch, case["block_tables"].astype(np.int32))
+    out = bf16_out(torch, 2, 24, 256)
+    workspace = torch.zeros(ops.packed_workspace_bytes(2, 2), dtype=torch.uint8, device="cuda")
+    ops.gated_packed(dev(torch, case["query"]), None, dev(torch, case["key_cache"]), dev(torch, case["value_cache"]),
+                     tables, dev(torch, case["contexts"]), blocks, out, 2, 0, 2, workspace, 64, None, None)
+    torch.cuda.synchronize()
+    check_attention(synth.bf16_value(host(out)), attention_oracle(case, 64), "wide plan")
+
+
+@pytest.mark.parametrize("kind", ["tiny", "large", "outlier", "spread"])
+def test_packed_attention_query_digits(cuda, ops, kind):
+    """Queries far from unit scale.  Three e4m3 digits below a head's largest element hold a bf16 exactly down to
+    2^-18 of it; what an element below that is off by, 2^-26 of the largest per dim, moves a score by less than
+    fp32 sums of 256 products do, so the bounds are those of every attention test."""
+    case = synth.attention_case(18, [300, 41], page_size=16, with_gate=True)
+    query = synth.bf16_value(case["query"]).astype(np.float32)
+    rng = np.random.default_rng(18)
+    if kind == "tiny":
+        query *= np.float32(2.0 ** -12)
+    elif kind == "large":  # the scores stay moderate: four dims of each head
+        query *= (rng.random(query.shape) < 4 / 256) * np.float32(8.0)
+    elif kind == "outlier":  # one dim 4096 times the others, on keys that are zero there
+        query[:, :, 7] = 4096.0
+        keys = synth.e4m3_decode(case["key_cache"])
+        keys[..., 7] = 0.0
+        case["key_cache"] = synth.e4m3_encode(keys)
+    else:
+        query *= np.exp2(-rng.integers(0, 24, query.shape)).astype(np.float32)
+    case["query"] = synth.bf16_bits(query)
+    for partitions in (1, 3):
+        check_attention(run_attention(cuda, ops, case, 16, partitions), attention_oracle(case, 16), kind)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_packed_attention_non_finite_query_stays_in_its_head(cuda, ops, value):
+    case = synth.attention_case(19, [300, 41], page_size=16)
+    clean = run_attention(cuda, ops, case, 16, 3)
+    query = synth.bf16_value(case["query"]).astype(np.float32)
+    query[0, 8, 100] = value
+    got = run_attention(cuda, ops, dict(case, query=synth.bf16_bits(query)), 16, 3)
+    same = np.ones((2, 24), dtype=bool)
+    same[0, 8] = False
+    assert np.array_equal(got[same], clean[same])
+    assert not np.array_equal(got[0, 8], clean[0, 8])
+
+
 def test_packed_attention_legacy_entry_uses_configured_page_size(cuda, ops):
     from qwencore_b200 import abi
 
