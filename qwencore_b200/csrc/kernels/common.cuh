@@ -95,6 +95,33 @@ inline bool runs_in_four_bits(int out_features, int in_features, int batch, bool
 int native_splits(int out_features, int in_features, bool swiglu);          // nvfp4_native.cuh
 int umma_splits(int out_features, int in_features, bool swiglu, bool fp8);  // nvfp4_umma.cu
 
+// Share of a CTA when `units` are cut into `parts` (at most 8): part i begins at units * i / parts.  The quotients are
+// the host's; on the device a division would stand in front of a CTA's first load.
+struct EvenCut {
+    int parts;
+    uint32_t inverse;  // ceil(2^32 / parts)
+    int quotient;      // units / parts ...
+    int rest;          // ... and what is left
+};
+
+inline EvenCut even_cut(int units, int parts) {
+    EvenCut cut;
+    cut.parts = parts;
+    cut.inverse = static_cast<uint32_t>(((1ull << 32) + parts - 1) / parts);
+    cut.quotient = units / parts;
+    cut.rest = units % parts;
+    return cut;
+}
+
+// n / parts for n < 65536 (the rounding error of the inverse stays below 1 / parts).
+__device__ __forceinline__ int cut_quotient(const EvenCut& cut, int n) {
+    return cut.parts == 1 ? n : static_cast<int>(__umulhi(static_cast<uint32_t>(n), cut.inverse));
+}
+
+__device__ __forceinline__ int cut_begin(const EvenCut& cut, int part) {
+    return cut.quotient * part + cut_quotient(cut, cut.rest * part);
+}
+
 // Process-wide shape selection (see qwc_configure in the C ABI).
 struct Shape {
     int delta_value_heads;

@@ -227,11 +227,10 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int cta = blockIdx.x;
-    const int S = p.stages_in_k;
-    const int pair = cta / p.splits;
+    const int pair = cut_quotient(p.cut, cta);
     const int slice = cta - pair * p.splits;
-    const int first_stage = S * slice / p.splits;
-    const int num_stages = S * (slice + 1) / p.splits - first_stage;
+    const int first_stage = cut_begin(p.cut, slice);
+    const int num_stages = cut_begin(p.cut, slice + 1) - first_stage;
     const int group_blocks = p.in_features / 64;
     // activation rows padded to 2, 4 or 8
     const int rows_shift = p.batch <= 2 ? 1 : p.batch <= 4 ? 2 : 3;
@@ -269,7 +268,10 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
             }
         }
     };
-    const int early_stages = min(num_stages, kWeightStages);
+    // One stage before the CTA's barrier and the others after it, and nothing else in front of it that takes time
+    // (nvfp4_streamk.cu): 34816 x 5120 at one row 18.3 -> 18.1 us, 5120 x 4096 6.29 -> 6.17.  The f16 kernel for
+    // bf16 rows (nvfp4_umma.cu) gained nothing from it: 34816 x 5120 at 16 rows 21.3 / 21.3, pair at 32 rows 25.8 / 25.9.
+    constexpr int early_stages = 1;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kWeightStages; ++s) {
             mbar_init(&bars.w_full[s], 1);
@@ -277,11 +279,16 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
             mbar_init(&bars.w_empty[s], 1);
         }
         mbar_fence_init();
-        for (int index = 0; index < early_stages; ++index) {
-            issue_stage(index);
-        }
+        issue_stage(0);
     }
-    if (threadIdx.x == 32) {
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars.tmem_base)),
+                     "r"(kTmemColumns)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+    if (threadIdx.x == 64) {
         for (int s = 0; s < kNativeMaxXSlots; ++s) {
             mbar_init(&bars.x_full[s], team);
             mbar_init(&bars.x_empty[s], 1);
@@ -289,12 +296,16 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
         }
         bars.rest_used = 0;
         mbar_init(&bars.done, 1);
-        bars.failed = status_is_set(p.status) ? 1 : 0;
-        bars.tmem_base = 0;
+        bars.failed = 0;
         mbar_fence_init();
     }
     __syncthreads();
-    uint32_t tmem_base = 0;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars.tmem_base);
+    // (by a thread that has time: whoever has to wait from here on looks at the flag)
+    if (threadIdx.x == 64 && status_is_set(p.status)) {
+        *reinterpret_cast<volatile int*>(&bars.failed) = 1;
+    }
     int issued = early_stages;  // the producer's thread: stages asked for
 
     if (warp == 0) {
@@ -317,14 +328,6 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
         }
     } else if (warp == 1) {
         // ---------------- tensor memory, scales, MMA ----------------
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars.tmem_base)),
-                     "r"(kTmemColumns)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars.tmem_base);
         // A and B e2m1 (1), scales e4m3, fp32 accumulators, M = 128
         const uint32_t idesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(N >> 3) << 17) | (8u << 24);
         const uint32_t weight_base = smem_u32(weight_ring);
@@ -549,7 +552,6 @@ __global__ void __launch_bounds__(kNativeThreads, 1)
              __all_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&bars.failed) == 0);
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars.tmem_base);
             const int quarter = e & 3;
             const int first_token = (e >> 2) * (R / 2);
             const uint32_t address = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + first_token;

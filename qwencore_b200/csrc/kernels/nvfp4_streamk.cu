@@ -119,9 +119,7 @@ struct StreamKParams {
     // slice (a CTA per tile pair: matrices with about as many pairs as SMs) the CTA finishes its pair
     // itself.  0 splits: equal shares with tickets.
     int splits;
-    uint32_t split_inverse;  // ceil(2^32 / splits): quotients of small numbers without a division
-    int slice_stages;        // stages_in_k / splits ...
-    int slice_rest;          // ... and what is left
+    EvenCut cut;  // of the K stages into `splits` slices
     float* split_out;
     // Latency mode (one activation row, weight rows split over ranks): the slices go to every rank's
     // exchange block as tagged words instead (exchange.cuh); split_out is null then.
@@ -233,16 +231,6 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 // First unit of CTA `cta` when `units` units are shared by `ctas` CTAs.
 __device__ __forceinline__ int share_begin(int units, int cta, int ctas) {
     return static_cast<int>(static_cast<long long>(units) * cta / ctas);
-}
-
-// n / splits for n < 65536 (splits <= 8; the rounding error of the inverse stays below 1 / splits).
-__device__ __forceinline__ int split_quotient(const StreamKParams& p, int n) {
-    return p.splits == 1 ? n : static_cast<int>(__umulhi(static_cast<uint32_t>(n), p.split_inverse));
-}
-
-// stages_in_k * slice / splits
-__device__ __forceinline__ int slice_begin(const StreamKParams& p, int slice) {
-    return p.slice_stages * slice + split_quotient(p, p.slice_rest * slice);
 }
 
 // The CTA whose share holds unit `unit` (ctas <= units, so no share is empty).
@@ -399,10 +387,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     int u_begin, u_end, pair_first;
     if (kSplitOut) {
         // (no divisions: every CTA of a launch stands at this point before its first weight is asked for)
-        pair_first = split_quotient(p, cta);
+        pair_first = cut_quotient(p.cut, cta);
         const int slice = cta - pair_first * p.splits;
-        u_begin = pair_first * S + slice_begin(p, slice);
-        u_end = pair_first * S + slice_begin(p, slice + 1);
+        u_begin = pair_first * S + cut_begin(p.cut, slice);
+        u_end = pair_first * S + cut_begin(p.cut, slice + 1);
     } else {
         u_begin = share_begin(p.units, cta, ctas);
         u_end = share_begin(p.units, cta + 1, ctas);
@@ -1457,9 +1445,7 @@ cudaError_t launch_streamk(StreamKParams p, const void* packed0, const void* pac
     p.units = shape.units;
     p.splits = shape.splits;
     if (shape.splits > 0) {
-        p.split_inverse = static_cast<uint32_t>(((1ull << 32) + shape.splits - 1) / shape.splits);
-        p.slice_stages = shape.stages_in_k / shape.splits;
-        p.slice_rest = shape.stages_in_k % shape.splits;
+        p.cut = even_cut(shape.stages_in_k, shape.splits);
     }
     unsigned char* base = static_cast<unsigned char*>(workspace);
     p.partials = reinterpret_cast<float*>(base);
@@ -1611,6 +1597,7 @@ cudaError_t launch_nvfp4_native(const void* packed0, const void* scales0, const 
     p.stages_in_k = in_features / (kChunkK * kStageChunks);
     p.units = p.pair_tiles * p.stages_in_k;
     p.splits = native_splits(out_features, in_features, swiglu);
+    p.cut = even_cut(p.stages_in_k, p.splits);
     CUtensorMap map0, map1;
     cudaError_t encoded = encode_weight_map(&map0, packed0, out_features, in_features / 2);
     if (encoded == cudaSuccess) {
