@@ -168,6 +168,17 @@ int qwc_delta_prepare_decode_split(const float* partial_sums, int slices, int wi
 int qwc_delta_gated_rmsnorm_split(const float* input, const float* partial_sums, int slices, int width,
                                   float weight_global_scale, int gate_column, const void* weight, void* output,
                                   void* staged_output, int batch, float epsilon, qwc_stream stream);
+/* As qwc_prepare_attention_decode_fp8_scaled on the rows [q | gate per head][k][v] of `width` outputs whose K
+ * slices (qwc_nvfp4_w4a16_split) are summed here.  The gates go as bf16 to their places in `gate_rows`
+ * [batch][width] (what qwc_paged_attention_packed_fp8_staged reads with gate_stride = width); the rest of those
+ * rows is left alone.  The norm weights must not be written by the kernels just before this one. */
+int qwc_prepare_attention_decode_fp8_split(const float* partial_sums, int slices, float weight_global_scale,
+                                           const void* query_norm_weight, const void* key_norm_weight,
+                                           const void* cosine, const void* sine, const void* physical_blocks,
+                                           const void* block_offsets, const float* key_scales,
+                                           const float* value_scales, void* query, void* key_cache, void* value_cache,
+                                           void* gate_rows, int batch, int page_size, int width, float epsilon,
+                                           qwc_stream stream);
 int qwc_nvfp4_sum_slices(const float* partial_sums, int slices, float weight_global_scale, void* rows, int batch,
                          int width, qwc_stream stream);
 /* The recurrent update in the step's own form: as qwc_delta_decode_int8, but the state slots and the

@@ -102,6 +102,8 @@ KERNEL_SYMBOLS = {
     "qwc_delta_prepare_decode": (c_int, [P] * 14 + [c_int, c_int, c_int, c_int, P]),
     "qwc_delta_gated_rmsnorm": (c_int, [P, P, P, P, c_int, c_float, c_int, P]),
     "qwc_prepare_attention_decode_fp8": (c_int, [P] * 12 + [c_int, c_float, P]),
+    "qwc_prepare_attention_decode_fp8_split": (c_int, [P, c_int, c_float] + [P] * 12 +
+                                               [c_int, c_int, c_int, c_float, P]),
     "qwc_prepare_attention_decode_fp8_scaled": (c_int, [P] * 14 + [c_int, c_int, c_int, c_int, c_int, c_float,
                                                                    P]),
     "qwc_rmsnorm_bf16": (c_int, [P, P, P, P, c_int, c_int, c_float, P]),

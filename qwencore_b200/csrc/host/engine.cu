@@ -684,14 +684,17 @@ int decode_forward(qwc_engine* e, int batch) {
             if (staged && phase(e, "gemm.attn_qkv")) {
                 QWC_TRY(qwc_nvfp4_w4a16_split(layer.qkv.packed, layer.qkv.scales, e->normed_staged, e->split_sums_wide,
                                               layer.qkv.out_features, layer.qkv.in_features, batch, s));
-                QWC_TRY(qwc_nvfp4_sum_slices(e->split_sums_wide,
-                                             qwc_nvfp4_split_count(layer.qkv.out_features, layer.qkv.in_features),
-                                             layer.qkv.global_scale, e->qkv_buf, batch, e->qkv_width, s));
             } else if (phase(e, "gemm.attn_qkv")) {
                 QWC_TRY(project(e, layer.qkv, e->normed, e->qkv_buf, batch));
             }
             const int q_width = kQueryHeads * 2 * kHeadDim;
-            if (phase(e, "attn.prepare")) {
+            if (staged && phase(e, "attn.prepare")) {
+                QWC_TRY(qwc_prepare_attention_decode_fp8_split(
+                    e->split_sums_wide, qwc_nvfp4_split_count(layer.qkv.out_features, layer.qkv.in_features),
+                    layer.qkv.global_scale, layer.q_norm, layer.k_norm, e->cosine, e->sine, e->physical_blocks,
+                    e->block_offsets, layer.k_scale, layer.v_scale, e->query, layer.k_cache, layer.v_cache, e->qkv_buf,
+                    batch, c.kv_page_size, e->qkv_width, kEps, s));
+            } else if (phase(e, "attn.prepare")) {
                 QWC_TRY(qwc_prepare_attention_decode_fp8_scaled(
                     e->qkv_buf, e->qkv_buf + q_width, e->qkv_buf + q_width + kKvHeads * kHeadDim, layer.q_norm,
                     layer.k_norm, e->cosine, e->sine, e->physical_blocks, e->block_offsets, layer.k_scale, layer.v_scale,
@@ -1419,7 +1422,7 @@ void qwc_engine_traffic(const qwc_engine* e, int rows, double context_tokens, qw
         } else {
             gemv_bytes += static_cast<double>(l.qkv.weight_bytes() + l.o.weight_bytes());
             gemv += 2;
-            kernels += 2 + 2 + (e->partitions > 1 ? 1 : 0) + (e->cfg.split_size == 1 ? 1 : 0 /*slice sum*/);
+            kernels += 2 + 2 + (e->partitions > 1 ? 1 : 0);
             out->kv_bytes += context_tokens * 2.0 * kKvHeads * kHeadDim;
         }
     }

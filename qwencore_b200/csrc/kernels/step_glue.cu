@@ -914,6 +914,13 @@ __global__ void __launch_bounds__(kDeltaHeadDim) gated_rmsnorm_kernel(const floa
 
 // ---- QK-norm + partial RoPE + FP8 page write (cuda/attention_prepare.cu:52-143) -----
 // One launch: blockIdx.x < 24 are query heads, the next 4 are KV heads.
+//
+// `kSums`: the fused q | gate | k | v projection ran as a K split, and this kernel finishes it: the slices of the
+// columns that a CTA works on are summed in slice order, scaled and rounded to bf16 as qwc_nvfp4_sum_slices would
+// have done, and a query head's CTA also stores its gate columns as bf16 rows for the attention merge.  The norm
+// weights are never written during a step: fetched before the wait.  (One launch less per attention layer: the
+// one-row step 4268 -> 4249 us.)
+template <bool kSums>
 __global__ void __launch_bounds__(kHeadDim) prepare_attention_kernel(
     const __nv_bfloat16* __restrict__ query_gate_projection, const __nv_bfloat16* __restrict__ key_projection,
     const __nv_bfloat16* __restrict__ value_projection, const __nv_bfloat16* __restrict__ query_norm_weight,
@@ -922,9 +929,11 @@ __global__ void __launch_bounds__(kHeadDim) prepare_attention_kernel(
     const uint32_t* __restrict__ block_offsets, const float* __restrict__ key_scales,
     const float* __restrict__ value_scales, __nv_bfloat16* __restrict__ query, uint8_t* __restrict__ key_cache,
     uint8_t* __restrict__ value_cache, int page_size, int query_stride, int key_stride, int value_stride,
-    float epsilon) {
+    float epsilon, const SplitSource split, __nv_bfloat16* __restrict__ gate_rows) {
     pdl_launch_dependents();
-    pdl_wait();
+    if (!kSums) {
+        pdl_wait();
+    }
     __shared__ float scratch[kHeadDim / 32];
     __shared__ __nv_bfloat16 normalized[kHeadDim];
     const int batch = blockIdx.y;
@@ -935,10 +944,42 @@ __global__ void __launch_bounds__(kHeadDim) prepare_attention_kernel(
         is_query ? query_gate_projection + static_cast<size_t>(batch) * query_stride + head * (2 * kHeadDim)
                  : key_projection + static_cast<size_t>(batch) * key_stride + head * kHeadDim;
     const __nv_bfloat16* norm_weight = is_query ? query_norm_weight : key_norm_weight;
-    const float raw = __bfloat162float(raw_row[dimension]);
+    const float gain = __bfloat162float(norm_weight[dimension]);
+    float raw, other = 0.0f;  // other: the gate of a query head, the value of a KV head
+    if (kSums) {
+        pdl_wait();
+        constexpr int kQueryWidth = kQueryHeads * 2 * kHeadDim;
+        const int column = is_query ? head * (2 * kHeadDim) + dimension : kQueryWidth + head * kHeadDim + dimension;
+        const int other_column = column + (is_query ? kHeadDim : kKvHeads * kHeadDim);
+        const size_t slice_stride = static_cast<size_t>(split.batch) * split.width;
+        const float* row = split.sums + static_cast<size_t>(batch) * split.width;
+        float sums[2] = {0.0f, 0.0f};
+        for (int first = 0; first < split.slices; first += 4) {
+            float part[2][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float* at = row + min(first + j, split.slices - 1) * slice_stride;
+                part[0][j] = __ldcg(at + column);
+                part[1][j] = __ldcg(at + other_column);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                sums[0] += first + j < split.slices ? part[0][j] : 0.0f;
+                sums[1] += first + j < split.slices ? part[1][j] : 0.0f;
+            }
+        }
+        raw = __bfloat162float(__float2bfloat16(sums[0] * split.scale));
+        const __nv_bfloat16 rounded = __float2bfloat16(sums[1] * split.scale);
+        other = __bfloat162float(rounded);
+        if (is_query) {
+            gate_rows[static_cast<size_t>(batch) * query_stride + other_column] = rounded;
+        }
+    } else {
+        raw = __bfloat162float(raw_row[dimension]);
+    }
     const float sum = block_sum(raw * raw, scratch);
     const float inverse = rsqrtf(sum / static_cast<float>(kHeadDim) + epsilon);
-    normalized[dimension] = __float2bfloat16(raw * inverse * (1.0f + __bfloat162float(norm_weight[dimension])));
+    normalized[dimension] = __float2bfloat16(raw * inverse * (1.0f + gain));
     __syncthreads();
     float rotated_value = __bfloat162float(normalized[dimension]);
     if (dimension < kRopeDim) {
@@ -959,8 +1000,9 @@ __global__ void __launch_bounds__(kHeadDim) prepare_attention_kernel(
         kHeadDim;
     const float k_inverse = key_scales ? 1.0f / key_scales[head] : 1.0f;
     const float v_inverse = value_scales ? 1.0f / value_scales[head] : 1.0f;
-    const float v = __bfloat162float(
-        value_projection[static_cast<size_t>(batch) * value_stride + head * kHeadDim + dimension]);
+    const float v = kSums ? other
+                          : __bfloat162float(
+                                value_projection[static_cast<size_t>(batch) * value_stride + head * kHeadDim + dimension]);
     key_cache[cache_base + dimension] = to_fp8(rotated_value * k_inverse);
     value_cache[cache_base + dimension] = to_fp8(v * v_inverse);
 }
@@ -1384,14 +1426,43 @@ extern "C" int qwc_prepare_attention_decode_fp8_scaled(
         return cudaErrorInvalidValue;
     }
     const dim3 grid(kQueryHeads + kKvHeads, batch);
-    return qwc::launch_chained(prepare_attention_kernel, dim3(grid), dim3(kHeadDim), 0, stream, 
+    return qwc::launch_chained(prepare_attention_kernel<false>, dim3(grid), dim3(kHeadDim), 0, stream,
         static_cast<const __nv_bfloat16*>(query_gate_projection), static_cast<const __nv_bfloat16*>(key_projection),
         static_cast<const __nv_bfloat16*>(value_projection), static_cast<const __nv_bfloat16*>(query_norm_weight),
         static_cast<const __nv_bfloat16*>(key_norm_weight), static_cast<const __nv_bfloat16*>(cosine),
         static_cast<const __nv_bfloat16*>(sine), static_cast<const uint32_t*>(physical_blocks),
         static_cast<const uint32_t*>(block_offsets), key_scales, value_scales, static_cast<__nv_bfloat16*>(query),
         static_cast<uint8_t*>(key_cache), static_cast<uint8_t*>(value_cache), page_size, query_stride, key_stride,
-        value_stride, epsilon);
+        value_stride, epsilon, SplitSource{}, nullptr);
+}
+
+extern "C" int qwc_prepare_attention_decode_fp8_split(
+    const float* partial_sums, int slices, float weight_global_scale, const void* query_norm_weight,
+    const void* key_norm_weight, const void* cosine, const void* sine, const void* physical_blocks,
+    const void* block_offsets, const float* key_scales, const float* value_scales, void* query, void* key_cache,
+    void* value_cache, void* gate_rows, int batch, int page_size, int width, float epsilon, cudaStream_t stream) {
+    if (partial_sums == nullptr || slices <= 0 || slices > 64 || !(weight_global_scale > 0.0f) ||
+        query_norm_weight == nullptr || key_norm_weight == nullptr || cosine == nullptr || sine == nullptr ||
+        physical_blocks == nullptr || block_offsets == nullptr || query == nullptr || key_cache == nullptr ||
+        value_cache == nullptr || gate_rows == nullptr || batch <= 0 || batch > 32 || !isfinite(epsilon) ||
+        epsilon <= 0.0f || (page_size != 16 && page_size != 64) ||
+        width < kQueryHeads * 2 * kHeadDim + 2 * kKvHeads * kHeadDim) {
+        return cudaErrorInvalidValue;
+    }
+    SplitSource split = {};
+    split.sums = partial_sums;
+    split.slices = slices;
+    split.batch = batch;
+    split.width = width;
+    split.scale = 1.0f / weight_global_scale;
+    return qwc::launch_chained(prepare_attention_kernel<true>, dim3(kQueryHeads + kKvHeads, batch), dim3(kHeadDim), 0,
+                               stream, nullptr, nullptr, nullptr, static_cast<const __nv_bfloat16*>(query_norm_weight),
+                               static_cast<const __nv_bfloat16*>(key_norm_weight),
+                               static_cast<const __nv_bfloat16*>(cosine), static_cast<const __nv_bfloat16*>(sine),
+                               static_cast<const uint32_t*>(physical_blocks), static_cast<const uint32_t*>(block_offsets),
+                               key_scales, value_scales, static_cast<__nv_bfloat16*>(query),
+                               static_cast<uint8_t*>(key_cache), static_cast<uint8_t*>(value_cache), page_size, width,
+                               width, width, epsilon, split, static_cast<__nv_bfloat16*>(gate_rows));
 }
 
 extern "C" int qwc_prepare_attention_decode_fp8(const void* query_gate_projection, const void* key_projection,

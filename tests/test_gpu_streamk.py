@@ -441,3 +441,87 @@ def test_delta_step_form_with_fused_gated_norm_is_the_two_kernels_bit_for_bit(cu
             stream) == abi.CUDA_ERROR_INVALID_VALUE
     finally:
         abi.configure(*before)
+
+
+@pytest.mark.parametrize("batch,slices", [(1, 1), (5, 4), (32, 5), (3, 8)])
+@pytest.mark.parametrize("v_heads,page_size", [(32, 16), (48, 64)])
+def test_prepare_steps_sum_any_number_of_slices(cuda, ops, batch, slices, v_heads, page_size):
+    """The DeltaNet and the attention prepare step on K slices give the bits they give on the rows that the plain
+    sum makes of those slices."""
+    from qwencore_b200 import abi
+
+    torch = cuda
+    before = abi.get_shape()
+    abi.configure(v_heads, page_size)
+    rng = np.random.default_rng(21)
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def summed(width):
+        sums = dev(torch, rng.standard_normal((slices, batch, width), dtype=np.float32))
+        rows = bf16_out(torch, batch, width)
+        abi.check(abi.lib.qwc_nvfp4_sum_slices(sums.data_ptr(), slices, 2.0, rows.data_ptr(), batch, width, stream),
+                  "qwc_nvfp4_sum_slices")
+        return sums, rows
+
+    try:
+        # DeltaNet: q | k | v | z | a | b
+        channels = 2 * 16 * 128 + v_heads * 128
+        a_offset = channels + v_heads * 128
+        width = a_offset + 2 * v_heads
+        sums, rows = summed(width)
+        capacity = batch + 1
+        slots = dev(torch, rng.permutation(capacity)[:batch].astype(np.uint32))
+        conv_weight = dev(torch, synth.normal_bf16(21, "conv", (channels * 4,), std=0.3))
+        a_log, dt_bias = (dev(torch, synth.normal_bf16(21, name, (v_heads,), std=0.5)) for name in ("alog", "dt"))
+        conv_init = rng.uniform(-1, 1, (capacity, channels, 3)).astype(np.float32)
+        results = []
+        for split in (False, True):
+            conv_state = dev(torch, conv_init)
+            outs = [torch.zeros(n, dtype=torch.float32, device="cuda")
+                    for n in (batch * 2048, batch * 2048, batch * v_heads * 128, batch * v_heads, batch * v_heads,
+                              batch * 16)]
+            if split:
+                abi.check(abi.lib.qwc_delta_prepare_decode_split(
+                    sums.data_ptr(), slices, width, 2.0, a_offset, a_offset + v_heads, conv_weight.data_ptr(),
+                    a_log.data_ptr(), dt_bias.data_ptr(), conv_state.data_ptr(), slots.data_ptr(),
+                    *[o.data_ptr() for o in outs], capacity, batch, stream), "qwc_delta_prepare_decode_split")
+            else:
+                ops.delta_prepare_decode(rows, a_offset, a_offset + v_heads, conv_weight, a_log, dt_bias, conv_state,
+                                         slots, *outs, capacity, batch, width)
+            torch.cuda.synchronize()
+            results.append([host(conv_state)] + [host(o) for o in outs])
+        for on_rows, on_slices in zip(*results):
+            assert np.array_equal(on_rows.view(np.uint8), on_slices.view(np.uint8))
+
+        # attention: (q | gate) per head, k, v
+        q_width, k_width = 24 * 512, 4 * 256
+        width = q_width + 2 * k_width
+        sums, rows = summed(width)
+        q_norm, k_norm = (dev(torch, synth.normal_bf16(21, name, (256,), std=0.05)) for name in ("qn", "kn"))
+        cosine, sine = (dev(torch, synth.normal_bf16(21, name, (batch, 64))) for name in ("cos", "sin"))
+        blocks = dev(torch, rng.permutation(batch + 1)[:batch].astype(np.uint32))
+        offsets = dev(torch, rng.integers(0, page_size, batch).astype(np.uint32))
+        scales = [dev(torch, (0.5 + rng.random(4)).astype(np.float32)) for _ in range(2)]
+        results = []
+        for split in (False, True):
+            query = bf16_out(torch, batch, 24, 256)
+            caches = [torch.zeros((batch + 1, 4, page_size, 256), dtype=torch.uint8, device="cuda") for _ in range(2)]
+            gates = bf16_out(torch, batch, width)
+            at = query.data_ptr(), caches[0].data_ptr(), caches[1].data_ptr()
+            common = [t.data_ptr() for t in (q_norm, k_norm, cosine, sine, blocks, offsets, scales[0], scales[1])]
+            if split:
+                abi.check(abi.lib.qwc_prepare_attention_decode_fp8_split(
+                    sums.data_ptr(), slices, 2.0, *common, *at, gates.data_ptr(), batch, page_size, width, 1e-6,
+                    stream), "qwc_prepare_attention_decode_fp8_split")
+            else:
+                abi.check(abi.lib.qwc_prepare_attention_decode_fp8_scaled(
+                    rows.data_ptr(), rows.data_ptr() + 2 * q_width, rows.data_ptr() + 2 * (q_width + k_width), *common,
+                    *at, batch, page_size, width, width, width, 1e-6, stream), "qwc_prepare_attention_decode_fp8_scaled")
+                gates = rows
+            torch.cuda.synchronize()
+            gate = host(gates)[:, :q_width].reshape(batch, 24, 2, 256)[:, :, 1]
+            results.append([host(query), host(caches[0]), host(caches[1]), np.ascontiguousarray(gate)])
+        for on_rows, on_slices in zip(*results):
+            assert np.array_equal(on_rows, on_slices)
+    finally:
+        abi.configure(*before)
