@@ -1015,6 +1015,7 @@ __global__ void __launch_bounds__(kHeadDim) prepare_attention_kernel(
 // integer maximum; the eight CTA winners meet in the first CTA's shared memory (one cluster barrier).
 // The caller's partial arrays of the two-launch form are not needed.
 constexpr int kArgmaxCtas = 8;
+constexpr int kArgmaxDepth = 10;
 
 __device__ __forceinline__ unsigned long long argmax_key(float value, uint32_t index) {
     const uint32_t raw = __float_as_uint(value);
@@ -1037,24 +1038,59 @@ __global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(kThreads)
     const int span = ((vocab + kArgmaxCtas - 1) / kArgmaxCtas + 3) & ~3;
     const int begin = rank * span;
     const int end = min(vocab, begin + span);
-    unsigned long long best = 0ull;
+    // A thread's columns ascend, so a later equal value never replaces an earlier one and the key is made once, at
+    // the end.  The loads of a batch are in flight together: with one at a time a thread's nineteen (151 936
+    // logits) were as many L2 round trips (head and argmax of five rows as a user
+    // calls them 154.9 -> 150.2 us).
+    float best_value = -INFINITY;
+    uint32_t best_column = UINT32_MAX;  // none yet
+    const auto consider = [&](float value, int column) {
+        if (value > best_value || (value == best_value && best_column == UINT32_MAX)) {
+            best_value = value;
+            best_column = static_cast<uint32_t>(column);
+        }
+    };
     if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
-        for (int column = begin + 4 * threadIdx.x; column < end; column += 4 * kThreads) {
-            if (column + 4 <= end) {
-                const float4 v = __ldcs(reinterpret_cast<const float4*>(row + column));
-                best = max(best, max(max(argmax_key(v.x, column), argmax_key(v.y, column + 1)),
-                                     max(argmax_key(v.z, column + 2), argmax_key(v.w, column + 3))));
-            } else {
-                for (int c = column; c < end; ++c) {
-                    best = max(best, argmax_key(row[c], c));
-                }
+#pragma unroll 1
+        for (int first = begin + 4 * threadIdx.x; first < end; first += 4 * kThreads * kArgmaxDepth) {
+            float4 v[kArgmaxDepth];
+#pragma unroll
+            for (int j = 0; j < kArgmaxDepth; ++j) {
+                const int column = first + 4 * kThreads * j;
+                // (what is not there, or not there as a whole, never wins)
+                v[j] = column + 4 <= end ? __ldcs(reinterpret_cast<const float4*>(row + column))
+                                         : make_float4(NAN, NAN, NAN, NAN);
+            }
+#pragma unroll
+            for (int j = 0; j < kArgmaxDepth; ++j) {
+                const int column = first + 4 * kThreads * j;
+                consider(v[j].x, column);
+                consider(v[j].y, column + 1);
+                consider(v[j].z, column + 2);
+                consider(v[j].w, column + 3);
+            }
+        }
+        const int whole = begin + (max(end - begin, 0) & ~3);
+        if (threadIdx.x == 0) {  // the last one to three of a row (its columns are behind all of this thread's)
+            for (int column = whole; column < end; ++column) {
+                consider(row[column], column);
             }
         }
     } else {
-        for (int column = begin + threadIdx.x; column < end; column += kThreads) {
-            best = max(best, argmax_key(row[column], column));
+#pragma unroll 1
+        for (int first = begin + threadIdx.x; first < end; first += kThreads * kArgmaxDepth) {
+            float v[kArgmaxDepth];
+#pragma unroll
+            for (int j = 0; j < kArgmaxDepth; ++j) {
+                v[j] = first + kThreads * j < end ? __ldcs(row + first + kThreads * j) : NAN;
+            }
+#pragma unroll
+            for (int j = 0; j < kArgmaxDepth; ++j) {
+                consider(v[j], first + kThreads * j);
+            }
         }
     }
+    unsigned long long best = best_column == UINT32_MAX ? 0ull : argmax_key(best_value, best_column);
 #pragma unroll
     for (int offset = 16; offset > 0; offset >>= 1) {
         best = max(best, __shfl_xor_sync(0xffffffffu, best, offset));

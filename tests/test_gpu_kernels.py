@@ -695,6 +695,27 @@ def test_argmax_ties_go_to_lower_index(cuda, ops):
     assert host(tokens).tolist() == [77, vocab - 1, 0, 0xFFFFFFFF, 0, 70000, 4]
 
 
+@pytest.mark.parametrize("vocab", [1, 3, 37, 10240, 10243, 81921, 151938])
+def test_argmax_any_width_and_alignment(cuda, ops, vocab):
+    """Widths that fill a thread's batch of loads partly, wholly and more than once, rows on and off 16-byte
+    boundaries, with many ties and NaNs."""
+    torch = cuda
+    rng = np.random.default_rng(vocab)
+    logits = rng.integers(-3, 4, (5, vocab)).astype(np.float32)
+    logits[rng.random((5, vocab)) < 0.2] = np.nan
+    logits[3] = np.where(rng.random(vocab) < 0.5, -np.inf, np.nan)
+    logits[4] = rng.permutation(vocab)
+    want = []
+    for row in logits:
+        there = np.flatnonzero(~np.isnan(row))
+        want.append(int(there[np.argmax(row[there])]) if there.size else 0xFFFFFFFF)
+    tokens = u32_out(torch, 5)
+    ops.argmax(dev(torch, logits), torch.zeros(5 * 256, dtype=torch.float32, device="cuda"), u32_out(torch, 5 * 256),
+               tokens, vocab, 5, 256)
+    torch.cuda.synchronize()
+    assert host(tokens).tolist() == want
+
+
 @pytest.mark.parametrize("v_heads", [32, 48], ids=["h32_oracle_generalisation", "h48_reference_shape"])
 def test_delta_prepare_and_gated_rmsnorm(cuda, ops, v_heads):
     """crates/qwc-cuda/tests/delta_net.rs:576-716 (CPU conv/gate check) and :716-777."""
