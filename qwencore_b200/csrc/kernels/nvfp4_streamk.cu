@@ -863,52 +863,29 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             __syncwarp();
         };
-        // A slice of a regular K split: fp32 rows [slice][batch][N] for the consumer to sum, this lane's two
-        // rows (batch == 0: the rehearsal, as above).
+        // A slice of a regular K split in latency mode, this lane's two rows (batch == 0: the rehearsal, as above;
+        // slices for a consumer on this GPU go the way of store_direct).  One activation row, the first column of
+        // the warps that hold the first rows: this rank's columns of the row go to every rank's copy of the slice
+        // array, its own included, as tagged words (exchange.cuh).
         auto store_slice = [&](int pair, int batch) {
             const bool rehearsal = batch == 0;
-            const int slice = kSplitOut ? cta - pair * p.splits : 0;
-            if (p.exchange.ranks > 0) {
-                // Latency mode, one activation row (the first column of the warps that hold the first
-                // rows): this rank's columns of the row go to every rank's copy of the slice array, its
-                // own included, as tagged words (exchange.cuh).
-                if (first_token != 0) {
-                    return;
-                }
-                const uint32_t tag = rehearsal ? 0u : exchange_tag(p.exchange.epoch, p.exchange.instance);
-                uint2* const sink = reinterpret_cast<uint2*>(g_rehearsal_sink + (cta * kEpilogueWarps + e) * 32);
-#pragma unroll
-                for (int t = 0; t < kTiles; ++t) {
-                    const int row = kSwiglu ? pair * kTileRows + quarter * 32 + lane
-                                            : (pair * kTiles + t) * kTileRows + quarter * 32 + lane;
-                    if (row < p.out_features) {
-                        // SwiGLU pair: the row is [gate | up], each half holding all ranks' columns
-                        const size_t element = static_cast<size_t>(slice) * p.exchange.width +
-                                               (kSwiglu ? t * (p.exchange.width / 2) : 0) + p.exchange.first_column +
-                                               row;
-                        const float value = stash[(t * kCols) * kStashPitch];
-                        for (int r = 0; r < p.exchange.ranks; ++r) {
-                            store_tagged(rehearsal ? sink + (lane >> 1) : p.exchange.copies[r] + element, value, tag);
-                        }
-                    }
-                }
+            if (first_token != 0) {
                 return;
             }
-            const int rows_stored = rehearsal ? kPad : batch;
-            float* const out = rehearsal ? g_rehearsal_sink + (cta * kEpilogueWarps + e) * 32
-                                         : p.split_out + static_cast<size_t>(slice) * p.batch * p.out_features;
-            const size_t row_pitch = rehearsal ? 0 : static_cast<size_t>(p.out_features);
+            const int slice = kSplitOut ? cta - pair * p.splits : 0;
+            const uint32_t tag = rehearsal ? 0u : exchange_tag(p.exchange.epoch, p.exchange.instance);
+            uint2* const sink = reinterpret_cast<uint2*>(g_rehearsal_sink + (cta * kEpilogueWarps + e) * 32);
 #pragma unroll
             for (int t = 0; t < kTiles; ++t) {
-                const int row = (pair * kTiles + t) * kTileRows + quarter * 32 + lane;
+                const int row = kSwiglu ? pair * kTileRows + quarter * 32 + lane
+                                        : (pair * kTiles + t) * kTileRows + quarter * 32 + lane;
                 if (row < p.out_features) {
-                    const size_t column = rehearsal ? lane : row;
-#pragma unroll
-                    for (int i = 0; i < kCols; ++i) {
-                        const int token = first_token + i;
-                        if (token < rows_stored) {
-                            out[token * row_pitch + column] = stash[(t * kCols + i) * kStashPitch];
-                        }
+                    // SwiGLU pair: the row is [gate | up], each half holding all ranks' columns
+                    const size_t element = static_cast<size_t>(slice) * p.exchange.width +
+                                           (kSwiglu ? t * (p.exchange.width / 2) : 0) + p.exchange.first_column + row;
+                    const float value = stash[(t * kCols) * kStashPitch];
+                    for (int r = 0; r < p.exchange.ranks; ++r) {
+                        store_tagged(rehearsal ? sink + (lane >> 1) : p.exchange.copies[r] + element, value, tag);
                     }
                 }
             }
