@@ -18,21 +18,25 @@
 //     stored: a stage is 128 tokens of one kv head, each unit of 16 tokens (a whole 16-token page, or a quarter
 //     of a 64-token page) two swizzled TMA boxes of 128 bytes per token.  K is the A operand of S^T = K Q^T
 //     (128 tokens x 256 dims, K-major), V the A operand of O^T = V^T P^T (dims x tokens, MN-major);
-//   * queries and probabilities enter as e4m3 digits.  An e4m3 has four significant bits, so a number x is
-//     written as x0 + x1 / 16 + x2 / 256, every digit rounded to nearest from what the digits before it left, and
-//     digit j of head h is column 8 j + h of the B operand: three accumulators per output, added with their
-//     weights in fp32.  A head's query is first brought to [128, 256) by a power of two: a bf16's eight bits are
-//     exact down to 2^-18 of the largest element, and an element below that is off by 2^-26 of the largest.
-//     A probability is kept to 2^-13 of itself (f16, which the kernel used to multiply with: 2^-12), down to
-//     2^-26 of the largest;
+//   * queries and probabilities enter as e4m3 digits.  An e4m3 has four significant bits, so a number is written as
+//     a sum of digits with powers of two for weights, every digit rounded to nearest from what the digits before it
+//     left, and digit j of head h is column 8 j + h of the B operand: one accumulator per digit and output, added
+//     with their weights in fp32.  A head's query is first brought to [128, 256) by a power of two and takes four
+//     digits, of weight 1, 2^-4, 2^-18 and 2^-23: the first two hold a bf16's eight bits down to 2^-14 of the
+//     largest element, the others (and the overlap) from there on, so that every element is exact down to 2^-32 of
+//     the binade of the largest.  That is all that f16, which the kernel used to multiply with, holds exactly (2^-17
+//     to 65504), whichever keys are zero.  A probability is p0 + p1 / 16 + p2 / 256, kept to 2^-13 of itself (f16:
+//     2^-12), down to 2^-26 of the largest;
 //   * O of one stage is read from tensor memory and added to fp32 registers, where a change of the running
 //     maximum costs one multiplication.
 //
 //   warps 0-3   softmax: thread = token of the stage.  S from tensor memory, maximum over the 128 tokens,
 //               exponentials, digits of P to shared memory
-//   warps 4-11  thread = output dim: digits of the next task's query, the accumulators of O, the result
+//   warps 4-11  thread = output dim: the accumulators of O, the result
 //   warp 12     issues the MMAs: S of stage n + 1 before O of stage n
 //   warps 13,14 fetch K and V into rings of three stages, ahead across task boundaries
+//   warps 15,16 the query's digits, half of the heads each
+//   warp 17     the tasks of one chunk after the other
 //
 // What it took to get there: widening every cache byte to f16 for mma.sync kept the conversion unit 76 % busy
 // and the stage on dependent instructions.  Measured (us, layers that L2 does not hold, before / now):
@@ -56,8 +60,9 @@ constexpr int kFirstOutputWarp = kSoftmaxWarps;
 constexpr int kMmaWarp = kFirstOutputWarp + kOutputWarps;
 constexpr int kKeyWarp = kMmaWarp + 1;
 constexpr int kValueWarp = kMmaWarp + 2;
-constexpr int kQueryWarp = kMmaWarp + 3;
-constexpr int kPlanWarp = kMmaWarp + 4;
+constexpr int kFirstQueryWarp = kMmaWarp + 3;
+constexpr int kQueryWarps = 2;
+constexpr int kPlanWarp = kFirstQueryWarp + kQueryWarps;
 constexpr int kListReaders = kPlanWarp;  // every warp before it reads the task lists
 constexpr int kThreads = (kPlanWarp + 1) * 32;
 constexpr int kUnitTokens = 16;
@@ -67,7 +72,8 @@ constexpr int kBoxBytes = kUnitTokens * 128;            // half the dims of a un
 constexpr int kHalfBytes = kStageUnits * kBoxBytes;     // ... of a stage
 constexpr int kStageBytes = 2 * kHalfBytes;             // K or V of a stage
 constexpr int kStages = 3;
-constexpr int kDigits = 3;
+constexpr int kQueryDigits = 4;                         // of weight 1, 2^-4, 2^-18, 2^-23
+constexpr int kProbabilityDigits = 3;                   // of weight 1, 2^-4, 2^-8
 constexpr int kColumns = 32;                            // digit j of head h is column 8 j + h; the rest is zero
 constexpr int kQueryBytes = kColumns * kHeadDim;        // B operand of S, K-major core matrices
 constexpr int kProbabilityBytes = kColumns * kStageTokens;  // B operand of O, MN-major core matrices
@@ -125,6 +131,7 @@ struct Smem {
 };
 
 static_assert(sizeof(Smem) + 1024 <= 232448, "shared memory of a CTA");
+static_assert(kGqaGroup % kQueryWarps == 0, "as many heads for each query warp");
 
 // (out of line, as in the projection kernels: a wait that is already satisfied costs one test)
 __device__ __noinline__ bool att_wait_slow(uint64_t* bar, uint32_t parity, Smem& sm, int* status) {
@@ -192,6 +199,36 @@ __device__ __forceinline__ uint32_t take_digit(float& lo, float& hi) {
     return digit;
 }
 
+__device__ __forceinline__ uint32_t f16x2_to_e4m3x2(__half2 value) {
+    uint16_t out;
+    asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(out) : "r"(*reinterpret_cast<const uint32_t*>(&value)));
+    return out;
+}
+
+__device__ __forceinline__ __half2 e4m3x2_to_half2(uint32_t digits) {
+    const uint32_t value = cvt_e4m3x2_to_f16x2(digits);
+    return *reinterpret_cast<const __half2*>(&value);
+}
+
+// The first two digits of two query elements, |x| < 256, in f16 arithmetic: exact, as all numbers in it have eight
+// significant bits at most (an x below 2^-17 becomes a multiple of 2^-24, which costs nothing: the digits after these
+// two start from x).  Together they are x itself from 2^-6 on, ...
+__device__ __forceinline__ void take_high_digits(float lo, float hi, uint32_t& d0, uint32_t& d1) {
+    const __half2 x = __floats2half2_rn(lo, hi);
+    d0 = f16x2_to_e4m3x2(x);
+    d1 = f16x2_to_e4m3x2(__hmul2(__hsub2(x, e4m3x2_to_half2(d0)), __float2half2_rn(16.0f)));
+}
+
+// ... and below they leave at most 2^-14 (a multiple of 2^-13 is what they make there), which the third holds as a
+// normal number down to 2^-24 and the fourth finishes.
+__device__ __forceinline__ void take_low_digits(float lo, float hi, uint32_t d0, uint32_t d1, uint32_t& d2, uint32_t& d3) {
+    const float2 taken =
+        __half22float2(__hfma2(e4m3x2_to_half2(d1), __float2half2_rn(0.0625f), e4m3x2_to_half2(d0)));
+    const __half2 rest = __floats2half2_rn((lo - taken.x) * 262144.0f, (hi - taken.y) * 262144.0f);
+    d2 = f16x2_to_e4m3x2(rest);
+    d3 = f16x2_to_e4m3x2(__hmul2(__hsub2(rest, e4m3x2_to_half2(d2)), __float2half2_rn(32.0f)));
+}
+
 // Largest value of the warp (a NaN counts as nothing).
 __device__ __forceinline__ float warp_highest(float value) {
     float out;
@@ -229,9 +266,15 @@ __device__ __forceinline__ int claimed_chunk(const ulonglong2* answer) {
     return index;
 }
 
-// Three accumulators of a digit each, with their weights.
+// Accumulators of a digit each, with their weights: of probabilities ...
 __device__ __forceinline__ float combine_digits(uint32_t d0, uint32_t d1, uint32_t d2) {
     return fmaf(fmaf(__uint_as_float(d2), 0.0625f, __uint_as_float(d1)), 0.0625f, __uint_as_float(d0));
+}
+
+// ... and of queries.
+__device__ __forceinline__ float combine_query_digits(uint32_t d0, uint32_t d1, uint32_t d2, uint32_t d3) {
+    const float low = fmaf(__uint_as_float(d3), 1.0f / 32.0f, __uint_as_float(d2));
+    return fmaf(fmaf(low, 1.0f / 16384.0f, __uint_as_float(d1)), 0.0625f, __uint_as_float(d0));
 }
 
 // Cache pages as rows of 256 bytes, fetched in boxes of 16 tokens x 128 bytes.  The launcher does not know how many
@@ -376,7 +419,7 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
             mbar_init(&sm.v_empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&sm.q_ready[i], 1);
+            mbar_init(&sm.q_ready[i], kQueryWarps);
             mbar_init(&sm.q_free[i], 1 + kSoftmaxWarps);
             mbar_init(&sm.s_ready[i], 1);
             mbar_init(&sm.s_free[i], kSoftmaxWarps);
@@ -766,9 +809,9 @@ if (keys) {
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    uint32_t d01[16], d2[8];
+                    uint32_t d01[16], d23[16];
                     tmem_load16_issue(s_lane + buffer * kColumns, d01);
-                    tmem_load8_issue(s_lane + buffer * kColumns + 16, d2);
+                    tmem_load16_issue(s_lane + buffer * kColumns + 16, d23);
                     tmem_load_wait();
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
@@ -781,7 +824,8 @@ if (keys) {
                     float mine = -INFINITY;
 #pragma unroll
                     for (int h = 0; h < kGqaGroup; ++h) {
-                        score[h] = valid ? combine_digits(d01[h], d01[8 + h], d2[h]) * score_scale[h] : -INFINITY;
+                        score[h] = valid ? combine_query_digits(d01[h], d01[8 + h], d23[h], d23[8 + h]) * score_scale[h]
+                                         : -INFINITY;
                         const float highest = warp_highest(score[h]);
                         mine = lane == h ? highest : mine;
                     }
@@ -810,9 +854,9 @@ if (keys) {
                         running_max[h] = new_max;
                         probability[h] *= 256.0f;
                     }
-                    uint32_t words[2 * kDigits];
+                    uint32_t words[2 * kProbabilityDigits];
 #pragma unroll
-                    for (int j = 0; j < kDigits; ++j) {
+                    for (int j = 0; j < kProbabilityDigits; ++j) {
                         const uint32_t pair0 = take_digit(probability[0], probability[1]);
                         const uint32_t pair1 = take_digit(probability[2], probability[3]);
                         words[2 * j] = pair0 | pair1 << 16;
@@ -868,8 +912,14 @@ if (keys) {
                 mbar_arrive(&sm.list_free[m & 1]);
             }
         }
-    } else if (warp == kQueryWarp) {
-        // ---------------- query digits: eight dims per lane, one head after the other ----------------
+    } else if (warp >= kFirstQueryWarp && warp < kPlanWarp) {
+        // ---------------- query digits: half of the heads per warp, eight dims per lane --------------
+        // (A task cannot start before they are there, so two warps share them, and no branch keeps one head's
+        // conversions from running beside another's.  Us per layer, one warp with three digits in fp32 / with four /
+        // two warps with four in f16: one row of 2048 12.2 / 12.7 / 11.2, 32 rows in [128, 2048] 25.1 / 27.4 / 24.3; the
+        // last two digits only for heads that need them: 11.1 and 24.3.)
+        constexpr int kHeads = kGqaGroup / kQueryWarps;
+        const int first_head = (warp - kFirstQueryWarp) * kHeads;
         pdl_wait();
         for (int m = 0; ok; ++m) {
             ok = att_wait(&sm.list_ready[m & 1], (m >> 1) & 1, sm, status);
@@ -880,24 +930,30 @@ if (keys) {
             for (int i = 0; i < count && ok; ++i) {
                 const Task task = sm.tasks[m & 1][i];
                 const uint2* at_lane = reinterpret_cast<const uint2*>(
-                    query + (static_cast<size_t>(task.row) * kQueryHeads + task.kv_head * kGqaGroup) * kHeadDim + 8 * lane);
-                uint2 raw[kGqaGroup][2];  // (rows start on 8-byte boundaries)
+                    query +
+                    (static_cast<size_t>(task.row) * kQueryHeads + task.kv_head * kGqaGroup + first_head) * kHeadDim +
+                    8 * lane);
+                uint32_t pairs[kHeads][4];  // (rows start on 8-byte boundaries)
 #pragma unroll
-                for (int h = 0; h < kGqaGroup; ++h) {
-                    raw[h][0] = at_lane[h * (kHeadDim / 4)];
-                    raw[h][1] = at_lane[h * (kHeadDim / 4) + 1];
+                for (int h = 0; h < kHeads; ++h) {
+                    const uint2 first = at_lane[h * (kHeadDim / 4)];
+                    const uint2 second = at_lane[h * (kHeadDim / 4) + 1];
+                    pairs[h][0] = first.x;
+                    pairs[h][1] = first.y;
+                    pairs[h][2] = second.x;
+                    pairs[h][3] = second.y;
                 }
                 ok = att_wait(&sm.q_free[t & 1], ((t >> 1) & 1) ^ 1, sm, status);
                 if (!ok) {
                     break;
                 }
+                uint32_t digits[kHeads][kQueryDigits][4];
 #pragma unroll
-                for (int h = 0; h < kGqaGroup; ++h) {
-                    const uint32_t pairs[4] = {raw[h][0].x, raw[h][0].y, raw[h][1].x, raw[h][1].y};
+                for (int h = 0; h < kHeads; ++h) {
                     uint32_t highest = 0;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        highest = max(highest, max(pairs[j] & 0x7fffu, (pairs[j] >> 16) & 0x7fffu));
+                        highest = max(highest, max(pairs[h][j] & 0x7fffu, (pairs[h][j] >> 16) & 0x7fffu));
                     }
                     highest = __reduce_max_sync(0xffffffffu, highest);
                     // largest magnitude to [128, 256).  With an infinity in the head only the infinities count, and
@@ -905,10 +961,9 @@ if (keys) {
                     const uint32_t exponent = max(highest >> 7, 8u);
                     const bool infinite = highest >= 0x7f80u;
                     const float up = __uint_as_float((261u - exponent) << 23);
-                    uint32_t bytes[kDigits][2];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        float lo = __uint_as_float(pairs[j] << 16), hi = __uint_as_float(pairs[j] & 0xffff0000u);
+                        float lo = __uint_as_float(pairs[h][j] << 16), hi = __uint_as_float(pairs[h][j] & 0xffff0000u);
                         if (infinite) {
                             lo = isnan(lo) ? lo : isinf(lo) ? copysignf(1.0f, lo) : 0.0f;
                             hi = isnan(hi) ? hi : isinf(hi) ? copysignf(1.0f, hi) : 0.0f;
@@ -916,19 +971,21 @@ if (keys) {
                             lo *= up;
                             hi *= up;
                         }
-#pragma unroll
-                        for (int d = 0; d < kDigits; ++d) {
-                            const uint32_t digit = take_digit(lo, hi);
-                            bytes[d][j >> 1] = (j & 1) ? bytes[d][j >> 1] | digit << 16 : digit;
-                        }
-                    }
-                    uint8_t* const at = &sm.q[t & 1][(lane >> 1) * 16 * kColumns + h * 16 + (lane & 1) * 8];
-#pragma unroll
-                    for (int d = 0; d < kDigits; ++d) {
-                        *reinterpret_cast<uint2*>(at + d * 128) = make_uint2(bytes[d][0], bytes[d][1]);
+                        take_high_digits(lo, hi, digits[h][0][j], digits[h][1][j]);
+                        take_low_digits(lo, hi, digits[h][0][j], digits[h][1][j], digits[h][2][j], digits[h][3][j]);
                     }
                     if (lane == 0) {
-                        sm.query_scale[t & 1][h] = infinite ? INFINITY : __uint_as_float((exponent - 7u) << 23);
+                        sm.query_scale[t & 1][first_head + h] =
+                            infinite ? INFINITY : __uint_as_float((exponent - 7u) << 23);
+                    }
+                }
+                uint8_t* const at = &sm.q[t & 1][(lane >> 1) * 16 * kColumns + first_head * 16 + (lane & 1) * 8];
+#pragma unroll
+                for (int h = 0; h < kHeads; ++h) {
+#pragma unroll
+                    for (int d = 0; d < kQueryDigits; ++d) {
+                        *reinterpret_cast<uint2*>(at + h * 16 + d * 128) = make_uint2(
+                            digits[h][d][0] | digits[h][d][1] << 16, digits[h][d][2] | digits[h][d][3] << 16);
                     }
                 }
                 fence_proxy_async();

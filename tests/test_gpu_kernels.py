@@ -336,9 +336,8 @@ def test_packed_attention_positions_beyond_32_bits(cuda, ops):
 
 @pytest.mark.parametrize("kind", ["tiny", "large", "outlier", "spread"])
 def test_packed_attention_query_digits(cuda, ops, kind):
-    """Queries far from unit scale.  Three e4m3 digits below a head's largest element hold a bf16 exactly down to
-    2^-18 of it; what an element below that is off by, 2^-26 of the largest per dim, moves a score by less than
-    fp32 sums of 256 products do, so the bounds are those of every attention test."""
+    """Queries far from unit scale.  The e4m3 digits of a query hold a bf16 exactly down to 2^-32 of the binade of its
+    head's largest element, so the bounds are those of every attention test."""
     case = synth.attention_case(18, [300, 41], page_size=16, with_gate=True)
     query = synth.bf16_value(case["query"]).astype(np.float32)
     rng = np.random.default_rng(18)
@@ -356,6 +355,26 @@ def test_packed_attention_query_digits(cuda, ops, kind):
     case["query"] = synth.bf16_bits(query)
     for partitions in (1, 3):
         check_attention(run_attention(cuda, ops, case, 16, partitions), attention_oracle(case, 16), kind)
+
+
+@pytest.mark.parametrize("binades", [0, 13, 14, 18, 20, 22, 25, 28, 31, 32])
+def test_packed_attention_query_holds_what_f16_holds(cuda, ops, binades):
+    """One dim of 2^15, on keys that are zero there, beside dims that decide the softmax, from the same binade down to
+    2^-17: f16 holds all of these exactly (eight significant bits), and so must the digits of the query.  The bounds are
+    those of every attention test; a query of three digits 2^-4 apart misses them from 2^18 on."""
+    case = synth.attention_case(20, [300, 41], page_size=16, scaled=True)
+    rng = np.random.default_rng(binades)
+    small = 2.0 ** (15 - binades)
+    codes = rng.integers(128, 256, (2, 24, 256)) * rng.choice([-1.0, 1.0], (2, 24, 256))  # eight significant bits each
+    query = (codes / 128.0 * small).astype(np.float32)
+    query[:, :, 7] = 2.0 ** 15
+    keys = rng.standard_normal(case["key_cache"].shape, dtype=np.float32)
+    keys[..., 7] = 0.0
+    # scores of order 1: 256 products of about 1.5 small, over 16
+    case.update(query=synth.bf16_bits(query), key_cache=synth.e4m3_encode(keys),
+                k_scale=np.full(4, 1.0 / small, dtype=np.float32))
+    for partitions in (1, 3):
+        check_attention(run_attention(cuda, ops, case, 16, partitions), attention_oracle(case, 16), f"2^{binades}")
 
 
 @pytest.mark.parametrize("value", [np.nan, np.inf])
