@@ -49,6 +49,7 @@
 // pool, as the reference allocates it): positions past the context are masked by
 // zero probabilities, not skipped.
 
+#include "attention_plan.h"
 #include "tcgen05.cuh"
 
 namespace qwc {
@@ -65,8 +66,6 @@ constexpr int kQueryWarps = 2;
 constexpr int kPlanWarp = kFirstQueryWarp + kQueryWarps;
 constexpr int kListReaders = kPlanWarp;  // every warp before it reads the task lists
 constexpr int kThreads = (kPlanWarp + 1) * 32;
-constexpr int kUnitTokens = 16;
-constexpr int kStageUnits = 8;
 constexpr int kStageTokens = kStageUnits * kUnitTokens;
 constexpr int kBoxBytes = kUnitTokens * 128;            // half the dims of a unit
 constexpr int kHalfBytes = kStageUnits * kBoxBytes;     // ... of a stage
@@ -83,13 +82,6 @@ constexpr int kOutputColumn = 2 * kColumns;             // two buffers of two ha
 constexpr int kPartialFloats = 2;
 constexpr size_t kPartialBytes = 2 * sizeof(float) + kHeadDim * sizeof(__half);  // 520
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr int kMaxListTasks = 96;     // tasks of one chunk; the plan keeps it below
-constexpr int kPlanMinPadding = 4;    // units a task costs beyond its tokens
-constexpr int kPlanPaddingDivisor = 64;  // padding = share / this at least: bounds the tasks of one chunk
-constexpr int kChunksPerSm = 4;       // one large chunk and three small ones
-constexpr int kDynamicShare = 192;    // units per SM from which on the line is cut into chunks of two sizes ...
-constexpr int kThreeSmallShare = 480;  // ... with three small ones instead of two
-constexpr int kPlanRows = 256;        // rows whose prefix fits the shared-memory table
 
 struct Task {
     int row;
@@ -131,6 +123,7 @@ struct Smem {
 };
 
 static_assert(sizeof(Smem) + 1024 <= 232448, "shared memory of a CTA");
+static_assert(kPlanKvHeads == kKvHeads, "the plan's pairs");
 static_assert(kGqaGroup % kQueryWarps == 0, "as many heads for each query warp");
 
 // (out of line, as in the projection kernels: a wait that is already satisfied costs one test)
@@ -296,87 +289,6 @@ cudaError_t encode_cache_map(CUtensorMap* map, const void* cache) {
     return result == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// The split plan.
-//
-// The (row, kv head) pairs are laid end to end, row-major, on a line of units; a pair takes
-// max(units, 1) + padding positions (the padding stands for what a task costs beyond its tokens).
-// The line is cut into chunks, and a task is the piece of one pair inside one chunk, partial number
-// c - (first chunk that touches the pair); a pair without context is one empty piece.  The last piece of a pair says
-// so in the sign of its sum: the merge kernel needs no plan.
-//   * One equal chunk per SM, up to kDynamicShare units.  Beyond that one large chunk (seven tenths of an SM's share)
-//     and two or, from kThreeSmallShare on, three small ones: a CTA starts with a large chunk and, once it has
-//     asked for its last bytes, takes the next chunk that nobody has.  The SMs do not get the same share of the
-//     memory's bandwidth (40 to 56 GB/s each, others every time): with equal chunks of 350 units the CTAs' ends
-//     lay 53 to 72 us after their first copies.  Measured (us, equal chunks / two small / three small / six small):
-//     share 350 (32 rows, log-uniform to 32768) 79.9 / 77.2 / 78.6 / 83.4, 330 76.0 / 71.8 / 72.8, 612 (20 rows,
-//     8192 to 32768) 128.5 / 123.0 / 121.1 / 126.1, 230 (32 x 4096) 56.3 / 55.2 / 58.2; at 166 (three rows of
-//     32768, forced) 42.8 / - / 52.1.
-//   * padding >= share / kPlanPaddingDivisor, so that a chunk never holds more than kPlanPaddingDivisor + 4 tasks;
-//   * every chunk >= capacity / (partitions - 1): a row never has more pieces than the workspace has slots;
-//   * every chunk is a whole number of stages.
-// Position: uint32_t, unless the block tables could describe a longer line (plan_is_wide).
-template <typename Position>
-struct SplitPlan {
-    Position large, small;
-    Position line;
-    int padding;
-};
-
-constexpr int kPlanSlack = 1 << 20;  // more than the padding of a pair can be while positions have 32 bits
-
-template <typename Position>
-__device__ __forceinline__ SplitPlan<Position> make_split_plan(Position total_row_units, int rows, int smallest_chunk,
-                                                               int ctas) {
-    // (shares in floating point, rounded up by more than the arithmetic can be off)
-    const float per_cta = 1.00001f / static_cast<float>(ctas);
-    const Position smallest = static_cast<Position>(smallest_chunk);
-    Position share = static_cast<Position>(static_cast<float>(total_row_units) * kKvHeads * per_cta) + 1;
-    share = share > smallest ? share : smallest;
-    SplitPlan<Position> plan;
-    plan.padding = static_cast<int>(share / kPlanPaddingDivisor) + 1;
-    plan.padding = plan.padding > kPlanMinPadding ? plan.padding : kPlanMinPadding;
-    plan.line = (total_row_units + static_cast<Position>(rows) * plan.padding) * kKvHeads;
-    share = static_cast<Position>(static_cast<float>(plan.line) * per_cta) + 1;
-    const bool dynamic = share >= kDynamicShare;
-    const Position tenth = share / 10;
-    plan.small = !dynamic ? share : share >= kThreeSmallShare ? tenth : tenth + tenth / 2;
-    plan.large = !dynamic ? share : share - (share >= kThreeSmallShare ? 3 : 2) * plan.small;
-    plan.large = ((plan.large > smallest ? plan.large : smallest) + kStageUnits - 1) / kStageUnits * kStageUnits;
-    plan.small = ((plan.small > smallest ? plan.small : smallest) + kStageUnits - 1) / kStageUnits * kStageUnits;
-    return plan;
-}
-
-// The chunk that holds a position of the line ...
-template <typename Position>
-__device__ __forceinline__ int chunk_of(const SplitPlan<Position>& plan, Position position, int ctas) {
-    const Position small_begin = plan.large * ctas;
-    return position < small_begin ? static_cast<int>(position / plan.large)
-                                  : ctas + static_cast<int>((position - small_begin) / plan.small);
-}
-
-// ... and where a chunk begins.
-template <typename Position>
-__device__ __forceinline__ Position chunk_begin(const SplitPlan<Position>& plan, int chunk, int ctas) {
-    return chunk < ctas ? plan.large * chunk : plan.large * ctas + plan.small * (chunk - ctas);
-}
-
-// first position of pair (row, kv head); units_before = units of the rows before it
-template <typename Position>
-__device__ __forceinline__ Position pair_position(const SplitPlan<Position>& plan, int row, int kv_head,
-                                                  Position units_before, Position row_units) {
-    return (units_before + static_cast<Position>(row) * plan.padding) * kKvHeads +
-           static_cast<Position>(kv_head) * (row_units + plan.padding);
-}
-
-// A context longer than the block table can describe is cut at the table's capacity.
-__device__ __forceinline__ int units_of_context(uint32_t context, int capacity_units) {
-    const uint32_t units = (context + kUnitTokens - 1) / kUnitTokens;
-    return static_cast<int>(units < static_cast<uint32_t>(capacity_units) ? units : capacity_units);
-}
-
-// Units a row occupies on the plan's line: a row without context still gets one task (it stores zeros).
-__device__ __forceinline__ int plan_units(int units) { return units > 0 ? units : 1; }
-
 template <bool kSplit, typename Position>
 __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
     const __grid_constant__ CUtensorMap key_map, const __grid_constant__ CUtensorMap value_map,
@@ -526,24 +438,23 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
                     if (r < rows) {
                         occupied = first_unit[r + 1] - first_unit[r];
                         start = pair_position(plan, r, kv, first_unit[r], occupied);
-                        inside = start < high && start + occupied > low;
+                        inside = piece_inside(start, occupied, low, high);
                     }
                     const uint32_t found = __ballot_sync(0xffffffffu, inside);
                     const int index = count + __popc(found & ((1u << lane) - 1u));
                     if (inside && index < kMaxListTasks) {
                         const uint32_t row_context = __ldcg(context_lengths + row_base + r);
                         const int row_units = units_of_context(row_context, capacity_units);
-                        const Position begin = low > start ? low - start : 0;
-                        const Position end = high - start < occupied ? high - start : occupied;
+                        const PlanPiece piece = piece_of_pair(plan, start, occupied, chunk, low, high, ctas);
                         Task task;
                         task.context =
                             static_cast<int>(min(row_context, static_cast<uint32_t>(capacity_units) * kUnitTokens));
                         task.row = row_base + r;
                         task.kv_head = kv;
-                        task.part = start < low ? chunk - chunk_of(plan, start, ctas) : 0;
-                        task.last = end == occupied;
-                        task.unit_begin = static_cast<int>(begin);
-                        task.units = max(0, min(static_cast<int>(end), row_units) - static_cast<int>(begin));
+                        task.part = piece.part;
+                        task.last = piece.last;
+                        task.unit_begin = piece.begin;
+                        task.units = max(0, min(piece.end, row_units) - piece.begin);
                         tasks[index] = task;
                     }
                     count += __popc(found);
@@ -1308,21 +1219,16 @@ cudaError_t launch_attention(const void* query, const void* query_gate_projectio
     // partials is a multiple of 24, so the f16 block starts on a 16-byte boundary.
     float* partial_stats = split ? static_cast<float*>(workspace) : nullptr;
     __half* partial_out = split ? reinterpret_cast<__half*>(partial_stats + partials * kPartialFloats) : nullptr;
-    const long long capacity_units = static_cast<long long>(max_blocks) * (page_size / kUnitTokens);
-    const int smallest_chunk = split ? static_cast<int>((capacity_units + partitions - 2) / (partitions - 1)) : 0;
-    // What the block tables could describe bounds the line: whether its positions fit 32 bits (a large chunk per
-    // SM among them), and whether an SM's share can reach the length from which on chunks have two sizes.
-    const long long longest = (capacity_units + kPlanSlack) * rows * kKvHeads;
-    const bool wide = split && (longest >= (1ll << 31) || static_cast<long long>(smallest_chunk) * sms >= (1ll << 30));
-    const bool may_be_dynamic = split && capacity_units * rows * kKvHeads / sms >= kDynamicShare / 2;
-    const AttentionKernel kernel = attention_kernels[split ? (wide ? 2 : 1) : 0];
+    const PlanShape plan =
+        split ? plan_shape(rows, max_blocks, page_size, partitions, sms) : PlanShape{0, false, false};
+    const AttentionKernel kernel = attention_kernels[split ? (plan.wide ? 2 : 1) : 0];
     const cudaError_t launched = qwc::launch_chained(
-        kernel, dim3(may_be_dynamic ? kChunksPerSm * sms : sms), dim3(kThreads), shared, stream, key_map, value_map,
+        kernel, dim3(plan.may_be_dynamic ? kChunksPerSm * sms : sms), dim3(kThreads), shared, stream, key_map, value_map,
         static_cast<const __nv_bfloat16*>(query), static_cast<const __nv_bfloat16*>(query_gate_projection),
         static_cast<const uint32_t*>(block_tables), static_cast<const uint32_t*>(context_lengths), key_scales,
         value_scales, split ? nullptr : static_cast<__nv_bfloat16*>(output),
         split ? nullptr : static_cast<__half*>(staged_output), padded_rows, partial_stats, partial_out, rows, max_blocks,
-        row_base, page_size, gate_stride, partitions, smallest_chunk, sms, softmax_scale, status);
+        row_base, page_size, gate_stride, partitions, plan.smallest_chunk, sms, softmax_scale, status);
     if (launched != cudaSuccess || !split) {
         return launched;
     }
