@@ -150,7 +150,7 @@ inline PlanShape plan_shape(int rows, int max_blocks, int page_size, int partiti
     PlanShape shape;
     shape.smallest_chunk = static_cast<int>(smallest);
     shape.wide = chunk * kChunksPerSm * ctas >= (1ll << 32);  // where the last chunk ends, used or not
-    shape.may_be_dynamic = described * rows * kPlanKvHeads / ctas >= kDynamicShare / 2;
+    shape.may_be_dynamic = padded_share >= kDynamicShare;
     return shape;
 }
 

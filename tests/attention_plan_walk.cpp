@@ -122,6 +122,10 @@ int main() {
     if (!check({60, 1800000, 64, 2, 148, std::vector<uint32_t>(60, 115200000u)})) {
         return 1;
     }
+    // short rows, whose padding brings the share of an SM over the line between one size of chunks and two
+    if (!check({196, 3, 16, 8, 28, std::vector<uint32_t>(196, 48u)})) {
+        return 1;
+    }
     // contexts at the largest numbers of tokens that a launch can be given
     if (!check({32, 1 << 28, 16, 2, 148, std::vector<uint32_t>(32, 0xfffffff0u)})) {
         return 1;
