@@ -484,10 +484,15 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
             }
             // The next chunk is claimed once the last bytes of this one have been asked for (an answer takes 0.2
             // us, the ring holds three stages); what lies past the end of the line is claimed too (it would
-            // start, and find nothing to do).
+            // start, and find nothing to do).  Where no small chunk has work, because the tables describe far more
+            // than the contexts take, there is nothing to wait for: the claims only clear the rest of the grid away,
+            // and the sooner that is done, the sooner the merge kernel may start (nine rows in [128, 2048] under
+            // tables of 32768 tokens 13.07 -> 12.92 us, as with a grid of one CTA per SM).
             chunk = -1;
-            ok = att_wait(&sm.list_free[(m + 1) & 1], (((m + 1) >> 1) & 1) ^ 1, sm, status) &&
-                 att_wait(&sm.list_wanted, m & 1, sm, status);
+            ok = att_wait(&sm.list_free[(m + 1) & 1], (((m + 1) >> 1) & 1) ^ 1, sm, status);
+            if (ok && gridDim.x > ctas && chunk_begin(plan, ctas, ctas) < plan.line) {
+                ok = att_wait(&sm.list_wanted, m & 1, sm, status);
+            }
             while (gridDim.x > ctas && ok) {
                 if (lane == 0) {
                     fence_proxy_async();  // the answer before this one has been read

@@ -318,6 +318,51 @@ def test_packed_attention_chunks(cuda, ops, contexts, page_size, partitions):
     check_attention(got, want, "chunks")
 
 
+@pytest.mark.parametrize("contexts,table_tokens", [([2048, 300, 1, 0, 777, 128, 129, 1500, 90], 32768),
+                                                   ([30000, 33, 0, 31001, 17, 30016, 29999], 32768)],
+                         ids=["no_small_chunk_has_work", "two_small"])
+def test_packed_attention_chunks_claimed_beside_another_stream(cuda, ops, contexts, table_tokens):
+    """Chunks are claimed while calls on another stream hold SMs: whoever is first takes them, and the outputs, gated
+    and scaled, are the same bits as alone (what a piece is does not depend on who works on it)."""
+    torch = cuda
+    contexts = np.asarray(contexts, dtype=np.uint32)
+    rows, blocks, partitions = contexts.size, table_tokens // 16, 128
+    case = synth.attention_case(21, [1024], page_size=16, scaled=True)
+    rng = np.random.default_rng(21)
+    tables = rng.integers(0, case["num_blocks"], (rows, blocks)).astype(np.uint32)
+    query = synth.bf16_bits(rng.standard_normal((rows, 24, 256), dtype=np.float32))
+    gate = synth.bf16_bits(rng.standard_normal((rows, 24, 512), dtype=np.float32))
+    keys, values, tables_d, query_d, gate_d, contexts_d, ks, vs = (
+        dev(torch, a) for a in (case["key_cache"], case["value_cache"], tables, query, gate, contexts, case["k_scale"],
+                                case["v_scale"]))
+    full_d = dev(torch, np.full(rows, table_tokens, dtype=np.uint32))
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    workspaces = [torch.full((ops.packed_workspace_bytes(rows, partitions),), 0xFF, dtype=torch.uint8, device="cuda")
+                  for _ in streams]
+    outs = [bf16_out(torch, rows, 24, 256) for _ in range(9)]
+    busy = bf16_out(torch, rows, 24, 256)
+
+    def call(lengths, out, workspace):
+        ops.gated_packed(query_d, gate_d, keys, values, tables_d, lengths, blocks, out, rows, 0, partitions, workspace, 16,
+                         ks, vs)
+
+    torch.cuda.synchronize()
+    call(contexts_d, outs[0], workspaces[0])
+    torch.cuda.synchronize()
+    for out in outs[1:]:
+        with torch.cuda.stream(streams[1]):
+            call(full_d, busy, workspaces[1])
+        with torch.cuda.stream(streams[0]):
+            call(contexts_d, out, workspaces[0])
+    torch.cuda.synchronize()
+    for out in outs[1:]:
+        assert torch.equal(out, outs[0])
+    want = attention_oracle(dict(case, contexts=contexts, block_tables=tables, max_blocks=blocks, query=query,
+                                 gate_projection=gate), 16)
+    want[contexts == 0] = 0.0  # (the oracle divides by a sum of nothing)
+    check_attention(synth.bf16_value(host(outs[0])), want, "two streams")
+
+
 def test_packed_attention_positions_beyond_32_bits(cuda, ops):
     """A block table that could describe 134 million tokens, with two slots per row: the plan's positions no longer
     fit 32 bits."""
