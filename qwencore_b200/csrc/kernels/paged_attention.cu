@@ -357,6 +357,8 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
     bool ok = true;
     int t = 0;  // tasks and ...
     int n = 0;  // ... stages so far, over all chunks
+    int issued = 0;  // the MMA warp: O of this many stages
+    int claims = 0;  // the plan warp: chunks asked for
 
     if (warp == kPlanWarp || warp == 0) {
         // ---------------- plan: the tasks of one chunk after the other ------------------------------
@@ -398,7 +400,6 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
             plan = make_split_plan(carry, rows, smallest_chunk, ctas);
         }
         int chunk = earlier_failure != 0 ? -1 : static_cast<int>(blockIdx.x);
-        int claims = 0;
 #pragma unroll 1
         for (int m = 0; ok; ++m) {
             Task* const tasks = rehearsal ? reinterpret_cast<Task*>(sm.p[1]) : sm.tasks[m & 1];
@@ -556,21 +557,11 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
             }
             __syncwarp();
             if (lane == 0 && ok) {
-if (keys) {
+                if (keys) {
                     mbar_arrive(&sm.list_wanted);
                 }
-                                mbar_arrive(&sm.list_free[m & 1]);
+                mbar_arrive(&sm.list_free[m & 1]);
             }
-        }
-        if (!ok) {
-            // copies that were asked for may still be landing in this CTA's shared memory: wait for the last trip
-            // round the ring, 0.2 ms per slot at most
-            for (int i = n > kStages ? n - kStages : 0; i < n; ++i) {
-                const long long start = clock64();
-                while (!mbar_try_wait(&full[i % kStages], (i / kStages) & 1) && clock64() - start < 400000ll) {
-                }
-            }
-            __syncwarp();
         }
     } else if (warp == kMmaWarp) {
         // ---------------- tensor-core issue ---------------------------------------------------
@@ -609,7 +600,6 @@ if (keys) {
             __syncwarp();
             return true;
         };
-        int issued = 0;  // O of this many stages
         for (int m = 0; ok; ++m) {
             ok = att_wait(&sm.list_ready[m & 1], (m >> 1) & 1, sm, status);
             const int count = ok ? sm.task_count[m & 1] : -1;
@@ -641,10 +631,10 @@ if (keys) {
                             }
                         }
                         umma_commit(&sm.k_empty[slot]);
-                        umma_commit(&sm.s_ready[buffer]);
                         if (st == stages - 1) {
                             umma_commit(&sm.q_free[t & 1]);
                         }
+                        umma_commit(&sm.s_ready[buffer]);
                     }
                     __syncwarp();
                     ++n;
@@ -676,16 +666,6 @@ if (keys) {
             if (lane == 0 && ok) {
                 mbar_arrive(&sm.list_free[m & 1]);
             }
-        }
-        if (!ok && n > 0) {
-            // the MMAs that were issued still read shared memory and write tensor memory: wait for the last of
-            // them (0.2 ms at most) before the CTA gives either back
-            const long long start = clock64();
-            while (!(mbar_try_wait(&sm.k_empty[(n - 1) % kStages], ((n - 1) / kStages) & 1) &&
-                     (issued == 0 || mbar_try_wait(&sm.v_empty[(issued - 1) % kStages], ((issued - 1) / kStages) & 1))) &&
-                   clock64() - start < 400000ll) {
-            }
-            __syncwarp();
         }
     } else if (warp < kSoftmaxWarps) {
         // ---------------- softmax: thread = token ---------------------------------------------
@@ -1027,6 +1007,30 @@ if (keys) {
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*reinterpret_cast<volatile int*>(&sm.failed) != 0) {
+        // A wait gave up somewhere.  Whoever asked for something that arrives by itself waits for it, 0.2 ms at most for
+        // each, whether its own waits went well or not: the memory it arrives in must still be this CTA's.
+        const auto arrived = [](uint64_t* bar, int index, int ring) {
+            const long long start = clock64();
+            while (!mbar_try_wait(&bar[index % ring], (index / ring) & 1) && clock64() - start < 400000ll) {
+            }
+        };
+        if (warp == kKeyWarp || warp == kValueWarp) {  // copies: the last trip round the ring
+            for (int i = n > kStages ? n - kStages : 0; i < n; ++i) {
+                arrived(warp == kKeyWarp ? sm.k_full : sm.v_full, i, kStages);
+            }
+        } else if (warp == kMmaWarp) {  // MMAs, to the last of their commits
+            if (n > 0) {
+                arrived(sm.s_ready, n - 1, 2);
+            }
+            if (issued > 0) {
+                arrived(sm.o_ready, issued - 1, 2);
+            }
+        } else if (warp == kPlanWarp && claims > 0) {  // the answer to a claim
+            arrived(&sm.claim_ready, claims - 1, 1);
+        }
+        __syncthreads();
+    }
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemColumns) : "memory");
     }
