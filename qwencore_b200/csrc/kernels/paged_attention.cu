@@ -120,15 +120,20 @@ struct Smem {
     int task_count[2];              // -1: there is nothing left
     uint32_t tmem_base;
     int failed;                     // a wait gave up
+    int stages_asked;               // of K, so far: a wait that spans more than a stage goes on while this grows
 };
 
 static_assert(sizeof(Smem) + 1024 <= 232448, "shared memory of a CTA");
 static_assert(kPlanKvHeads == kKvHeads, "the plan's pairs");
 static_assert(kGqaGroup % kQueryWarps == 0, "as many heads for each query warp");
 
+// Gives up after 20 ms in which the CTA asked for nothing new.  (Some waits span a whole task or chunk: the queries of
+// the task after the next, the next list.  At 40 to 100 GB/s an SM streams a gigabyte in 20 ms, so on contexts of
+// millions of tokens such a wait is longer than that while everything goes on.)
 // (out of line, as in the projection kernels: a wait that is already satisfied costs one test)
 __device__ __noinline__ bool att_wait_slow(uint64_t* bar, uint32_t parity, Smem& sm, int* status) {
-    const long long start = clock64();
+    long long start = clock64();
+    int asked = *reinterpret_cast<volatile int*>(&sm.stages_asked);
     for (;;) {
 #pragma unroll 1
         for (int spin = 0; spin < 64; ++spin) {
@@ -140,7 +145,12 @@ __device__ __noinline__ bool att_wait_slow(uint64_t* bar, uint32_t parity, Smem&
             return false;
         }
         if (clock64() - start > 40000000ll) {
-            break;
+            const int asked_now = *reinterpret_cast<volatile int*>(&sm.stages_asked);
+            if (asked_now == asked) {
+                break;
+            }
+            asked = asked_now;
+            start = clock64();
         }
     }
     atomicCAS(status, 0, kStatusAttentionPageWait);
@@ -348,6 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
         mbar_init(&sm.list_wanted, 1);
         mbar_init(&sm.claim_ready, 1);
         sm.failed = 0;
+        sm.stages_asked = 0;
         mbar_fence_init();
     }
     fence_proxy_async();
@@ -544,6 +555,9 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
                     }
                     if (lane == 0) {
                         mbar_arrive_expect_tx(&full[slot], static_cast<uint32_t>(units) * 2 * kBoxBytes);
+                        if (keys) {
+                            *reinterpret_cast<volatile int*>(&sm.stages_asked) = n + 1;
+                        }
                     }
                     __syncwarp();
                     if (unit < units) {

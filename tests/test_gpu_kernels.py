@@ -402,6 +402,29 @@ def test_packed_attention_query_digits(cuda, ops, kind):
         check_attention(run_attention(cuda, ops, case, 16, partitions), attention_oracle(case, 16), kind)
 
 
+@pytest.mark.parametrize("long_tokens,rows,partitions", [(6 << 20, 75, 1), (400 << 20, 1, 1000)],
+                         ids=["three_whole_pairs_on_one_sm", "small_chunks"])
+def test_packed_attention_waits_longer_than_their_limit_while_the_stream_goes_on(cuda, ops, long_tokens, rows,
+                                                                                 partitions):
+    """Contexts of millions of tokens, on which the query of the task after the next and the next list of tasks are
+    waited for longer than the 20 ms in which a wait gives up when nothing moves.  All of a row's table names one page,
+    so that the result is attention over that page."""
+    torch = cuda
+    case = synth.attention_case(22, [64] * rows, page_size=64, with_gate=True)
+    blocks = long_tokens // 64
+    contexts = np.full(rows, 64, dtype=np.uint32)
+    contexts[0::37] = long_tokens  # (pairs are dealt round the SMs: with 148 of them these rows meet on four)
+    tables = dev(torch, case["block_tables"][:, :1].astype(np.int32)).repeat(1, blocks)
+    out = bf16_out(torch, rows, 24, 256)
+    workspace = torch.zeros(max(16, ops.packed_workspace_bytes(rows, partitions)), dtype=torch.uint8, device="cuda")
+    ops.gated_packed(dev(torch, case["query"]), dev(torch, case["gate_projection"]), dev(torch, case["key_cache"]),
+                     dev(torch, case["value_cache"]), tables, dev(torch, contexts), blocks, out, rows, 0, partitions,
+                     workspace, 64, None, None)
+    torch.cuda.synchronize()
+    assert ops.abi.lib.qwc_device_status() == 0
+    check_attention(synth.bf16_value(host(out)), attention_oracle(case, 64), "long waits")
+
+
 @pytest.mark.parametrize("binades", [0, 13, 14, 18, 20, 22, 25, 28, 31, 32])
 def test_packed_attention_query_holds_what_f16_holds(cuda, ops, binades):
     """One dim of 2^15, on keys that are zero there, beside dims that decide the softmax, from the same binade down to
