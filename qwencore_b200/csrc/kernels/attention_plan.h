@@ -19,7 +19,8 @@ constexpr int kStageUnits = 8;
 constexpr int kPlanKvHeads = 4;
 constexpr int kPlanMinPadding = 4;        // units a task costs beyond its tokens
 constexpr int kPlanPaddingDivisor = 64;   // padding = share / this at least: bounds the tasks of one chunk
-constexpr int kMaxListTasks = 96;         // tasks of one chunk; the plan keeps it below
+constexpr int kMaxPairsPerSm = 38;        // (256 rows on 27 SMs)
+constexpr int kMaxListTasks = kMaxPairsPerSm + kPlanPaddingDivisor + 4;  // tasks of one chunk (plan_fits)
 constexpr int kChunksPerSm = 4;           // one large chunk and three small ones
 constexpr int kDynamicShare = 192;        // units per SM from which on the line is cut into chunks of two sizes ...
 constexpr int kThreeSmallShare = 480;     // ... with three small ones instead of two
@@ -40,7 +41,8 @@ constexpr int kPlanRows = 256;            // rows whose prefix fits the shared-m
 //     share 350 (32 rows, log-uniform to 32768) 79.9 / 77.2 / 78.6 / 83.4, 330 76.0 / 71.8 / 72.8, 612 (20 rows,
 //     8192 to 32768) 128.5 / 123.0 / 121.1 / 126.1, 230 (32 x 4096) 56.3 / 55.2 / 58.2; at 166 (three rows of
 //     32768, forced) 42.8 / - / 52.1.
-//   * padding >= share / kPlanPaddingDivisor, so that a chunk never holds more than kPlanPaddingDivisor + 4 tasks;
+//   * padding >= share / kPlanPaddingDivisor, so that a chunk never holds more than kPlanPaddingDivisor + 4 tasks and
+//     one per pair and SM (what the padding itself adds to a share);
 //   * every chunk >= capacity / (partitions - 1): a row never has more pieces than the workspace has slots;
 //   * every chunk is a whole number of stages.
 // Position: uint32_t, unless a launch could have chunks that end beyond that (PlanShape::wide).
@@ -126,6 +128,9 @@ QWC_PLAN_FUNCTION int units_of_context(uint32_t context, int capacity_units) {
 
 // Units a row occupies on the plan's line: a row without context still gets one task (it stores zeros).
 QWC_PLAN_FUNCTION int plan_units(int units) { return units > 0 ? units : 1; }
+
+// Whether a list holds the tasks of every chunk (undivided rows: one per pair and SM).
+inline bool plan_fits(int rows, int ctas) { return (rows * kPlanKvHeads + ctas - 1) / ctas <= kMaxPairsPerSm; }
 
 // What the launcher decides about the plan before it knows any context: a bound over all contexts that the block
 // tables can describe.

@@ -124,6 +124,7 @@ struct Smem {
 };
 
 static_assert(sizeof(Smem) + 1024 <= 232448, "shared memory of a CTA");
+static_assert(kMaxListTasks * sizeof(Task) <= kProbabilityBytes, "the rehearsal's list");
 static_assert(kPlanKvHeads == kKvHeads, "the plan's pairs");
 static_assert(kGqaGroup % kQueryWarps == 0, "as many heads for each query warp");
 
@@ -1214,15 +1215,13 @@ cudaError_t launch_attention(const void* query, const void* query_gate_projectio
     if (*opted != cudaSuccess) {
         return *opted;
     }
-    // One CTA per SM at a time, whatever the batch: the task lists are cut on the device.  A list holds
-    // kMaxListTasks entries; the plan gives a chunk at most kPlanPaddingDivisor + 4 (undivided rows: one per row
-    // and kv head and CTA).
+    // One CTA per SM at a time, whatever the batch: the task lists are cut on the device.
     int device = 0, sms = 0;
     if (cudaGetDevice(&device) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) {
         return cudaErrorInvalidDevice;
     }
-    if ((rows * kKvHeads + sms - 1) / sms + kPlanPaddingDivisor + 4 > kMaxListTasks) {
+    if (!plan_fits(rows, sms)) {
         return cudaErrorInvalidValue;
     }
     CUtensorMap key_map, value_map;

@@ -80,6 +80,9 @@ bool walk(const Call& c, const PlanShape& shape) {
 }
 
 bool check(const Call& c) {
+    if (!plan_fits(c.rows, c.ctas)) {
+        return fail(c, "refused", c.rows, c.ctas);
+    }
     const PlanShape shape = plan_shape(c.rows, c.max_blocks, c.page_size, c.partitions, c.ctas);
     return shape.wide ? walk<unsigned long long>(c, shape) : walk<uint32_t>(c, shape);
 }
@@ -90,14 +93,14 @@ int main() {
     std::mt19937_64 rng(1);
     const auto below = [&rng](double limit) { return std::uniform_real_distribution<double>(0.0, limit)(rng); };
     long long calls = 0, wide = 0, dynamic = 0;
-    const int cta_counts[] = {148, 132, 74, 40, 37, 28};
+    const int cta_counts[] = {148, 132, 74, 37, 27, 8};
     for (int round = 0; round < 6000; ++round) {
         Call c;
         c.ctas = cta_counts[round % 6];
         c.page_size = rng() % 2 ? 16 : 64;
-        const int most_rows = static_cast<int>(std::min<long long>(
-            kPlanRows, (kMaxListTasks - kPlanPaddingDivisor - 4) * static_cast<long long>(c.ctas) / kPlanKvHeads));
-        c.rows = 1 + static_cast<int>(std::exp2(below(8.0)) - 1) % most_rows;
+        // up to 38 (row, kv head) pairs per SM
+        const int most_rows = std::min(kPlanRows, 38 * c.ctas / kPlanKvHeads);
+        c.rows = round % 7 == 0 ? most_rows : 1 + static_cast<int>(std::exp2(below(8.0)) - 1) % most_rows;
         c.max_blocks = static_cast<int>(std::exp2(below(28.0)));
         c.partitions = 2 + static_cast<int>(std::exp2(below(12.0)) - 1);
         const int kind = static_cast<int>(rng() % 4);
