@@ -370,4 +370,11 @@ __device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t word) {
     return out;
 }
 
+// One bf16 -> f16 likewise: finite saturation, a NaN stays a NaN.
+__device__ __forceinline__ __half bf16_to_f16(__nv_bfloat16 value) {
+    unsigned short out;
+    asm("cvt.rn.satfinite.f16.f32 %0, %1;" : "=h"(out) : "f"(__bfloat162float(value)));
+    return __ushort_as_half(out);
+}
+
 }  // namespace qwc

@@ -1003,8 +1003,7 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
                         if (staged_output != nullptr) {
                             // the same value as f16 in the operand layout of the output projection
                             const int feature = head * kHeadDim + dim;
-                            staged_output[(static_cast<size_t>(feature >> 3) * padded_rows + row) * 8 + (feature & 7)] =
-                                __float2half_rn(fminf(fmaxf(__bfloat162float(rounded), -65504.0f), 65504.0f));
+                            staged_output[(static_cast<size_t>(feature >> 3) * padded_rows + row) * 8 + (feature & 7)] = bf16_to_f16(rounded);
                         }
                     }
                 }
@@ -1161,8 +1160,7 @@ __global__ void __launch_bounds__(kMergeWarps * 32) reduce_partitions_kernel(
     if (staged_output != nullptr) {
         // the same value as f16 in the operand layout of the output projection
         const int feature = head * kHeadDim + dim;
-        staged_output[(static_cast<size_t>(feature >> 3) * padded_rows + row) * 8 + (feature & 7)] =
-            __float2half_rn(fminf(fmaxf(__bfloat162float(rounded), -65504.0f), 65504.0f));
+        staged_output[(static_cast<size_t>(feature >> 3) * padded_rows + row) * 8 + (feature & 7)] = bf16_to_f16(rounded);
     }
 }
 static_assert(kMergeWarps * 32 == kHeadDim, "a thread per dim");

@@ -458,6 +458,35 @@ def test_packed_attention_non_finite_query_stays_in_its_head(cuda, ops, value):
     assert not np.array_equal(got[0, 8], clean[0, 8])
 
 
+@pytest.mark.parametrize("partitions", [1, 3])
+def test_packed_attention_staged_output_holds_the_bf16_output(cuda, ops, partitions):
+    """The staged f16 output is the bf16 output, NaN for NaN (of a gate, and of a query whose scores are infinite);
+    values beyond f16 saturate."""
+    from qwencore_b200 import abi
+
+    torch = cuda
+    case = synth.attention_case(23, [300, 41], page_size=16, with_gate=True, scaled=True)
+    query = synth.bf16_value(case["query"]).astype(np.float32)
+    query[0, 8, 100] = np.inf
+    gate = synth.bf16_value(case["gate_projection"]).astype(np.float32)
+    gate[1, 3, 256 + 7] = np.nan
+    v_scale = case["v_scale"].copy()
+    v_scale[3] *= 1e7  # the heads of the last kv head reach beyond 65504
+    out, staged = bf16_out(torch, 2, 24, 256), ops.new_staged(2, 24 * 256)
+    workspace = torch.zeros(max(16, ops.packed_workspace_bytes(2, partitions)), dtype=torch.uint8, device="cuda")
+    held = [dev(torch, a) for a in (synth.bf16_bits(query), synth.bf16_bits(gate), case["key_cache"],
+                                    case["value_cache"], case["block_tables"], case["contexts"], case["k_scale"], v_scale)]
+    abi.check(abi.lib.qwc_paged_attention_packed_fp8_staged(
+        *[a.data_ptr() for a in held], out.data_ptr(), staged.data_ptr(), workspace.data_ptr(), workspace.numel(), 2, 0,
+        case["max_blocks"], 16, 0, partitions, 1.0 / 16.0, torch.cuda.current_stream().cuda_stream), "staged")
+    torch.cuda.synchronize()
+    want = synth.bf16_value(host(out)).reshape(2, 24 * 256)
+    got = host(ops.unstage(staged, 2, 24 * 256)).astype(np.float32)
+    assert np.isnan(want[0, 8 * 256:9 * 256]).all() and np.isnan(want[1, 3 * 256 + 7])
+    assert np.count_nonzero(np.abs(want) > 65504) > 100  # (infinities where f16 partials have been merged)
+    assert np.array_equal(got, np.clip(want, -65504, 65504).astype(np.float16).astype(np.float32), equal_nan=True)
+
+
 def test_packed_attention_legacy_entry_uses_configured_page_size(cuda, ops):
     from qwencore_b200 import abi
 
