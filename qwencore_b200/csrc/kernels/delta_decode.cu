@@ -329,8 +329,7 @@ __global__ void __launch_bounds__(kThreads, kLanes == 8 ? 7 : 4) delta_decode_in
         const float silu = gate_value / (1.0f + __expf(-gate_value));
         const __nv_bfloat16 result = __float2bfloat16(__bfloat162float(weighted) * silu);
         const int feature = h * kDim + dimension;
-        norm.staged[(static_cast<size_t>(feature >> 3) * norm.padded_rows + b) * 8 + (feature & 7)] =
-            __float2half_rn(fminf(fmaxf(__bfloat162float(result), -65504.0f), 65504.0f));
+        norm.staged[(static_cast<size_t>(feature >> 3) * norm.padded_rows + b) * 8 + (feature & 7)] = bf16_to_f16(result);
     } else {
         float* op = out + (static_cast<size_t>(b) * v_heads + h) * kDim + row_begin;
         for (int i = threadIdx.x; i < rows_here; i += kThreads) {

@@ -785,8 +785,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                                     y[token * row_pitch + column] = rounded;
                                 }
                                 if (p.y_staged != nullptr) {
-                                    y_staged[(column >> 3) * staged_pitch + token * 8 + (column & 7)] =
-                                        __float2half_rn(fminf(fmaxf(__bfloat162float(rounded), -65504.0f), 65504.0f));
+                                    y_staged[(column >> 3) * staged_pitch + token * 8 + (column & 7)] = bf16_to_f16(rounded);
                                 }
                             }
                         }
@@ -813,8 +812,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                                 y[token * row_pitch + column] = rounded;
                             }
                             if (p.y_staged != nullptr) {
-                                y_staged[(column >> 3) * staged_pitch + token * 8 + (column & 7)] =
-                                    __float2half_rn(fminf(fmaxf(__bfloat162float(rounded), -65504.0f), 65504.0f));
+                                y_staged[(column >> 3) * staged_pitch + token * 8 + (column & 7)] = bf16_to_f16(rounded);
                             }
                         }
                     }
@@ -930,8 +928,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                                 y[token * row_pitch] = rounded;
                             }
                             if (staged_wanted) {
-                                y_staged[token * staged_pitch] =
-                                    __float2half_rn(fminf(fmaxf(__bfloat162float(rounded), -65504.0f), 65504.0f));
+                                y_staged[token * staged_pitch] = bf16_to_f16(rounded);
                             }
                         }
                     }

@@ -907,8 +907,7 @@ __global__ void __launch_bounds__(kDeltaHeadDim) gated_rmsnorm_kernel(const floa
     }
     if (staged != nullptr) {
         const int feature = head * kDeltaHeadDim + dimension;
-        staged[(static_cast<size_t>(feature >> 3) * padded_rows + batch) * 8 + (feature & 7)] =
-            __float2half_rn(fminf(fmaxf(__bfloat162float(result), -65504.0f), 65504.0f));
+        staged[(static_cast<size_t>(feature >> 3) * padded_rows + batch) * 8 + (feature & 7)] = bf16_to_f16(result);
     }
 }
 

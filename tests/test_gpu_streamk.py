@@ -525,3 +525,63 @@ def test_prepare_steps_sum_any_number_of_slices(cuda, ops, batch, slices, v_head
             assert np.array_equal(on_rows, on_slices)
     finally:
         abi.configure(*before)
+
+
+@pytest.mark.parametrize("out_features,in_features", [(40, 512), (17408, 5120)], ids=["through_the_stash", "direct"])
+def test_staged_projections_keep_a_nan(cuda, ops, workspace, out_features, in_features):
+    """A row with a NaN is NaN in the bf16 and in the staged output, plain and SwiGLU; the other rows hold the same
+    values in both."""
+    torch = cuda
+    batch = 3
+    gate = synth.nvfp4_matrix(7, "nan.gate", out_features, in_features)
+    up = synth.nvfp4_matrix(7, "nan.up", out_features, in_features)
+    x = synth.bf16_value(synth.normal_bf16(7, "nan.x", (batch, in_features))).astype(np.float32)
+    x[1, 3] = np.nan
+    linears = [ops.Linear(dev(torch, m[0]), dev(torch, m[2]), 1.0, out_features, in_features) for m in (gate, up)]
+    staged_x = staged_input(torch, ops, synth.bf16_bits(x), batch, in_features)
+    for swiglu in (False, True):
+        out, staged = bf16_out(torch, batch, out_features), ops.new_staged(batch, out_features)
+        if swiglu:
+            ops.swiglu_w4a16_staged(*linears, staged_x, out, staged, batch, workspace)
+        else:
+            ops.w4a16_staged(linears[0], staged_x, out, staged, batch, workspace)
+        torch.cuda.synchronize()
+        rows = synth.bf16_value(host(out))
+        got = host(ops.unstage(staged, batch, out_features))
+        assert np.isnan(rows[1]).all() and np.isnan(got[1]).all()
+        for row in (0, 2):
+            assert_staged_holds(got[row], rows[row], f"swiglu {swiglu} row {row}")
+
+
+def test_staged_gated_norms_keep_a_nan(cuda, ops):
+    """A NaN gate, in the gated RMSNorm and in the recurrent update that fuses it."""
+    from qwencore_b200 import abi
+
+    torch = cuda
+    v_heads, batch = 32, 32
+    before = abi.get_shape()
+    abi.configure(v_heads, 16)
+    try:
+        case = synth.delta_case(9, batch, v_heads)
+        gates = synth.bf16_value(synth.normal_bf16(9, "z", (batch, v_heads * 128))).astype(np.float32)
+        gates[5, 1000] = np.nan
+        gate_dev = dev(torch, synth.bf16_bits(gates))
+        out_norm = dev(torch, synth.normal_bf16(9, "onorm", (128,), std=0.05))
+        stream = torch.cuda.current_stream().cuda_stream
+        inputs = [dev(torch, case[name]) for name in ("slots", "q", "k", "v", "alpha", "beta", "kq")]
+        state, scales = dev(torch, case["state"]), dev(torch, case["scales"])
+        out = torch.zeros((batch, v_heads, 128), dtype=torch.float32, device="cuda")
+        fused, alone = ops.new_staged(batch, v_heads * 128), ops.new_staged(batch, v_heads * 128)
+        abi.check(abi.lib.qwc_delta_decode_int8_step(
+            state.data_ptr(), scales.data_ptr(), *[t.data_ptr() for t in inputs], out.data_ptr(), case["capacity"],
+            batch, None, 0, 1.0, gate_dev.data_ptr(), v_heads * 128, 0, out_norm.data_ptr(), 1e-6, fused.data_ptr(),
+            stream), "qwc_delta_decode_int8_step")
+        abi.check(abi.lib.qwc_delta_gated_rmsnorm_staged(
+            dev(torch, case["v"]).data_ptr(), gate_dev.data_ptr(), out_norm.data_ptr(), None, alone.data_ptr(), batch,
+            1e-6, v_heads * 128, stream), "qwc_delta_gated_rmsnorm_staged")
+        torch.cuda.synchronize()
+        for staged in (fused, alone):
+            got = host(ops.unstage(staged, batch, v_heads * 128)).astype(np.float32)
+            assert np.argwhere(np.isnan(got)).tolist() == [[5, 1000]]
+    finally:
+        abi.configure(*before)
