@@ -1034,9 +1034,10 @@ __global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(kThreads)
     const int row_index = blockIdx.y;
     const int rank = static_cast<int>(cluster.block_rank());
     const float* row = logits + static_cast<size_t>(row_index) * vocab;
-    const int span = ((vocab + kArgmaxCtas - 1) / kArgmaxCtas + 3) & ~3;
+    // (what is left of a share is counted down: columns past it could pass the largest int)
+    const int span = ((vocab - 1) / kArgmaxCtas + 4) & ~3;
     const int begin = rank * span;
-    const int end = min(vocab, begin + span);
+    const int end = begin + max(min(span, vocab - begin), 0);
     // A thread's columns ascend, so a later equal value never replaces an earlier one and the key is made once, at
     // the end.  The loads of a batch are in flight together: with one at a time a thread's nineteen (151 936
     // logits) were as many L2 round trips (head and argmax of five rows as a user
@@ -1051,14 +1052,14 @@ __global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(kThreads)
     };
     if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
 #pragma unroll 1
-        for (int first = begin + 4 * threadIdx.x; first < end; first += 4 * kThreads * kArgmaxDepth) {
+        for (int left = end - begin - 4 * static_cast<int>(threadIdx.x); left > 0; left -= 4 * kThreads * kArgmaxDepth) {
+            const int first = end - left;
             float4 v[kArgmaxDepth];
 #pragma unroll
             for (int j = 0; j < kArgmaxDepth; ++j) {
-                const int column = first + 4 * kThreads * j;
                 // (what is not there, or not there as a whole, never wins)
-                v[j] = column + 4 <= end ? __ldcs(reinterpret_cast<const float4*>(row + column))
-                                         : make_float4(NAN, NAN, NAN, NAN);
+                v[j] = 4 * kThreads * j + 4 <= left ? __ldcs(reinterpret_cast<const float4*>(row + first + 4 * kThreads * j))
+                                                    : make_float4(NAN, NAN, NAN, NAN);
             }
 #pragma unroll
             for (int j = 0; j < kArgmaxDepth; ++j) {
@@ -1069,7 +1070,7 @@ __global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(kThreads)
                 consider(v[j].w, column + 3);
             }
         }
-        const int whole = begin + (max(end - begin, 0) & ~3);
+        const int whole = begin + ((end - begin) & ~3);
         if (threadIdx.x == 0) {  // the last one to three of a row (its columns are behind all of this thread's)
             for (int column = whole; column < end; ++column) {
                 consider(row[column], column);
@@ -1077,11 +1078,12 @@ __global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(kThreads)
         }
     } else {
 #pragma unroll 1
-        for (int first = begin + threadIdx.x; first < end; first += kThreads * kArgmaxDepth) {
+        for (int left = end - begin - static_cast<int>(threadIdx.x); left > 0; left -= kThreads * kArgmaxDepth) {
+            const int first = end - left;
             float v[kArgmaxDepth];
 #pragma unroll
             for (int j = 0; j < kArgmaxDepth; ++j) {
-                v[j] = first + kThreads * j < end ? __ldcs(row + first + kThreads * j) : NAN;
+                v[j] = kThreads * j < left ? __ldcs(row + first + kThreads * j) : NAN;
             }
 #pragma unroll
             for (int j = 0; j < kArgmaxDepth; ++j) {

@@ -832,6 +832,18 @@ def test_argmax_any_width_and_alignment(cuda, ops, vocab):
     assert host(tokens).tolist() == want
 
 
+@pytest.mark.parametrize("vocab", [2 ** 31 - 1, 2 ** 31 - 4096])
+def test_argmax_up_to_the_largest_width(cuda, ops, vocab):
+    """The last columns that an int can count; nothing behind the row is read."""
+    torch = cuda
+    logits = torch.zeros(vocab, dtype=torch.float32, device="cuda")
+    logits[vocab - 1] = 1.0
+    tokens = u32_out(torch, 1)
+    ops.argmax(logits, torch.zeros(256, dtype=torch.float32, device="cuda"), u32_out(torch, 256), tokens, vocab, 1, 256)
+    torch.cuda.synchronize()
+    assert host(tokens).tolist() == [vocab - 1]
+
+
 @pytest.mark.parametrize("v_heads", [32, 48], ids=["h32_oracle_generalisation", "h48_reference_shape"])
 def test_delta_prepare_and_gated_rmsnorm(cuda, ops, v_heads):
     """crates/qwc-cuda/tests/delta_net.rs:576-716 (CPU conv/gate check) and :716-777."""
