@@ -697,6 +697,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (t == 0) {
             QWC_TRACE_LANE0(5);  // last MMA issued
         }
+        // The CTA may leave because some wait has given up: not before the last of these MMAs has read shared memory
+        // and written tensor memory (0.2 ms at most; none issued: a phase that counts as passed).
+        const int last_buf = buf == 0 ? kABuffers - 1 : buf - 1;
+        const long long start = clock64();
+        while (!mbar_try_wait(&bars.a_free[t][last_buf], buf == 0 ? a_parity ^ 1 : a_parity) &&
+               clock64() - start < 400000ll) {
+        }
+        __syncwarp();
     } else if (warp == kXWarp) {
         // ---------------- activation chunks ----------------
         // Everything above starts before the kernel that produces the activations has finished; these
