@@ -154,6 +154,13 @@ __device__ __noinline__ bool wait_or_fail_slow(uint64_t* bar, uint32_t parity, B
     return false;
 }
 
+// For what must have arrived before the CTA ends, whether it is used or not: 0.2 ms at most.
+__device__ __forceinline__ void wait_a_little(uint64_t* bar, uint32_t parity) {
+    const long long start = clock64();
+    while (!mbar_try_wait(bar, parity) && clock64() - start < 400000ll) {
+    }
+}
+
 __device__ __forceinline__ bool wait_or_fail(uint64_t* bar, uint32_t parity, Barriers* b, int* status) {
     if (mbar_try_wait(bar, parity)) {
         return true;
@@ -297,6 +304,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     float result[32];
     bool have_result = false;
+    int asked = early_stages;  // the producer: stages
 
     if (warp < kDequantWarps) {
         // ---------------- dequantise: thread = row ----------------
@@ -446,6 +454,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 issue_stage(wstage);
             }
             __syncwarp();
+            asked = wstage + 1;
         }
         if (ok && p.next.valid && elect_one()) {
             for (int cta = blockIdx.x; cta < p.next.ctas; cta += gridDim.x) {
@@ -523,6 +532,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                 x_parity ^= 1;
             }
         }
+        // (whatever made the CTA give up: not before the last of these MMAs is done)
+        wait_a_little(&bars.a_free[t][buf == 0 ? kABuffers - 1 : buf - 1], buf == 0 ? a_parity ^ 1 : a_parity);
     } else {
         // ---------------- activation rows: bf16 -> f16, K-major core matrices ----------------
         // Converting warp w owns operand stage w and the chunks w, w + 4, ...  The bf16 rows of a
@@ -566,6 +577,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
+                wait_a_little(&bars.raw_full[w], raw_parity);  // (the rows may still be landing)
                 break;
             }
 #pragma unroll
@@ -708,14 +720,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         cluster.sync();  // nobody leaves while a peer may still read its shared memory
     }
 
-    // A CTA that gave up must not return while the stages it asked for before the barrier are still
-    // landing in its shared memory: their thread waits for them, with a limit of 0.2 ms per ring slot
-    // (a stage that was consumed has completed its first phase long ago and the wait falls through).
+    // A CTA that gave up must not return while stages it asked for are still landing in its shared memory: their
+    // thread waits for the last trip round the ring (a stage that was consumed has completed its phase long ago).
     if (failed && threadIdx.x == kProducerWarp * 32) {
-        for (int slot = 0; slot < kWeightStages; ++slot) {
-            const long long start = clock64();
-            while (!mbar_try_wait(&bars.w_full[slot], 0) && clock64() - start < 400000ll) {
-            }
+        for (int i = asked > kWeightStages ? asked - kWeightStages : 0; i < asked; ++i) {
+            wait_a_little(&bars.w_full[i % kWeightStages], (i / kWeightStages) & 1);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
