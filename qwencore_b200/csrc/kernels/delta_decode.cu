@@ -374,6 +374,7 @@ using DeltaKernel = void (*)(int8_t*, float*, const uint32_t*, const float*, con
 // lanes): 48 heads at 1 row 3.49 / 4.79, at 9 rows (432 CTAs) 7.24 / 11.2, at 12 rows (576) 7.63 / 11.7; 32 heads
 // at 20 rows (640) 11.1 / 11.7, at 22 rows (704) 11.2 / 11.9, at 23 rows (736) 11.6 / 12.2, at 25 rows (800)
 // 12.5 / 12.0, at 32 rows (1024) 13.6 / 12.8; 48 heads at 16 rows (768) 12.1 / 12.0, at 32 rows (1536) 19.7 / 18.4.
+// (test_delta_decode_both_forms takes the batches on either side of this line.)
 template <bool kEarly>
 DeltaKernel kernel_for(int ctas) {
     return ctas <= 5 * sm_count_delta() ? delta_decode_int8_kernel<kEarly, 4> : delta_decode_int8_kernel<kEarly, 8>;

@@ -564,15 +564,21 @@ def test_delta_decode_int8_matches_oracle(cuda, ops, batch, v_heads):
         assert np.array_equal(scales[slot], case["scales"][slot])
 
 
-@pytest.mark.parametrize("batch,v_heads", [(21, 32), (22, 32), (14, 48), (15, 48), (1, 32), (2, 32), (3, 48)],
-                         ids=["ctas_672", "ctas_704", "ctas_672_h48", "ctas_720_h48", "row_split_16", "row_split_8",
-                              "row_split_4"])
+@pytest.mark.parametrize("batch,v_heads", [("last_four_lanes", 32), ("first_eight_lanes", 32), ("last_four_lanes", 48),
+                                           ("first_eight_lanes", 48), (32, 32), (32, 48), (1, 32), (2, 32), (3, 48)],
+                         ids=["last_four_lanes", "first_eight_lanes", "last_four_lanes_h48", "first_eight_lanes_h48",
+                              "full_batch", "full_batch_h48", "row_split_16", "row_split_8", "row_split_4"])
 @pytest.mark.parametrize("exponent", [0, -100, 92], ids=["unit_q", "tiny_q", "huge_q"])
 def test_delta_decode_both_forms(cuda, ops, batch, v_heads, exponent):
-    """On either side of the line between four and eight lanes per row, with row splits, with a key of zeros
+    """On either side of the line between four and eight lanes per row (five CTAs per SM; with 148 SMs 23 | 24 rows of
+    32 heads and 15 | 16 of 48), at the full batch, with row splits, with a key of zeros
     and with a query at the ends of the fp32 range (a power of two: only `out` scales with it, the update
     does not see q).  Bounds: out within 1e-5 of its row's largest value (128 fp32 roundings of 6e-8 on either
     side, in different orders), codes within one step, where row . k moves by a unit in the last place."""
+    line = 5 * cuda.cuda.get_device_properties(0).multi_processor_count // v_heads
+    if isinstance(batch, str):
+        batch = line if batch == "last_four_lanes" else line + 1
+        assert 3 < batch <= 32, "both forms have a batch of their own"
     case = synth.delta_case(11, batch, v_heads)
     k, q = case["k"].copy(), case["q"].copy()
     k[0] = 0.0
