@@ -153,16 +153,6 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
-// 16-byte streaming load that does not allocate in L1: weights and cache pages are
-// read exactly once per launch.
-__device__ __forceinline__ uint4 ldg_stream(const void* ptr) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(ptr));
-    return v;
-}
-
 // ---- mbarrier / bulk-copy (TMA 1-D) wrappers -------------------------------------
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -261,10 +251,6 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 
 __device__ __forceinline__ void bulk_wait_all_read() {
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-
-__device__ __forceinline__ void bulk_wait_all() {
-    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // Programmatic dependent launch.  A kernel launched with the programmatic-serialization attribute
