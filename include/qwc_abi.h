@@ -331,8 +331,8 @@ int qwc_paged_attention_packed_fp8_scaled(const void* query, const void* query_g
  * larger is refused with cudaErrorInvalidValue before a launch.  The first call on a device
  * looks the scratch address up (cudaGetSymbolAddress with that device current) and should
  * therefore be made before any stream capture begins.  All calls share the one array: it keeps
- * whatever the previous call left (every slot a call reads it has written first, so nothing has
- * to be cleared), and two calls whose kernels overlap on the GPU - different streams, or
+ * whatever the previous call left (a call uses no slot that it has not written itself, so nothing
+ * has to be cleared), and two calls whose kernels overlap on the GPU - different streams, or
  * different host threads - race on it.  Callers that need concurrency pass their own workspace
  * to the _scaled entry point instead.
  */

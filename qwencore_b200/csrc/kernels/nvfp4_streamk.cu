@@ -31,7 +31,7 @@
 //   warp 16     weight producer: per stage one tiled TMA copy per tile (128 rows x 128 bytes,
 //               128-byte swizzle) and one bulk copy of the tile's swizzled scale blocks; 4-stage ring.
 //   warps 17-18 issue tcgen05.mma, one warp per tile (elect.sync region).
-//   warp 19     activation producer: one bulk copy per chunk into a 6-chunk ring; the only warp
+//   warp 19     activation producer: one bulk copy per chunk into a 5-chunk ring; the only warp
 //               besides the epilogue that waits for the previous kernel (programmatic launch).
 //   warps 20-27 epilogue: warp e reads TMEM lanes 32 (e % 4) .. + 31 (those output rows) of both tiles
 //               for half of the activation rows (e / 4).  Both tiles in one thread means the gate and up
@@ -740,8 +740,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else {
         // ---------------- epilogue ----------------
         // Warp e: output rows 32 (e % 4) .. + 31 of both tiles, activation rows (e / 4) * kPad / 2 .. .
-        // Everything goes through the warp's 4 KiB stash in shared memory ([tile * kCols + column][lane]),
-        // eight columns at a time, so that no step holds more than a few registers.
+        // Results go through the warp's 4 KiB stash in shared memory ([tile * kCols + column][lane]), eight columns
+        // at a time, so that no step holds more than a few registers; where nothing has to be summed or sampled they
+        // leave straight from tensor memory (store_direct).
         constexpr int kCols = kPad / 2;  // accumulator columns per tile and warp
         const int e = warp - kFirstEpilogueWarp;
         const int quarter = e & 3;
@@ -1058,6 +1059,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                         }
                     }
                 }
+                // (store_direct reads the accumulators only after this; its CTAs have a single segment, so no MMA waits
+                // for them to be free)
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) {

@@ -7,13 +7,14 @@
 //
 // The op reads every K and V byte of the row's context once and nothing else of
 // size, so it is HBM-bound.  Layout for sm_100a:
-//   * a persistent grid of one CTA per SM.  The rows of a ragged batch differ in context by
-//     orders of magnitude, so the work is cut on the device into equal shares: the 16-token
-//     units of all (row, kv head) pairs are laid end to end, CTA c owns positions
-//     [c share, (c + 1) share) of that line, and a task is the piece of one pair inside one
-//     CTA's share (its partial is merged by the second kernel).  Every CTA streams the same
-//     number of bytes whatever the contexts are, and the launch shape depends only on the SM
-//     count, so the step stays capturable in a CUDA graph;
+//   * one CTA per SM at a time.  The rows of a ragged batch differ in context by orders of magnitude, so the
+//     work is cut on the device (attention_plan.h): the 16-token units of all (row, kv head) pairs are laid end
+//     to end, chunks of that line are dealt to the CTAs, and a task is the piece of one pair inside one chunk (its
+//     partial is merged by the second kernel).  Up to 192 units per SM a chunk is an equal share of the line.
+//     Beyond, there are a large chunk per SM and small ones, which go to whoever is done first: the grid has a
+//     CTA for each, and a running CTA takes over those that have not started.  The launch shape depends on the SM
+//     count, the rows and what the block tables could describe, not on the contexts, so the step stays
+//     capturable in a CUDA graph;
 //   * nobody converts a cache byte.  K and V go from memory to tcgen05.mma.kind::f8f6f4 as they are
 //     stored: a stage is 128 tokens of one kv head, each unit of 16 tokens (a whole 16-token page, or a quarter
 //     of a 64-token page) two swizzled TMA boxes of 128 bytes per token.  K is the A operand of S^T = K Q^T
@@ -986,7 +987,8 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
                             float* stats = partial_stats + slot * kPartialFloats;
                             stats[0] = sm.task_max[t & 1][h];
                             // the last piece of a pair carries a sign
-                        stats[1] = task.last ? __uint_as_float(__float_as_uint(denominator) | 0x80000000u) : fabsf(denominator);
+                            stats[1] = task.last ? __uint_as_float(__float_as_uint(denominator) | 0x80000000u)
+                                                 : fabsf(denominator);
                         }
                         partial_out[slot * kHeadDim + dim] = __float2half_rn(value);
                     } else {
@@ -1372,9 +1374,9 @@ extern "C" int qwc_paged_attention_packed_fp8_noalloc(const void* query, const v
     if (resolved != cudaSuccess) {
         return resolved;
     }
-    // Every partial slot the merge reads was written by this call (the merge recomputes which of
-    // a row's slots the attention kernel used), so nothing left over from an earlier call is read
-    // and nothing needs clearing first.
+    // Nothing needs clearing first.  The merge loads statistics and outputs of slots that this call may not have
+    // written, but what it uses ends at the last piece of a pair, which the sign of its sum marks: the pieces of a
+    // pair lie side by side from slot 0 on, and all of them are written by every call.
     return qwc::launch_attention(query, query_gate_projection, key_cache, value_cache, block_tables,
                                  context_lengths, key_scales, value_scales, output, scratch,
                                  qwc::kStaticScratchBytes, rows, row_base, max_blocks, page_size, gate_stride,

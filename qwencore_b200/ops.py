@@ -178,9 +178,10 @@ def packed_partition_count(rows: int, context: int, sms: int = 148) -> int:
     """Upper bound on the context partitions of a decode row, which sizes the workspace.
 
     Same role as packed_partition_count (crates/qwc-cuda/src/paged_attention.rs:230-253), with a
-    different meaning of the result: the kernel cuts the rows into tasks of equal size on the
-    device (from the sum of the contexts it finds), and `partitions` only caps how many tasks one
-    row may become.  Spans of at least 128 tokens; at most 4096 partial slots per head.
+    different meaning of the result: the kernel cuts the rows on the device, at the ends of the
+    chunks that it deals to the SMs (from the sum of the contexts it finds), and `partitions` only
+    caps how many pieces one row may become.  Spans of at least 128 tokens; at most 4096 partial
+    slots per head.
     """
     assert rows > 0 and context > 0
     want = max(1, (context + 127) // 128)
