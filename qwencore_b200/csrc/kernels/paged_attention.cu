@@ -41,8 +41,8 @@
 //
 // What it took to get there: widening every cache byte to f16 for mma.sync kept the conversion unit 76 % busy
 // and the stage on dependent instructions.  Measured (us, layers that L2 does not hold, before / now):
-// 32 rows in [128, 2048] 26.4 / 23.4, one row of 2048 12.3 / 11.4, three rows of 32768 45.3 / 42.4 (6.1 TB/s while it
-// streams), 32 rows log-uniform to 32768 82.8 / 77.2, 20 rows from 8192 to 32768 134.1 / 121.1 (6.1 TB/s all in all).
+// 32 rows in [128, 2048] 26.4 / 23.1, one row of 2048 12.3 / 10.3, three rows of 32768 45.3 / 42.5 (6.1 TB/s while it
+// streams), 32 rows log-uniform to 32768 82.8 / 77.0, 20 rows from 8192 to 32768 134.1 / 121.4 (6.1 TB/s all in all).
 // The new operands alone, on the old plan and merge, gave 26.4 / 25.5 and 82.9 / 82.6: what had been hidden behind
 // the conversions was the plan, the merge and CTAs that ended early (SplitPlan, reduce_partitions_kernel).
 //
