@@ -50,6 +50,7 @@
 // pool, as the reference allocates it): positions past the context are masked by
 // zero probabilities, not skipped.
 
+#include <algorithm>
 #include "attention_plan.h"
 #include "tcgen05.cuh"
 
@@ -74,7 +75,7 @@ constexpr int kStageBytes = 2 * kHalfBytes;             // K or V of a stage
 constexpr int kStages = 3;
 constexpr int kQueryDigits = 4;                         // of weight 1, 2^-4, 2^-18, 2^-23
 constexpr int kProbabilityDigits = 3;                   // of weight 1, 2^-4, 2^-8
-constexpr int kColumns = 32;                            // digit j of head h is column 8 j + h; the rest is zero
+constexpr int kColumns = 32;                            // digit j of head h is column 8 j + h; the rest is not used
 constexpr int kQueryBytes = kColumns * kHeadDim;        // B operand of S, K-major core matrices
 constexpr int kProbabilityBytes = kColumns * kStageTokens;  // B operand of O, MN-major core matrices
 constexpr int kTmemColumns = 256;
@@ -319,15 +320,6 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
     const int units_per_page = page_size / kUnitTokens;
     const int capacity_units = max_blocks * units_per_page;
 
-    // Stale bytes of a partly filled stage are multiplied by zero probabilities, so they
-    // must be finite: clear the value ring once (every later byte comes from the cache).  The columns of a
-    // query that belong to no digit stay zero.
-    for (int i = threadIdx.x; i < kStages * kStageBytes / 16; i += kThreads) {
-        reinterpret_cast<uint4*>(&sm.v[0][0])[i] = make_uint4(0, 0, 0, 0);
-    }
-    for (int i = threadIdx.x; i < 2 * kQueryBytes / 16; i += kThreads) {
-        reinterpret_cast<uint4*>(&sm.q[0][0])[i] = make_uint4(0, 0, 0, 0);
-    }
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
                      "r"(kTmemColumns)
@@ -555,16 +547,22 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attention_packed_kernel(
                     if (!ok) {
                         break;
                     }
+                    // V that a partly filled stage leaves out is multiplied by probabilities of zero and must be
+                    // finite, whatever the stage before it held: boxes in front of the first row arrive as zeros.  (The
+                    // ring used to be cleared at the start of every CTA: 24 rows of at most 192 tokens 12.95 -> 12.68
+                    // us, 32 rows in [128, 2048] 23.9 -> 23.6.)
+                    const int boxes = keys ? units : kStageUnits;
                     if (lane == 0) {
-                        mbar_arrive_expect_tx(&full[slot], static_cast<uint32_t>(units) * 2 * kBoxBytes);
+                        mbar_arrive_expect_tx(&full[slot], static_cast<uint32_t>(boxes) * 2 * kBoxBytes);
                         if (keys) {
                             *reinterpret_cast<volatile int*>(&sm.stages_asked) = n + 1;
                         }
                     }
                     __syncwarp();
-                    if (unit < units) {
-                        const int row = (static_cast<int>(physical) * kKvHeads + task.kv_head) * page_size +
-                                        (first + unit) % units_per_page * kUnitTokens;
+                    if (unit < boxes) {
+                        const int row = unit < units ? (static_cast<int>(physical) * kKvHeads + task.kv_head) * page_size +
+                                                           (first + unit) % units_per_page * kUnitTokens
+                                                     : -kUnitTokens;
                         tma_box_g2s(ring + slot * kStageBytes + half * kHalfBytes + unit * kBoxBytes, map, half * 128, row,
                                     &full[slot]);
                     }
@@ -1244,8 +1242,10 @@ cudaError_t launch_attention(const void* query, const void* query_gate_projectio
     const PlanShape plan =
         split ? plan_shape(rows, max_blocks, page_size, partitions, sms) : PlanShape{0, false, false};
     const AttentionKernel kernel = attention_kernels[split ? (plan.wide ? 2 : 1) : 0];
+    // (undivided rows: no CTA without a task; 24 rows of 128 tokens 6.23 -> 6.01 us)
+    const int grid = !split ? std::min(sms, rows * kKvHeads) : plan.may_be_dynamic ? kChunksPerSm * sms : sms;
     const cudaError_t launched = qwc::launch_chained(
-        kernel, dim3(plan.may_be_dynamic ? kChunksPerSm * sms : sms), dim3(kThreads), shared, stream, key_map, value_map,
+        kernel, dim3(grid), dim3(kThreads), shared, stream, key_map, value_map,
         static_cast<const __nv_bfloat16*>(query), static_cast<const __nv_bfloat16*>(query_gate_projection),
         static_cast<const uint32_t*>(block_tables), static_cast<const uint32_t*>(context_lengths), key_scales,
         value_scales, split ? nullptr : static_cast<__nv_bfloat16*>(output),

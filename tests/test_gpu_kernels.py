@@ -510,6 +510,20 @@ def test_packed_attention_staged_output_holds_the_bf16_output(cuda, ops, partiti
     assert np.array_equal(got, np.clip(want, -65504, 65504).astype(np.float16).astype(np.float32), equal_nan=True)
 
 
+@pytest.mark.parametrize("partitions", [1, 4])
+def test_packed_attention_non_finite_value_stays_in_its_row(cuda, ops, partitions):
+    """Rows whose stages are partly filled, on CTAs that have had full stages of a row with NaN values before."""
+    contexts = np.full(150, 16, dtype=np.uint32)
+    contexts[:37] = 1024  # (with 148 SMs undivided rows 37 apart meet on a CTA)
+    case = synth.attention_case(25, contexts, page_size=16)
+    clean = run_attention(cuda, ops, case, 16, partitions)
+    values = case["value_cache"].copy()
+    values[case["block_tables"][0, :64]] = 0x7F
+    got = run_attention(cuda, ops, dict(case, value_cache=values), 16, partitions)
+    assert np.isnan(got[0]).all()
+    assert np.array_equal(got[1:], clean[1:])
+
+
 def test_packed_attention_legacy_entry_uses_configured_page_size(cuda, ops):
     from qwencore_b200 import abi
 
